@@ -1777,8 +1777,13 @@ int bcr_batch_s::tune_class(size_t ci) {
   cudaEventCreate(&e1);
   float best = 1e30f;
   int bf = c.fam, bc = c.chunk;
+  // both schedules of a shape run one family, so that their results stay
+  // bit-identical whichever was tuned first
+  int only = bcr::PAIR_AUTO;
+  for (const auto& t : g_batch_tuning)
+    if (t.n == dm.n && t.nrm == nrm && t.nxm == nxm && t.mixed == c.mixed && t.persist != c.persist) only = t.fam;
   for (int f : {bcr::PAIR_TC, bcr::PAIR_GRP, bcr::PAIR_ROWS}) {
-    if (!bcr::batch_family_ok(f, dm, c.mixed != 0)) continue;
+    if (!bcr::batch_family_ok(f, dm, c.mixed != 0) || (only != bcr::PAIR_AUTO && f != only)) continue;
     for (int ch : {2, 4, 8, 16}) {
       c.fam = f;
       c.chunk = ch;

@@ -594,17 +594,61 @@ __global__ void __launch_bounds__(128) k_factor_lu_rows(FactorArgs<T> a0, const 
 //   phase 1 (SIMT, lane = panel row): partial-pivot LU of the 2N x N panel
 //     [E_jp; D_j] in registers, with getrf's row order replayed on positions
 //     (mypos) and the pivot chosen by exact integer reductions on the bits of
-//     |a| (largest |a|, then smallest position: the idamax rule).  The nr
-//     border rows ride along as a second register row of lanes 0..nr-1 and
-//     come out as C_j U^-1.
-//   phase 2 (SIMT): the elimination operator on the trailing columns,
-//       G = [ L^-1 ; -M L^-1 ; -(C_j U^-1) L^-1 ]      ((2N+8) x N)
-//     by a right triangular solve X L = [I; -M; -C'] per lane.
-//   phase 3 (FP64 tensor cores, mma.sync m8n8k4): one GEMM
+//     |a| (largest |a|, then smallest position: the idamax rule).  The columns
+//     already eliminated are reused, Gauss-Jordan style, for the operator that
+//     the eliminations apply to the trailing columns,
+//       G = [ L^-1 ; -M L^-1 ; -(C_j U^-1) L^-1 ]      ((2N+8) x N),
+//     so that no triangular solve follows.  The nr border rows are spread over
+//     the warp.
+//   phase 2 (FP64 tensor cores, mma.sync m8n8k4): one GEMM
 //       [U-row | reduced row | border update] = G (PW)_top + [0; (PW)_bot; 0]
 //     over the 2N + nx trailing columns [x_jp | x_jpp | xb].
-// The results are staged in shared memory and written with coalesced stores.
+//
+// Bound by the pivot steps' dependency chains (4 warps per scheduler) and the L1
+// data pipe (61% busy: 1,380 wavefronts per pair, level 1 of n = 16).  Keeping
+// the operator in the eliminated columns instead of solving X L = [I; -M; -C']
+// after the LU took a pair from 3,093 to 2,616 instructions and level 1 of
+// 40,000 blocks from 179 to 165 us.
+//
+// T_j and C_j hold the operator form: T_j = [L^-1 below the diagonal, U on and
+// above it; -M L^-1], C_j = -C_j U^-1 L^-1.  The forward sweep applies them as
+// one matrix-vector product (SweepArgs::op).
 // ---------------------------------------------------------------------------
+template <typename T> __device__ __forceinline__ T rcp_rn(T x);
+template <> __device__ __forceinline__ double rcp_rn<double>(double x) { return __drcp_rn(x); }
+template <> __device__ __forceinline__ float rcp_rn<float>(float x) { return __frcp_rn(x); }
+
+// Pivot candidate of one lane: |a| as an integer key (upper word + 1, lower
+// word; NaN below every number, finished rows below everything) and the
+// reciprocal of a by Newton-Raphson steps r <- r + r (1 - a r) from the
+// hardware's approximation, which doubles the correct bits each time (FP64:
+// about 20, 40, 80; FP32: 23, then rounding): at most one unit in the last
+// place off for the magnitudes tc_plain_pivot() accepts, and free of the range
+// branches of a correctly rounded reciprocal, which would cut the step into
+// pieces the scheduler cannot overlap.
+__device__ __forceinline__ void tc_candidate(double v, bool done, unsigned& hi, unsigned& lo, double& rc) {
+  const unsigned h = (unsigned)__double2hiint(v) & 0x7fffffffu;
+  hi = done ? 0u : h > 0x7ff00000u ? 1u : h + 1u;
+  lo = (unsigned)__double2loint(v);
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(v));
+  r = fma(fma(-v, r, 1.0), r, r);
+  rc = fma(fma(-v, r, 1.0), r, r);
+}
+__device__ __forceinline__ void tc_candidate(float v, bool done, unsigned& hi, unsigned& lo, float& rc) {
+  const unsigned h = __float_as_uint(v) & 0x7fffffffu;
+  hi = done ? 0u : h > 0x7f800000u ? 1u : h + 1u;
+  lo = 0u;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  rc = fmaf(fmaf(-v, r, 1.0f), r, r);
+}
+// the pivot's magnitude (key hi) is a normal number whose reciprocal is one too
+template <typename T>
+__device__ __forceinline__ bool tc_plain_pivot(unsigned hi) {
+  return sizeof(T) == 8 ? hi - 0x00200000u < 0x7fc00000u - 0x00200000u : hi - 0x01000000u < 0x7e000000u - 0x01000000u;
+}
+
 __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                : "+d"(d0), "+d"(d1)
@@ -625,7 +669,7 @@ struct TcShape {
   static constexpr int MTILES = MT / 8;
   static constexpr int WS = 2 * N * LDW;            // doubles: the 2N panel rows' trailing part
   static constexpr int GS = MT * LDG;
-  static constexpr size_t BYTES = (size_t)(WS + GS + N + 2) * sizeof(T) + 2 * N * sizeof(int);
+  static constexpr size_t BYTES = (size_t)(WS + GS) * sizeof(T) + 2 * N * sizeof(int);
 };
 
 // element (row, col) of the trailing part from the compact rows
@@ -676,8 +720,7 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
   using S = TcShape<N, T>;
   constexpr unsigned FULL = 0xffffffffu;
   T* Gs = Wt + S::WS;
-  T* bc = Gs + S::GS;                             // pivot row + its reciprocal
-  int* rowof = reinterpret_cast<int*>(bc + N + 2);
+  int* rowof = reinterpret_cast<int*>(Gs + S::GS);
   const Dims d = a.d;
   const int nr = d.nr, nx = d.nx;
   constexpr int n = N, n2 = 2 * N;
@@ -789,143 +832,106 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
       Wt[r * S::LDW + c - n] = T(0);
     }
   }
-  // --------------------------------------------------- phase 1: panel LU
+  // ------------------- phase 1: panel LU with the operator rows in place
+  // After step i a row not yet a pivot is orig_r + sum_{c <= i} X_r[c] orig(pivot c):
+  // eliminating column i frees its register, which takes X_r[i] = -l, and the
+  // same multiplier updates the X of the earlier columns with the pivot row's
+  // X, so one run of N - 1 fused multiply-adds per step yields U, L^-1 (the
+  // pivot rows' X, strictly lower), -M L^-1 and -C' L^-1 (see the comment above).
   int mypos = lane, info = 0;
   bool done = !act;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    // every lane forms the reciprocal of its own candidate while the pivot is
-    // searched; the pivot lane publishes its value with the pivot row
-    // pivot: max |a| over rows not yet used, ties to the smaller position
-    // (FP64: upper word of |a|, then the lower word; FP32: the whole word)
+    // pivot: max |a| over the rows not yet used, ties to the smaller position;
+    // every lane forms the reciprocal of its own candidate meanwhile
+    unsigned hi, lo, hmax, m;
     T rc;
-    unsigned hi, lob;
+    tc_candidate(rowA[i], done, hi, lo, rc);
+    hmax = __reduce_max_sync(FULL, hi);
     if constexpr (sizeof(T) == 8) {
-      rc = __drcp_rn(rowA[i]);
-      const double av = fabs(rowA[i]);
-      const unsigned long long bits = (unsigned long long)__double_as_longlong(av);
-      hi = (unsigned)(bits >> 32) + 1u;
-      if (done) hi = 0u;
-      else if (av != av) hi = 1u;  // NaN loses against every number
-      lob = (unsigned)bits;
-    } else {
-      rc = __frcp_rn(rowA[i]);
-      const float av = fabsf(rowA[i]);
-      hi = __float_as_uint(av) + 1u;
-      if (done) hi = 0u;
-      else if (av != av) hi = 1u;
-      lob = 0u;
-    }
-    const unsigned hmax = __reduce_max_sync(FULL, hi);
-    unsigned m = __ballot_sync(FULL, hi == hmax && !done);
-    unsigned pmin;
-    if (__popc(m) == 1) {  // unique maximum in the upper word: the usual case
-      pmin = (unsigned)__shfl_sync(FULL, mypos, __ffs(m) - 1);
-    } else {               // exact tie handling: lower word, then smallest position
-      const unsigned lo = (hi == hmax) ? lob : 0u;
+      lo = hi == hmax ? lo : 0u;
       const unsigned lmax = __reduce_max_sync(FULL, lo);
-      const bool cand = (hi == hmax) && (lo == lmax) && !done;
-      pmin = __reduce_min_sync(FULL, cand ? (unsigned)mypos : 0xffffffffu);
-      m = __ballot_sync(FULL, cand && (unsigned)mypos == pmin);
+      m = __ballot_sync(FULL, hi == hmax && lo == lmax);
+    } else {
+      m = __ballot_sync(FULL, hi == hmax);
     }
-    const int p = __ffs(m) - 1;
-    if (!done && mypos == i && lane != p) mypos = (int)pmin;
-    if (lane == p) {
-      mypos = i;
-#pragma unroll
-      for (int c = (i & ~1); c < N; c += 2) store2(&bc[c], rowA[c], rowA[c + 1]);
-      bc[N] = rc;
-    }
-    __syncwarp();
-    const T piv = bc[i];
-    if (piv == T(0) && info == 0) info = i + 1;
-    const T rinv = piv != T(0) ? bc[N] : T(0);
-    T u[N];
-#pragma unroll
-    for (int c = (i + 1) & ~1; c < N; c += 2) load2(&bc[c], u[c], u[c + 1]);
-    if (!done && lane != p) {
-      const T l = rowA[i] * rinv;
-      rowA[i] = l;
-#pragma unroll
-      for (int c = i + 1; c < N; ++c) rowA[c] = fma(-l, u[c], rowA[c]);
-    }
-    {  // border rows: multiplier from the lane holding column i of the row
-      const T ci = __shfl_sync(FULL, cb[i % CPL], (lane & ~(LPR - 1)) | (i / CPL));
-      const T l = ci * rinv;
-#pragma unroll
-      for (int q = 0; q < CPL; ++q) {
-        const int c = bc0 + q;
-        if (c == i) cb[q] = l;
-        else if (c > i) cb[q] = fma(-l, bc[c], cb[q]);
+    if (__popc(m) != 1 || !tc_plain_pivot<T>(hmax)) {  // exact tie, or zero, tiny, huge or no number
+      const unsigned pm = __reduce_min_sync(FULL, (m >> lane) & 1u ? (unsigned)mypos : 0xffffffffu);
+      m = __ballot_sync(FULL, ((m >> lane) & 1u) && (unsigned)mypos == pm);
+      rc = rcp_rn(rowA[i]);
+      const T pv = __shfl_sync(FULL, rowA[i], __ffs(m) - 1);
+      if (pv == T(0)) {
+        if (info == 0) info = i + 1;
+        rc = T(0);
       }
     }
-    if (lane == p) done = true;
+    const int p = __ffs(m) - 1;
+    const int pmin = __shfl_sync(FULL, mypos, p);
+    const bool isp = lane == p;
+    mypos = isp ? i : (mypos == i ? pmin : mypos);
+    T* prow = Gs + i * S::LDG;  // the pivot row [X | U], then its reciprocal
+    if (isp) {
+      prow[N] = rc;
+#pragma unroll
+      for (int c = 0; c < N; c += 2) store2(&prow[c], rowA[c], rowA[c + 1]);
+    }
     __syncwarp();
+    done = done || isp;
+    const T rinv = prow[N];
+    const T l = done ? T(0) : rowA[i] * rinv;
+    // the next column first: its search is what the next step waits for
+    if (i + 1 < N) rowA[i + 1] = fma(-l, prow[i + 1], rowA[i + 1]);
+#pragma unroll
+    for (int c = 0; c < N; c += 2) {
+      T u0, u1;
+      load2(&prow[c], u0, u1);
+      if (c != i && c != i + 1) rowA[c] = fma(-l, u0, rowA[c]);
+      if (c + 1 != i && c + 1 != i + 1) rowA[c + 1] = fma(-l, u1, rowA[c + 1]);
+    }
+    if (!done) rowA[i] = -l;
+    {  // border rows: multiplier from the lane holding column i of the row
+      const T ci = __shfl_sync(FULL, cb[i % CPL], (lane & ~(LPR - 1)) | (i / CPL));
+      const T lb = ci * rinv;
+#pragma unroll
+      for (int q = 0; q < CPL; ++q) {
+        const T v = fma(-lb, prow[bc0 + q], cb[q]);
+        cb[q] = (q == i % CPL && bc0 + q == i) ? -lb : v;
+      }
+    }
   }
   if (info != 0) {
     if (lane == 0) report(a.st, DEV_ZERO_PIVOT, j, info, k);
+    __syncwarp();
     return false;
   }
-  // panel factors T_j (L\U and M in getrf row order), pivots, C_j U^-1
+  // panel factors T_j in getrf row order (operator form: [L^-1 \ U; -M L^-1],
+  // the unit diagonal of L^-1 not stored), pivots, the border operator
+  // -C_j U^-1 L^-1; operator rows of the reduced and border rows for the product
   {
     T* Tj = a.Tm + (size_t)j * szT(d);
     if (act) {
 #pragma unroll
       for (int c = 0; c < N; ++c) Tj[(size_t)mypos + (size_t)c * n2] = rowA[c];
       rowof[mypos] = lane;
-    }
-    if (act) a.P[(size_t)j * szP(d) + mypos] = (unsigned char)lane;
-    if (blive) {
+      a.P[(size_t)j * szP(d) + mypos] = (unsigned char)lane;
+      if (mypos >= n) {
 #pragma unroll
-      for (int q = 0; q < CPL; ++q) a.C[(size_t)j * nrn + (size_t)(bc0 + q) * nr + br] = cb[q];
-    }
-    // rows of L (row m contiguous) for the triangular solve
-    if (act && mypos < n) {
-#pragma unroll
-      for (int c = 0; c < N; c += 2) store2(&Gs[mypos * S::LDG + c], rowA[c], rowA[c + 1]);
-    }
-  }
-  __syncwarp();
-  // ------------------------------------ phase 2: operator G (X L = R)
-  // R rows: identity for U-row positions, -M for reduced positions, -C' for border rows
-  {
-    T x[N];
-#pragma unroll
-    for (int c = 0; c < N; ++c) x[c] = (mypos < n) ? (c == mypos ? T(1) : T(0)) : -rowA[c];
-#pragma unroll
-    for (int q = 0; q < CPL; ++q) cb[q] = -cb[q];
-    // right-looking: once x[mm] is final, update every x[c], c < mm (the
-    // updates of one step are independent, so the dependent chain is N long)
-#pragma unroll
-    for (int mm = N - 1; mm > 0; --mm) {
-      const T xm = x[mm];
-      const T cm = __shfl_sync(FULL, cb[mm % CPL], (lane & ~(LPR - 1)) | (mm / CPL));
-      const T* Lrow = Gs + mm * S::LDG;  // L(mm, 0..mm-1)
-#pragma unroll
-      for (int c = 0; c < mm; c += 2) {
-        T l0, l1;
-        load2(&Lrow[c], l0, l1);
-        x[c] = fma(-xm, l0, x[c]);
-        if (c + 1 < mm) x[c + 1] = fma(-xm, l1, x[c + 1]);
+        for (int c = 0; c < N; c += 2) store2(&Gs[mypos * S::LDG + c], rowA[c], rowA[c + 1]);
       }
-#pragma unroll
-      for (int q = 0; q < CPL; ++q)
-        if (bc0 + q < mm) cb[q] = fma(-cm, Lrow[bc0 + q], cb[q]);
     }
-    __syncwarp();
-    if (act) {
-#pragma unroll
-      for (int c = 0; c < N; c += 2) store2(&Gs[mypos * S::LDG + c], x[c], x[c + 1]);
-    }
-    // border rows of G (zero for rows >= nr, and rows NRM..7 of the tile)
 #pragma unroll
     for (int q = 0; q < CPL; ++q) {
+      if (blive) a.C[(size_t)j * nrn + (size_t)(bc0 + q) * nr + br] = cb[q];
+      // border rows of G (zero for rows >= nr, and rows NRM..7 of the tile)
       Gs[(n2 + br) * S::LDG + bc0 + q] = blive ? cb[q] : T(0);
       if constexpr (NRM < 8) Gs[(n2 + NRM + br) * S::LDG + bc0 + q] = T(0);
     }
   }
   __syncwarp();
-  // ----------------------------------------- phase 3: the product
+  // ----------------------------------------- phase 2: the product
+  // G = [L^-1; -M L^-1; -C' L^-1] times (PW)_top: rows 0..N-1 of Gs hold L^-1
+  // below the diagonal and U from the diagonal on, so those fragments are masked
+  // to unit lower triangular (the tiles above the diagonal are skipped).
   // FP64 tensor cores (DMMA 8x8x4) for double, the FP32 pipe for float, with
   // the same accumulator layout; two passes over the column tiles keep the
   // accumulators within budget
@@ -960,7 +966,12 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
         }
 #pragma unroll
         for (int mt = 0; mt < S::MTILES; ++mt) {
-          const double afr = Gs[(mt * 8 + g) * S::LDG + ks * 4 + t];
+          if (mt * 8 < n && ks * 4 >= mt * 8 + 8) continue;  // above the diagonal of L^-1
+          double afr = Gs[(mt * 8 + g) * S::LDG + ks * 4 + t];
+          if (mt * 8 < n && ks * 4 + 3 >= mt * 8) {
+            const int dk = ks * 4 + t - (mt * 8 + g);
+            afr = dk < 0 ? afr : dk == 0 ? 1.0 : 0.0;
+          }
 #pragma unroll
           for (int ni = 0; ni < PC; ++ni)
             if (pass * PC + ni < S::NTILES) dmma_8x8x4(acc[mt][ni][0], acc[mt][ni][1], afr, bfr[ni]);
@@ -980,7 +991,11 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
         }
 #pragma unroll
         for (int mt = 0; mt < S::MTILES; ++mt) {
-          const T av = Gs[(mt * 8 + g) * S::LDG + kk];
+          T av = Gs[(mt * 8 + g) * S::LDG + kk];
+          if (mt * 8 < n) {
+            const int dk = kk - (mt * 8 + g);
+            av = dk < 0 ? av : dk == 0 ? T(1) : T(0);
+          }
 #pragma unroll
           for (int ni = 0; ni < PC; ++ni) {
             acc[mt][ni][0] = fma(av, bv[ni][0], acc[mt][ni][0]);
@@ -1245,10 +1260,6 @@ __global__ void __launch_bounds__(128, 4) k_factor_tree_tc(FactorArgs<double> a,
 // FP64 tensor cores (DMMA 8x8x4) for double, as a 3xTF32 split on the tensor
 // cores for float at n = 32, on the FP32 pipe for float at n = 16.
 // ---------------------------------------------------------------------------
-template <typename T> __device__ __forceinline__ T rcp_rn(T x);
-template <> __device__ __forceinline__ double rcp_rn<double>(double x) { return __drcp_rn(x); }
-template <> __device__ __forceinline__ float rcp_rn<float>(float x) { return __frcp_rn(x); }
-
 // total order of pivot candidates: (hi, lo) of |a|, NaN below every number,
 // finished rows below everything
 __device__ __forceinline__ void pivot_key(double av, bool done, unsigned& hi, unsigned& lo) {
@@ -2327,6 +2338,7 @@ struct SweepArgs {
   int ldx, nrhs;
   double* XB;
   int k, ldw, sel;
+  int op;           // T_j and C_j hold the operator form of the warp-per-pair LU kernel (launch argument)
   const int* done;  // batch, mixed path: nonzero once this system's refinement converged
 };
 
@@ -2859,7 +2871,8 @@ __global__ void __launch_bounds__(512, 1) k_backward_top(SweepArgs<T> a, int k_t
 // Forward sweep for LU factors, n = 8 or 16 (FP64 or FP32; single systems and
 // batch classes, see PipeItems): the pair arithmetic of k_forward_rows (lane = position r < 2n of the stacked
 // [x_jp; x_j], row map gathered by one shuffle, n broadcast steps of L and M,
-// xb partial -C'_j x_j), with the factors of the warp's NEXT pair (the 2n x n
+// xb partial -C'_j x_j; with the operator form, one matrix-vector product
+// whose terms do not depend on each other), with the factors of the warp's NEXT pair (the 2n x n
 // L\U and M block of T, and C_j) copied into shared memory by cp.async while
 // the current pair is computed, and the next pair's row-map entry read into a
 // register one pair ahead.  Two buffers per warp.
@@ -2897,6 +2910,7 @@ __global__ void __launch_bounds__(256, 2) k_forward_pipe(SweepArgs<T> a0, const 
   T* bufs = reinterpret_cast<T*>(smem_raw) + (size_t)warp * 2 * Bf::WORDS;
   const PipeItems<BATCH, T> items(a0, tab, map, ecnt, nent, wpb, warp);
   const int k = a0.k;
+  const bool op = a0.op != 0;
   // the row-map entry of a pair (read a pair ahead, into a register)
   auto row_src = [&](const SweepArgs<T>& a, long q) -> int {
     const int j = k + (int)(2L * k * q);
@@ -2935,17 +2949,25 @@ __global__ void __launch_bounds__(256, 2) k_forward_pipe(SweepArgs<T> a0, const 
       const T* buf = bufs + cur * Bf::WORDS;
       double t[N], cp[NRM];
 #pragma unroll
-      for (int c = 0; c < N; ++c) t[c] = (act && c < n) ? double(buf[c * n2 + lane]) : 0.0;
+      for (int c = 0; c < N; ++c) t[c] = (act && (!op || lane > c)) ? double(buf[c * n2 + lane]) : 0.0;
 #pragma unroll
       for (int r = 0; r < NRM; ++r) cp[r] = (lane < n && r < nr) ? double(buf[Bf::TT + lane * nr + r]) : 0.0;
       for (int col = 0; col < nrhs; ++col) {
         double* xc = a.x + (size_t)col * a.ldx;
         const double orig =
             col == 0 ? orig0 : (act ? (lane < n ? xc[(size_t)jp * n + lane] : xc[(size_t)j * n + lane - n]) : 0.0);
-        double w = __shfl_sync(FULL, orig, src);
+        const double b = __shfl_sync(FULL, orig, src);
+        double w = b, w2 = 0.0;
+        if (op) {  // one product with the operator: no serial chain
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-          if (i < n) {
+          for (int i = 0; i < N; i += 2) {
+            w = fma(t[i], __shfl_sync(FULL, b, i), w);
+            w2 = fma(t[i + 1], __shfl_sync(FULL, b, i + 1), w2);
+          }
+          w += w2;
+        } else {
+#pragma unroll
+          for (int i = 0; i < N; ++i) {
             const double wi = __shfl_sync(FULL, w, i);
             if (lane > i && act) w = fma(-t[i], wi, w);
           }
@@ -2954,12 +2976,13 @@ __global__ void __launch_bounds__(256, 2) k_forward_pipe(SweepArgs<T> a0, const 
           if (lane < n) xc[(size_t)j * n + lane] = w;
           else xc[(size_t)jp * n + lane - n] = w;
         }
-        const double wt = lane < n ? w : 0.0;
+        // operator form: -C' L^-1 times the permuted rows; else -C' times y
+        const double wt = lane < n ? (op ? b : -w) : 0.0;
 #pragma unroll
         for (int r = 0; r < NRM; ++r) {
           if (r < nr) {
             const double sr = warp_sum(cp[r] * wt);
-            if (lane == 0) a.XB[(size_t)j * nr * nrhs + (size_t)col * nr + r] = -sr;
+            if (lane == 0) a.XB[(size_t)j * nr * nrhs + (size_t)col * nr + r] = sr;
           }
         }
       }
@@ -4156,6 +4179,16 @@ struct FactorPlan {
   int tc_cols = 0;                                   // trailing-column capacity of tc
 };
 
+// the warp-per-pair LU kernel eliminates the pairs of this state (its factors
+// are in operator form, which the forward sweep has to know).  The tree and
+// gather schedules are FP64 only.
+static bool tc_pair_selected(const DevState& s) {
+  const Dims d = s.d;
+  if (s.sel != SEL_LU || d.nr > 8 || d.nx > 8 || (d.n != 16 && d.n != 8) || !s.use_tc) return false;
+  return s.pair_kernel == PAIR_AUTO || s.pair_kernel == PAIR_TC ||
+         (!s.mixed && (s.pair_kernel == PAIR_TREE || s.pair_kernel == PAIR_TC_GATHER));
+}
+
 template <typename T>
 static FactorPlan<T> plan_factor(const DevState& s) {
   const Dims d = s.d;
@@ -4170,9 +4203,7 @@ static FactorPlan<T> plan_factor(const DevState& s) {
            : s.sel == SEL_QR ? k_factor_level<T, SEL_QR> : k_factor_level<T, SEL_QRP>;
   if (p.smem <= SMEM_MAX) smem_limit_once(p.smem_k, p.smem);
   if constexpr (sizeof(T) == 8) {
-    if (s.sel == SEL_LU && d.nr <= 8 && d.nx <= 8 && (n == 16 || n == 8) && s.use_tc &&
-        (s.pair_kernel == PAIR_AUTO || s.pair_kernel == PAIR_TC || s.pair_kernel == PAIR_TREE ||
-         s.pair_kernel == PAIR_TC_GATHER)) {
+    if (tc_pair_selected(s)) {
       p.tc_smem = tc_smem_per_warp(n) * 4;
       // border rows spread over the warp: 8 lanes per row when nr <= 4, else 4
       const bool r4 = d.nr <= 4;
@@ -4204,8 +4235,7 @@ static FactorPlan<T> plan_factor(const DevState& s) {
   } else {
     // FP32 factors (mixed path): the same warp-per-pair kernel with FP32
     // products, level by level, no fused right-hand sides
-    if (s.sel == SEL_LU && d.nr <= 8 && d.nx <= 8 && (n == 16 || n == 8) && s.use_tc &&
-        (s.pair_kernel == PAIR_AUTO || s.pair_kernel == PAIR_TC)) {
+    if (tc_pair_selected(s)) {
       p.tc_smem = tc_smem_per_warp_t<T>(n) * 4;
       const bool r4 = d.nr <= 4;
       if (n == 16) p.tc = r4 ? k_factor_lu_tc<16, false, false, 4, T> : k_factor_lu_tc<16, false, false, 8, T>;
@@ -4404,6 +4434,7 @@ struct SweepPlan {
   // the backward top in one CTA
   void (*fwd_pipe)(SweepArgs<T>, const SweepArgs<T>*, const BatchCta*, const long*, long) = nullptr;
   size_t fwd_pipe_smem = 0;
+  int op = 0;  // the factors are in operator form
   void (*bwd_pipe)(SweepArgs<T>, const SweepArgs<T>*, const BatchCta*, const long*, long) = nullptr;
   size_t bwd_pipe_smem = 0;
   void (*bwd_top)(SweepArgs<T>, int, int) = nullptr;
@@ -4437,6 +4468,7 @@ static SweepPlan<T> plan_sweeps(const DevState& s) {
       p.fwd_pipe_smem = 8 * (r4 ? FwdBuf<8, 4, T>::BYTES : FwdBuf<8, 8, T>::BYTES);
     }
     smem_limit_once(p.fwd_pipe, p.fwd_pipe_smem);
+    p.op = tc_pair_selected(s);
   }
   if ((n == 16 || n == 8) && d.nx <= 8) {  // both precisions
     const bool x4 = d.nx <= 4;
@@ -4467,6 +4499,7 @@ static SweepArgs<T> sweep_args(DevState& s, const WorkSet<T>& w, double* x, int 
   a.d = s.d;
   a.D = w.D; a.E = w.E; a.B = w.B; a.C = w.C; a.Tm = w.Tm; a.P = s.P;
   a.x = x; a.ldx = ldx; a.nrhs = nrhs; a.XB = s.XB; a.sel = s.sel;
+  a.op = 0;
   a.done = nullptr;
   return a;
 }
@@ -4492,6 +4525,7 @@ static void forward_levels(DevState& s, const SweepPlan<T>& p, const WorkSet<T>&
   const Dims d = s.d;
   SweepArgs<T> a = sweep_args(s, w, x, ldx, nrhs);
   a.ldw = odd_ld(2 * d.n);
+  a.op = p.op;
   const size_t smem_f = (size_t)a.ldw * nrhs * 8 * WARPS_PANEL;
   smem_limit_once(k_forward_level<T>, smem_f);
   for (int K = 1; K < d.nblock; K *= 2) {
@@ -5630,6 +5664,7 @@ static void batch_sweeps_rows(BatchClass& c, cudaStream_t st, bool forward, int 
   const bool r4 = c.nrm <= 4, x4 = c.nxm <= 4;
   SweepArgs<T> a0{};
   a0.k = 1 << L;
+  a0.op = c.fam == PAIR_TC;
   if constexpr (N == 8 || N == 16) {
     if (c.n == N) {  // pipelined: a fixed grid walks the level's map entries
       const long nent = c.scnt[L];

@@ -1,0 +1,73 @@
+"""GPU tests of the pair kernels at the sizes and values where they can go
+wrong, against the CPU oracle.
+
+Bar: forward error against the oracle's solution <= 1e-10, the bar of the other
+parity tests.  Both sides solve the same system backward stably, so they differ
+by cond(A) * 2^-53 times a modest power of n; cond(A) of these systems is at
+most 6e3 (dense SVD), which gives 7e-13 times that power."""
+import numpy as np
+import pytest
+
+from alglin_b200 import bcr as B
+from alglin_b200 import synth
+from oracle import pyoracle as po
+from tests._util import fwd_err
+
+pytestmark = pytest.mark.gpu
+
+
+def solve_both(s, rhs, select="LU"):
+    """Solutions of the library (factorize, then solve), of the library in one
+    factorize + solve, and of the oracle."""
+    o = po.Oracle(s, select, "LU")
+    assert o.factorize(), o.last_error()
+    xo = o.solve(rhs)
+    out = []
+    for fused in (False, True):
+        h = B.BorderedCR()
+        h.load_system(s)
+        h.select(select)
+        h.select_last("LU")
+        x = rhs.copy()
+        if fused:
+            assert h.factorize_solve(x.shape[0], x.reshape(-1), x.shape[1]), h.last_error()
+        else:
+            assert h.factorize(), h.last_error()
+            assert h.solve_n(x.shape[0], x.reshape(-1), x.shape[1]), h.last_error()
+        out.append(x)
+    return out[0], out[1], xo
+
+
+def check(s, rhs, select="LU", bar=1e-10):
+    x1, x2, xo = solve_both(s, rhs, select)
+    for x in (x1, x2):
+        for c in range(rhs.shape[0]):
+            assert fwd_err(x[c, :s.ncols], xo[c, :s.ncols]) < bar
+
+
+@pytest.mark.parametrize("n", [8, 16])
+@pytest.mark.parametrize("exponent", [0, -1021, 1010])
+def test_pivots_of_every_magnitude(n, exponent):
+    """Block rows scaled by 2^exponent, to about the ends of the range in which the
+    oracle itself stays finite.  At 2^-1021 the intermediate values are rounded
+    to 2^-53 of the entries at worst, so the bar stands."""
+    s = synth.collocation(37, n, 1, 1, 3, 3, seed=5)
+    for a in (s.D, s.E, s.B):
+        np.ldexp(a, exponent, out=a)
+    rhs = synth.rhs(s, 2, seed=6)
+    rhs[:, :s.n * s.nblock] = np.ldexp(rhs[:, :s.n * s.nblock], exponent)
+    check(s, rhs)
+
+
+@pytest.mark.parametrize("n", [8, 16])
+@pytest.mark.parametrize("nblock", [2, 3, 33])
+def test_pivot_ties_follow_getrf(n, nblock):
+    """Entries of +-1 and +-1/2 only: many candidates of exactly equal
+    magnitude, where getrf takes the first position.  The oracle applies that
+    rule, so a different choice would show as another rounding, not as an
+    error; cond(A) <= 2e4 here, so the bar is 1e-8, whichever row wins."""
+    s = synth.dominant(nblock, n, 0, 0, 2, 2, seed=3)
+    rng = np.random.default_rng(7)
+    s.D[:] = rng.choice([-1.0, -0.5, 0.5, 1.0], s.D.shape)
+    s.E[:] = rng.choice([-1.0, -0.5, 0.5, 1.0], s.E.shape)
+    check(s, synth.rhs(s, 1, seed=8), bar=1e-8)
