@@ -1732,15 +1732,14 @@ __global__ void __launch_bounds__(2 * N + 32, grp_min_blocks<T, N>())
 }
 
 // ---------------------------------------------------------------------------
-// Large blocks, LU: blocked right-looking elimination of the pair's work
-// matrix (one CTA per pair, the matrix in the CTA's global slab, L2
+// Large blocks, FP32 LU where the tensor-core kernel does not apply: blocked
+// right-looking elimination of the pair's work matrix (one CTA per pair, the matrix in the CTA's global slab, L2
 // resident).  The panel columns go in blocks of BLK_W: a block is factored in
 // shared memory with the getrf pivot rule (border rows eliminated, never
 // pivots), its row interchanges are applied to every other column, the
 // BLK_W rows of the trailing columns are solved with the block's unit lower
 // triangle, and the rows below are updated with one product of depth BLK_W
-// -- FP64 tensor cores (DMMA 8x8x4) for double, FMA tiles for float.  The
-// result equals the unblocked elimination (getrf on the panel followed by
+// (FMA tiles).  FP64 blocks go to k_factor_lu_lub.  The result equals the unblocked elimination (getrf on the panel followed by
 // the trailing updates) up to rounding order.
 // ---------------------------------------------------------------------------
 constexpr int BLK_W = 32;
@@ -1749,91 +1748,35 @@ constexpr int LAST_BLOCKED_MIN = 64;  // last blocks of this order and above: bl
 
 // W[c*R + rowp[r]] -= sum_m L[m*LD + r] * W[c*R + rowp[k0 + m]] for positions r in
 // [r0, R), c in [c0, NC), m < w; L: the factored block in shared memory (column m,
-// position r); rowp: position -> row of W
+// position r); rowp: position -> row of W.  4 x 4 outputs per thread.
 template <typename T>
 __device__ void blk_update(T* W, int R, int NC, const T* Lsm, int LD, int k0, int w, int r0, int c0,
                            const int* rowp) {
   const int tid = threadIdx.x, bs = blockDim.x;
   const int rows = R - r0, cols = NC - c0;
   if (rows <= 0 || cols <= 0) return;
-  if constexpr (sizeof(T) == 8) {
-    // 16 x 16 output per warp iteration (2 x 2 DMMA tiles)
-    const int lane = tid & 31, warp = tid >> 5, nw = bs >> 5;
-    const int g = lane >> 2, q = lane & 3;
-    const int tr = (rows + 15) / 16, tc = (cols + 15) / 16;
-    constexpr int KS = BLK_W / 4;
-    for (int t = warp; t < tr * tc; t += nw) {
-      const int rb = r0 + (t % tr) * 16, cb = c0 + (t / tr) * 16;
-      // every global load of the tile (B fragments, C) is in flight at once
-      double bf[KS][2], cv[2][2][2];
-#pragma unroll
-      for (int ks = 0; ks < KS; ++ks) {
-        const int m = ks * 4 + q;
-#pragma unroll
-        for (int v = 0; v < 2; ++v) {
-          const int c = cb + v * 8 + g;
-          bf[ks][v] = (m < w && c < NC) ? W[(size_t)c * R + rowp[k0 + m]] : 0.0;
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int v = 0; v < 2; ++v)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int r = rb + u * 8 + g, c = cb + v * 8 + 2 * q + h;
-            cv[u][v][h] = (r < R && c < NC) ? W[(size_t)c * R + rowp[r]] : 0.0;
-          }
-      double acc[2][2][2] = {};
-#pragma unroll
-      for (int ks = 0; ks < KS; ++ks) {
-        const int m = ks * 4 + q;
-        double af[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int r = rb + u * 8 + g;
-          af[u] = (m < w && r < R) ? Lsm[(size_t)m * LD + r] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-#pragma unroll
-          for (int v = 0; v < 2; ++v) dmma_8x8x4(acc[u][v][0], acc[u][v][1], af[u], bf[ks][v]);
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int v = 0; v < 2; ++v)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int r = rb + u * 8 + g, c = cb + v * 8 + 2 * q + h;
-            if (r < R && c < NC) W[(size_t)c * R + rowp[r]] = cv[u][v][h] - acc[u][v][h];
-          }
-    }
-  } else {
-    // 4 x 4 output per thread
-    const int tr = (rows + 3) / 4, tc = (cols + 3) / 4;
-    for (int t = tid; t < tr * tc; t += bs) {
-      const int rb = r0 + (t % tr) * 4, cb = c0 + (t / tr) * 4;
-      T acc[4][4] = {};
+  const int tr = (rows + 3) / 4, tc = (cols + 3) / 4;
+  for (int t = tid; t < tr * tc; t += bs) {
+    const int rb = r0 + (t % tr) * 4, cb = c0 + (t / tr) * 4;
+    T acc[4][4] = {};
 #pragma unroll 4
-      for (int m = 0; m < w; ++m) {
-        T av[4], bv[4];
+    for (int m = 0; m < w; ++m) {
+      T av[4], bv[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          av[u] = rb + u < R ? Lsm[(size_t)m * LD + rb + u] : T(0);
-          bv[u] = cb + u < NC ? W[(size_t)(cb + u) * R + rowp[k0 + m]] : T(0);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) acc[u][v] = fma(av[u], bv[v], acc[u][v]);
+      for (int u = 0; u < 4; ++u) {
+        av[u] = rb + u < R ? Lsm[(size_t)m * LD + rb + u] : T(0);
+        bv[u] = cb + u < NC ? W[(size_t)(cb + u) * R + rowp[k0 + m]] : T(0);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int v = 0; v < 4; ++v)
-          if (rb + u < R && cb + v < NC) W[(size_t)(cb + v) * R + rowp[rb + u]] -= acc[u][v];
+        for (int v = 0; v < 4; ++v) acc[u][v] = fma(av[u], bv[v], acc[u][v]);
     }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        if (rb + u < R && cb + v < NC) W[(size_t)(cb + v) * R + rowp[rb + u]] -= acc[u][v];
   }
 }
 
@@ -2338,7 +2281,7 @@ struct SweepArgs {
   int ldx, nrhs;
   double* XB;
   int k, ldw, sel;
-  int op;           // T_j and C_j hold the operator form of the warp-per-pair LU kernel (launch argument)
+  int op;           // T_j and C_j hold the operator form, by blocks of op columns (launch argument; 0: L and M)
   const int* done;  // batch, mixed path: nonzero once this system's refinement converged
 };
 
@@ -2347,6 +2290,8 @@ __device__ __forceinline__ bool system_active(const SweepArgs<T>& a) { return !(
 
 __device__ __forceinline__ void take_level(SweepArgs<float>& a, const SweepArgs<float>& a0) { a.k = a0.k; }
 __device__ __forceinline__ void take_level(SweepArgs<double>& a, const SweepArgs<double>& a0) { a.k = a0.k; }
+
+#include "bcr_lub.cuh"
 
 template <typename T, bool BATCH = false>
 __global__ void __launch_bounds__(WARPS_PANEL * 32) k_forward_level(SweepArgs<T> a0, const SweepArgs<T>* tab,
@@ -3927,25 +3872,20 @@ __global__ void k_last_factor(Dims d, LastBufs b, int sel_last, StatusWords* st)
 // load_and_factorize_last with LU for larger blocks (cc:1319-1346, getrf): the
 // blocked elimination of the pair kernels on the whole block, FP64 tensor-core
 // products, rows left in place (kind FACT_LU_ROWS, piv[pos] = row)
-__global__ void __launch_bounds__(256, 1) k_last_lu_blocked(Dims d, LastBufs b, StatusWords* st) {
+template <int NB>
+__global__ void __launch_bounds__(512, 1) k_last_lu_blocked(Dims d, LastBufs b, StatusWords* st, int bw) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double sv[32];
-  __shared__ int si[32];
-  __shared__ int s_perm[BLK_ROWS_MAX];
+  __shared__ LubShared<512> sh;
   const int N = d.Nc, tid = threadIdx.x;
-  if (d.Nr != N || N > BLK_ROWS_MAX) {
+  if (d.Nr != N || N > LUB_ROWS_MAX) {
     if (tid == 0) report(st, DEV_BAD_SHAPE, -1, 0, -1);
     return;
   }
-  for (int r = tid; r < N; r += blockDim.x) s_perm[r] = r;
-  __syncthreads();
-  double* Pb = reinterpret_cast<double*>(smem_raw);
-  const int info = blk_eliminate<double>(b.A, N, N, N, N, Pb, s_perm, sv, si);
+  const int info = lub_square<NB>(sh, reinterpret_cast<double*>(smem_raw), b.A, N, bw, b.piv);
   if (info != 0) {
     if (tid == 0) report(st, DEV_LAST_SINGULAR, -1, info, -1);
     return;
   }
-  for (int r = tid; r < N; r += blockDim.x) b.piv[r] = s_perm[r];
   if (tid == 0) st->kind = FACT_LU_ROWS;
 }
 
@@ -4066,7 +4006,7 @@ __global__ void k_mv_tail(Dims d, const double* H, const double* Cq, const doubl
 // later calls (for instance inside a CUDA graph capture) only launch.
 template <typename K>
 static void smem_limit_once(K* kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return;
+  if (bytes <= 32 * 1024) return;  // 48 KB less what a kernel may hold statically
   static const void* keys[64];
   static size_t done[64];
   static int used = 0;
@@ -4154,11 +4094,19 @@ static WorkSet<float> work_set(DevState& s, float*) {
 // ---------------------------------------------------------------------------
 // pair-kernel choice for the factorization
 // ---------------------------------------------------------------------------
+using LubKernel = void (*)(FactorArgs<double>, double*, size_t, int);
+static LubKernel lub_kernel(const LubPlan& p) {
+  if (p.threads == 256)
+    return p.depth == 32 ? k_factor_lu_lub<256, 4> : p.depth == 48 ? k_factor_lu_lub<256, 6> : k_factor_lu_lub<256, 8>;
+  return p.depth == 32 ? k_factor_lu_lub<512, 4> : p.depth == 48 ? k_factor_lu_lub<512, 6> : k_factor_lu_lub<512, 8>;
+}
+
 template <typename T>
 struct FactorPlan {
   void (*cta)(FactorArgs<T>, T*, size_t) = nullptr;  // CTA per pair (large n)
-  void (*blk)(FactorArgs<T>, T*, size_t) = nullptr;  // CTA per pair, blocked LU (large n)
+  void (*blk)(FactorArgs<T>, T*, size_t) = nullptr;  // CTA per pair, blocked LU (large n, FP32)
   size_t blk_smem = 0;
+  LubPlan lub;                                       // CTA or cluster per pair, blocked LU (large n, FP64)
   void (*umma)(FactorArgs<T>, T*, size_t) = nullptr;  // CTA per pair, tcgen05 products (FP32, large n)
   size_t umma_smem = 0;
   void (*tc)(FactorArgs<T>, const FactorArgs<T>*, const BatchCta*) = nullptr;               // tensor-core LU (FP64, n = 8, 16)
@@ -4270,11 +4218,16 @@ static FactorPlan<T> plan_factor(const DevState& s) {
       (s.pair_kernel != PAIR_SMEM || !smem_fits)) {
     p.cta = s.sel == SEL_LU ? k_factor_cta<T, SEL_LU>
           : s.sel == SEL_QR ? k_factor_cta<T, SEL_QR> : k_factor_cta<T, SEL_QRP>;
-    const size_t bsm = (size_t)BLK_W * (2 * n + d.nr) * sizeof(T);
-    if (s.sel == SEL_LU && n <= 128 && 2 * n + d.nr <= BLK_ROWS_MAX && bsm <= SMEM_MAX) {
-      p.blk = k_factor_lu_blocked<T>;
-      p.blk_smem = bsm;
-      smem_limit_once(p.blk, bsm);
+    if constexpr (sizeof(T) == 8) {
+      p.lub = s.sel == SEL_LU ? lub_plan(2 * n + d.nr, n, false) : LubPlan{};
+      if (p.lub.threads) smem_limit_once(lub_kernel(p.lub), p.lub.smem);
+    } else {
+      const size_t bsm = (size_t)BLK_W * (2 * n + d.nr) * sizeof(T);
+      if (s.sel == SEL_LU && n <= 128 && 2 * n + d.nr <= BLK_ROWS_MAX && bsm <= SMEM_MAX) {
+        p.blk = k_factor_lu_blocked<T>;
+        p.blk_smem = bsm;
+        smem_limit_once(p.blk, bsm);
+      }
     }
     if constexpr (sizeof(T) == 4) {
       if (s.sel == SEL_LU && umma_fits(d) && (s.pair_kernel == PAIR_AUTO || s.pair_kernel == PAIR_UMMA)) {
@@ -4292,6 +4245,29 @@ template <typename T>
 static int fusable_rhs(const DevState& s, const FactorPlan<T>& p, int nrhs) {
   if (!p.tc || nrhs < 1 || nrhs > 16) return 0;
   return 2 * s.d.n + s.d.nx + nrhs <= p.tc_cols ? nrhs : 0;
+}
+
+// One level of k_factor_lu_lub.  Where the level has fewer pairs than CTAs fit
+// on the GPU, the trailing columns of a pair are split over a cluster of 2, 4 or
+// 8 CTAs (at least 24 columns each: every CTA repeats the panel).
+static void launch_lub(const FactorArgs<double>& a, double* slab, size_t slab_elems, const LubPlan& p, long np,
+                       cudaStream_t st) {
+  const long ctas = 148L * (512 / p.threads);
+  const int trail = 2 * a.d.n + a.d.nx;
+  int slices = 1;
+  while (slices < LUB_SLICES_MAX && np * slices * 2 <= ctas && trail >= slices * 2 * 24) slices *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(slices > 1 ? np * slices : std::min(np, ctas)));
+  cfg.blockDim = dim3((unsigned)p.threads);
+  cfg.dynamicSmemBytes = p.smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)slices;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, lub_kernel(p), a, slab, slab_elems, p.bw);
 }
 
 // every CR level: pair eliminations and the C_jpp border fix-up.  Returns true
@@ -4363,7 +4339,9 @@ static bool factor_levels(DevState& s, const FactorPlan<T>& p, const WorkSet<T>&
       }
     }
     if (p.umma) p.umma<<<grid_for(np, 1, 148), UM_NT, p.umma_smem, st>>>(a, w.slab, s.slab_elems);
-    else if (p.blk) p.blk<<<grid_for(np, 1, s.slab_ctas), 256, p.blk_smem, st>>>(a, w.slab, s.slab_elems);
+    else if (p.lub.threads) {
+      if constexpr (sizeof(T) == 8) launch_lub(a, w.slab, s.slab_elems, p.lub, np, st);
+    } else if (p.blk) p.blk<<<grid_for(np, 1, s.slab_ctas), 256, p.blk_smem, st>>>(a, w.slab, s.slab_elems);
     else if (p.cta) p.cta<<<grid_for(np, 1, s.slab_ctas), 256, 0, st>>>(a, w.slab, s.slab_elems);
     else if (p.grp) p.grp<<<grid_for(np, 1, p.grp_ctas), p.grp_threads, p.grp_smem, st>>>(a, nullptr, nullptr);
     else if (p.tc) p.tc<<<grid_for(np, 4, 148 * 16), 128, p.tc_smem, st>>>(a, nullptr, nullptr);
@@ -4393,10 +4371,11 @@ static void factor_last(DevState& s, const WorkSet<T>& w, cudaStream_t st, bool 
     cudaMemcpyAsync(s.Al, s.Hl, (size_t)d.Nr * d.Nc * 8, cudaMemcpyDeviceToDevice, st);
   }
   const LastBufs lb = last_bufs(s);
-  if (s.sel_last == LAST_LU && d.Nr == d.Nc && d.Nc >= LAST_BLOCKED_MIN && d.Nc <= BLK_ROWS_MAX) {
-    const size_t sm = (size_t)BLK_W * d.Nc * sizeof(double);
-    smem_limit_once(k_last_lu_blocked, sm);
-    k_last_lu_blocked<<<1, 256, sm, st>>>(d, lb, s.st);
+  const LubPlan lp = lub_plan(d.Nc, d.Nc, true);
+  if (s.sel_last == LAST_LU && d.Nr == d.Nc && d.Nc >= LAST_BLOCKED_MIN && lp.threads) {
+    auto* kern = lp.depth == 32 ? k_last_lu_blocked<4> : lp.depth == 48 ? k_last_lu_blocked<6> : k_last_lu_blocked<8>;
+    smem_limit_once(kern, lp.smem);
+    kern<<<1, 512, lp.smem, st>>>(d, lb, s.st, lp.bw);
     check_launch("k_last_lu_blocked");
   } else if (s.sel_last == LAST_LU && d.Nr == d.Nc && d.Nc <= LAST_SMALL) {
     k_last_lu_small<<<1, 256, 0, st>>>(d, lb, s.st);
@@ -4434,11 +4413,12 @@ struct SweepPlan {
   // the backward top in one CTA
   void (*fwd_pipe)(SweepArgs<T>, const SweepArgs<T>*, const BatchCta*, const long*, long) = nullptr;
   size_t fwd_pipe_smem = 0;
-  int op = 0;  // the factors are in operator form
+  int op = 0;  // the factors are in operator form, by blocks of op columns
   void (*bwd_pipe)(SweepArgs<T>, const SweepArgs<T>*, const BatchCta*, const long*, long) = nullptr;
   size_t bwd_pipe_smem = 0;
   void (*bwd_top)(SweepArgs<T>, int, int) = nullptr;
   void (*fwd_cta)(SweepArgs<T>, const SweepArgs<T>*, const BatchCta*) = nullptr;  // CTA per pair (large n)
+  bool fwd_op = false;  // k_forward_op (the blocked FP64 kernel's operator form)
   void (*bwd_cta)(SweepArgs<T>, const SweepArgs<T>*, const BatchCta*) = nullptr;
 };
 
@@ -4468,7 +4448,6 @@ static SweepPlan<T> plan_sweeps(const DevState& s) {
       p.fwd_pipe_smem = 8 * (r4 ? FwdBuf<8, 4, T>::BYTES : FwdBuf<8, 8, T>::BYTES);
     }
     smem_limit_once(p.fwd_pipe, p.fwd_pipe_smem);
-    p.op = tc_pair_selected(s);
   }
   if ((n == 16 || n == 8) && d.nx <= 8) {  // both precisions
     const bool x4 = d.nx <= 4;
@@ -4489,6 +4468,15 @@ static SweepPlan<T> plan_sweeps(const DevState& s) {
   } else if (n > 16 && n <= SWP_MAXN) {
     if (s.sel == SEL_LU) p.fwd_cta = k_forward_cta<T>;
     p.bwd_cta = k_backward_cta<T>;
+  }
+  // the form of the factors follows the kernel that made them
+  const FactorPlan<T> fp = plan_factor<T>(s);
+  if (fp.tc) p.op = n;
+  if constexpr (sizeof(T) == 8) {
+    if (fp.lub.threads) {
+      p.op = fp.lub.bw;
+      p.fwd_op = true;
+    }
   }
   return p;
 }
@@ -4531,7 +4519,9 @@ static void forward_levels(DevState& s, const SweepPlan<T>& p, const WorkSet<T>&
   for (int K = 1; K < d.nblock; K *= 2) {
     a.k = K;
     const long np = pairs_at_level(d.nblock, K);
-    if (p.fwd_pipe)
+    if (p.fwd_op) {
+      if constexpr (sizeof(T) == 8) k_forward_op<<<grid_for(np, 1, 148 * 4), FWD_OP_NT, 0, st>>>(a);
+    } else if (p.fwd_pipe)
       p.fwd_pipe<<<grid_for(np, 8, 148 * 2), 256, p.fwd_pipe_smem, st>>>(a, nullptr, nullptr, nullptr, 0);
     else if (p.fwd_cta) p.fwd_cta<<<grid_for(np, 1, 148 * 8), 256, 0, st>>>(a, nullptr, nullptr);
     else if (p.fwd) p.fwd<<<grid_for(np, 8, 148 * 32), 256, 0, st>>>(a, nullptr, nullptr, nullptr);
@@ -5664,7 +5654,7 @@ static void batch_sweeps_rows(BatchClass& c, cudaStream_t st, bool forward, int 
   const bool r4 = c.nrm <= 4, x4 = c.nxm <= 4;
   SweepArgs<T> a0{};
   a0.k = 1 << L;
-  a0.op = c.fam == PAIR_TC;
+  a0.op = c.fam == PAIR_TC ? c.n : 0;
   if constexpr (N == 8 || N == 16) {
     if (c.n == N) {  // pipelined: a fixed grid walks the level's map entries
       const long nent = c.scnt[L];

@@ -71,3 +71,17 @@ def test_pivot_ties_follow_getrf(n, nblock):
     s.D[:] = rng.choice([-1.0, -0.5, 0.5, 1.0], s.D.shape)
     s.E[:] = rng.choice([-1.0, -0.5, 0.5, 1.0], s.E.shape)
     check(s, synth.rhs(s, 1, seed=8), bar=1e-8)
+
+
+@pytest.mark.parametrize("n,nr,nx", [(25, 0, 0), (32, 9, 9), (33, 1, 2), (40, 3, 3), (63, 5, 5), (64, 8, 8), (65, 2, 2),
+                                     (72, 0, 0), (100, 17, 17), (127, 4, 4), (128, 16, 16)])
+@pytest.mark.parametrize("nblock", [2, 3, 37])
+def test_large_block_lu(n, nr, nx, nblock):
+    """The blocked FP64 kernel at the edges of its tiles: block widths that are no
+    multiple of 8 or 16, one and two panel blocks, no borders and borders that
+    pass a tile, one pair (columns split over a cluster) and many.  cond(A) is at
+    most 3e4 here (dense SVD), so the bar is 1e-9: 3e4 * 2^-53 * 256 rows."""
+    qx = max(0, nr - nx)
+    qr = max(0, nx - nr)
+    s = synth.collocation(nblock, n, qr, qx, nr, nx, seed=n)
+    check(s, synth.rhs(s, 3, seed=n + 1), bar=1e-9)
