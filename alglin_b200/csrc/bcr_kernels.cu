@@ -2197,6 +2197,25 @@ __global__ void __launch_bounds__(256) k_factor_cta(FactorArgs<T> a, T* slab, si
   }
 }
 
+// Element of a batch of loads, 0 where p is false.  volatile keeps the loads of
+// an unrolled batch together: scheduled by the compiler, each one waits for the
+// use of the one before (the same 262 KB read by one CTA: 80,000 cycles from
+// DRAM, against 13,000).
+__device__ __forceinline__ double ld_batch(bool p, const double* a) {
+  double v;
+  asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; mov.f64 %0, 0d0000000000000000; @q ld.global.f64 %0, [%1]; }\n"
+               : "=d"(v)
+               : "l"(a), "r"((unsigned)p));
+  return v;
+}
+__device__ __forceinline__ float ld_batch(bool p, const float* a) {
+  float v;
+  asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; mov.f32 %0, 0f00000000; @q ld.global.f32 %0, [%1]; }\n"
+               : "=f"(v)
+               : "l"(a), "r"((unsigned)p));
+  return v;
+}
+
 // copy of loaded FP64 blocks into the working precision
 template <typename T>
 __global__ void k_convert_blocks(const double* src, T* dst, size_t count) {
@@ -2236,13 +2255,18 @@ __device__ void reduce_tree_body(const T* buf, int stride, long first, long coun
   const long b0 = first + (long)blk * chunk;
   const long b1 = min(first + count, b0 + chunk);
   T a0 = T(0), a1 = T(0);
-  if (g < S) {
-    long b = b0 + g;
-    for (; b + S < b1; b += 2 * S) {
-      a0 += buf[(size_t)b * stride + e];
-      a1 += buf[(size_t)(b + S) * stride + e];
+  if (g < S) {  // eight loads in flight
+    const T* p = buf + e;
+    for (long b = b0 + g; b < b1; b += 8 * S) {
+      T v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = ld_batch(b + u * S < b1, p + (size_t)(b + u * S) * stride);
+#pragma unroll
+      for (int u = 0; u < 8; u += 2) {
+        a0 += v[u];
+        a1 += v[u + 1];
+      }
     }
-    if (b < b1) a0 += buf[(size_t)b * stride + e];
   }
   red[tid] = a0 + a1;
   __syncthreads();
@@ -3050,188 +3074,7 @@ __global__ void __launch_bounds__(256, 2) k_backward_rows32(SweepArgs<TF> a0, co
 // values of the pair in shared memory, the triangular solves blocked by 32
 // rows (one warp solves a diagonal block with shuffles, the CTA applies it to
 // the rows that follow)
-// ---------------------------------------------------------------------------
-constexpr int SWP_MAXN = 128;
-
-template <typename TF, bool BATCH = false>
-__global__ void __launch_bounds__(256) k_forward_cta(SweepArgs<TF> a0, const SweepArgs<TF>* tab,
-                                                     const BatchCta* cmap) {
-  constexpr unsigned FULL = 0xffffffffu;
-  __shared__ double w[2 * SWP_MAXN];
-  __shared__ double tb[32][33];  // diagonal 32 x 32 block of the triangle
-  const int tid = threadIdx.x, bs = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  SweepArgs<TF> ab;
-  long q0, q1, qs;
-  pair_range<BATCH>(a0, tab, cmap, 1, 0, ab, q0, q1, qs);
-  const SweepArgs<TF>& a = BATCH ? ab : a0;
-  const Dims d = a.d;
-  const int n = d.n, n2 = 2 * n, nr = d.nr, nrhs = a.nrhs, k = a.k;
-  for (long q = q0; q < q1; q += qs) {
-    const int j = k + (int)(2L * k * q), jp = j - k;
-    const TF* Tj = a.Tm + (size_t)j * szT(d);
-    const unsigned char* Pj = a.P + (size_t)j * szP(d);
-    const TF* Cj = a.C + (size_t)j * nr * n;
-    for (int col = 0; col < nrhs; ++col) {
-      double* xc = a.x + (size_t)col * a.ldx;
-      __syncthreads();  // w of the previous column / pair is no longer read
-      for (int pos = tid; pos < n2; pos += bs) {
-        const int r = Pj[pos];  // original row at this position
-        w[pos] = r < n ? xc[(size_t)jp * n + r] : xc[(size_t)j * n + (r - n)];
-      }
-      __syncthreads();
-      // unit lower L on positions [0, n), then the rows below: w -= T(:, c) w[c]
-      for (int cb = 0; cb < n; cb += 32) {
-        const int cw = n - cb < 32 ? n - cb : 32;
-        // the diagonal block of L through shared memory (one coalesced load)
-        for (int e = tid; e < cw * 32; e += bs) {
-          const int c = e >> 5, r = e & 31;
-          tb[c][r] = r < cw ? double(Tj[(size_t)(cb + c) * n2 + cb + r]) : 0.0;
-        }
-        __syncthreads();
-        if (warp == 0) {
-          double v = lane < cw ? w[cb + lane] : 0.0;
-          for (int c = 0; c < cw; ++c) {
-            const double vc = __shfl_sync(FULL, v, c);
-            if (lane > c && lane < cw) v = fma(-tb[c][lane], vc, v);
-          }
-          if (lane < cw) w[cb + lane] = v;
-        }
-        __syncthreads();
-        for (int r = cb + cw + tid; r < n2; r += bs) {
-          double s = w[r];
-          for (int c0 = 0; c0 < cw; c0 += 8) {  // 8 loads in flight
-            double tv[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) tv[u] = c0 + u < cw ? double(Tj[(size_t)(cb + c0 + u) * n2 + r]) : 0.0;
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-              if (c0 + u < cw) s = fma(-tv[u], w[cb + c0 + u], s);
-          }
-          w[r] = s;
-        }
-        __syncthreads();
-      }
-      for (int pos = tid; pos < n2; pos += bs) {
-        if (pos < n) xc[(size_t)j * n + pos] = w[pos];
-        else xc[(size_t)jp * n + pos - n] = w[pos];
-      }
-      // xb contribution of this pair: -C'_j w[0, n)
-      for (int r = warp; r < nr; r += bs >> 5) {
-        double sr = 0.0;
-        for (int c = lane; c < n; c += 32) sr = fma(double(Cj[(size_t)c * nr + r]), w[c], sr);
-        sr = warp_sum(sr);
-        if (lane == 0) a.XB[(size_t)j * nr * nrhs + (size_t)col * nr + r] = -sr;
-      }
-    }
-  }
-}
-
-template <typename TF, bool BATCH = false>
-__global__ void __launch_bounds__(256) k_backward_cta(SweepArgs<TF> a0, const SweepArgs<TF>* tab,
-                                                      const BatchCta* cmap) {
-  constexpr unsigned FULL = 0xffffffffu;
-  __shared__ double xa[SWP_MAXN], xz[SWP_MAXN], y[SWP_MAXN];
-  __shared__ double part[256];
-  __shared__ double tb[32][33];  // diagonal 32 x 32 block of the triangle
-  const int tid = threadIdx.x, bs = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  SweepArgs<TF> ab;
-  long q0, q1, qs;
-  pair_range<BATCH>(a0, tab, cmap, 1, 0, ab, q0, q1, qs);
-  const SweepArgs<TF>& a = BATCH ? ab : a0;
-  const Dims d = a.d;
-  const int n = d.n, n2 = 2 * n, nx = d.nx, nb = d.nblock, nrhs = a.nrhs, k = a.k;
-  const bool qrp = a.sel == SEL_QRP;
-  const size_t xb_off = (size_t)(nb + 1) * n + d.qx;
-  const size_t nn = (size_t)n * n;
-  const int G = bs / n;  // threads per row in the product (n <= 128: G >= 2)
-  for (long q = q0; q < q1; q += qs) {
-    const int j = k + (int)(2L * k * q), jp = j - k, jpp = min(j + k, nb);
-    const TF* Dj = a.D + (size_t)j * nn;
-    const TF* Ej = a.E + (size_t)j * nn;
-    const TF* Bj = a.B + (size_t)j * n * nx;
-    const TF* Tj = a.Tm + (size_t)j * szT(d);
-    for (int col = 0; col < nrhs; ++col) {
-      double* xc = a.x + (size_t)col * a.ldx;
-      __syncthreads();
-      for (int i = tid; i < n; i += bs) {
-        xa[i] = xc[(size_t)jp * n + i];
-        xz[i] = xc[(size_t)jpp * n + i];
-      }
-      __syncthreads();
-      // y = x_j - D'_j x_jp - E'_j x_jpp - B'_j xb, G threads per row, fixed order
-      {
-        const int i = tid % n, g = tid / n;
-        double s = 0.0;
-        if (g < G) {
-          for (int c0 = g; c0 < n; c0 += 4 * G) {  // 8 loads in flight
-            double dv[4], ev[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int c = c0 + u * G;
-              dv[u] = c < n ? double(Dj[(size_t)c * n + i]) : 0.0;
-              ev[u] = c < n ? double(Ej[(size_t)c * n + i]) : 0.0;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int c = c0 + u * G;
-              if (c < n) {
-                s = fma(dv[u], xa[c], s);
-                s = fma(ev[u], xz[c], s);
-              }
-            }
-          }
-          for (int c = g; c < nx; c += G) s = fma(double(Bj[(size_t)c * n + i]), xc[xb_off + c], s);
-        }
-        part[tid] = s;
-        __syncthreads();
-        for (int i2 = tid; i2 < n; i2 += bs) {
-          double t = 0.0;
-          for (int g2 = 0; g2 < G; ++g2) t += part[g2 * n + i2];
-          y[i2] = xc[(size_t)j * n + i2] - t;
-        }
-        __syncthreads();
-      }
-      // U y = rhs, from the last block of 32 rows up
-      for (int rb = ((n - 1) / 32) * 32; rb >= 0; rb -= 32) {
-        const int rw = n - rb < 32 ? n - rb : 32;
-        // the diagonal block of U through shared memory (one coalesced load)
-        for (int e = tid; e < rw * 32; e += bs) {
-          const int c = e >> 5, r = e & 31;
-          tb[c][r] = r < rw ? double(Tj[(size_t)(rb + c) * n2 + rb + r]) : 0.0;
-        }
-        __syncthreads();
-        if (warp == 0) {
-          double v = lane < rw ? y[rb + lane] : 0.0;
-          const double rdi = lane < rw ? 1.0 / tb[lane][lane] : 0.0;
-          for (int ii = rw - 1; ii >= 0; --ii) {
-            const double xi = __shfl_sync(FULL, v * rdi, ii);
-            if (lane == ii) v = xi;
-            else if (lane < ii) v = fma(-tb[ii][lane], xi, v);
-          }
-          if (lane < rw) y[rb + lane] = v;
-        }
-        __syncthreads();
-        for (int r = tid; r < rb; r += bs) {
-          double s = y[r];
-          for (int c0 = 0; c0 < rw; c0 += 8) {  // 8 loads in flight
-            double tv[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) tv[u] = c0 + u < rw ? double(Tj[(size_t)(rb + c0 + u) * n2 + r]) : 0.0;
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-              if (c0 + u < rw) s = fma(-tv[u], y[rb + c0 + u], s);
-          }
-          y[r] = s;
-        }
-        __syncthreads();
-      }
-      for (int i = tid; i < n; i += bs) {
-        const int dst = qrp ? (int)a.P[(size_t)j * szP(d) + n2 + i] : i;
-        xc[(size_t)j * n + dst] = y[i];
-      }
-    }
-  }
-}
+#include "bcr_sweep_big.cuh"
 
 // ---------------------------------------------------------------------------
 // last block (load_and_factorize_last, cc:1281-1374; solve_last, cc:1385-1479)
@@ -4054,7 +3897,11 @@ static void reduce_blocks(DevState& s, const double* buf, long first, long count
                           const double* base, int ldb, double* out, int ldo, cudaStream_t st) {
   if (m <= 0 || h <= 0) return;
   const int cols = m / h, cw = h <= 256 ? 256 / h : 1;
-  const long chunk = 1024;
+  // about 96 parts: enough CTAs to have the sums in flight, few enough for the
+  // one CTA that adds the parts (16,383 sums of 64 elements took 46 us in 16
+  // parts of 1,024); whole rounds of the CTA's 256 / (column height) groups
+  const long unit = std::max(1, 256 / (std::min(cols, cw) * h)) * 8;
+  const long chunk = std::max(unit, (count / 96 + unit) / unit * unit);
   const int nparts = count > 0 ? (int)((count + chunk - 1) / chunk) : 0;
   for (int c0 = 0; c0 < cols; c0 += cw) {
     const int cn = cols - c0 < cw ? cols - c0 : cw, mm = cn * h;
@@ -4417,9 +4264,11 @@ struct SweepPlan {
   void (*bwd_pipe)(SweepArgs<T>, const SweepArgs<T>*, const BatchCta*, const long*, long) = nullptr;
   size_t bwd_pipe_smem = 0;
   void (*bwd_top)(SweepArgs<T>, int, int) = nullptr;
-  void (*fwd_cta)(SweepArgs<T>, const SweepArgs<T>*, const BatchCta*) = nullptr;  // CTA per pair (large n)
-  bool fwd_op = false;  // k_forward_op (the blocked FP64 kernel's operator form)
-  void (*bwd_cta)(SweepArgs<T>, const SweepArgs<T>*, const BatchCta*) = nullptr;
+  // CTA per pair (16 < n, see bcr_sweep_big.cuh): threads, shared memory per right-hand side
+  void (*fwd_big)(SweepArgs<T>) = nullptr;
+  void (*bwd_big)(SweepArgs<T>) = nullptr;
+  int fwd_big_nt = 0, bwd_big_nt = 0;
+  size_t fwd_big_smem = 0, bwd_big_smem = 0;
 };
 
 template <typename T>
@@ -4465,17 +4314,33 @@ static SweepPlan<T> plan_sweeps(const DevState& s) {
   if (n == 32) {
     if (s.sel == SEL_LU && d.nr <= 8) p.fwd = d.nr <= 4 ? k_forward_rows32<T, 4> : k_forward_rows32<T, 8>;
     if (d.nx <= 8) p.bwd = d.nx <= 4 ? k_backward_rows32<T, 4> : k_backward_rows32<T, 8>;
-  } else if (n > 16 && n <= SWP_MAXN) {
-    if (s.sel == SEL_LU) p.fwd_cta = k_forward_cta<T>;
-    p.bwd_cta = k_backward_cta<T>;
+  }
+  if (n > 16 && n <= 128) {
+    if (s.sel == SEL_LU && !p.fwd) {
+      p.fwd_big = n <= 32 ? k_forward_lm<64, T> : n <= 64 ? k_forward_lm<128, T> : k_forward_lm<256, T>;
+      const int rw = n <= 32 ? 64 : n <= 64 ? 128 : 256;
+      p.fwd_big_nt = rw * (rw / 64);
+      p.fwd_big_smem = (size_t)rw * 8;
+    }
+    if (!p.bwd) {
+      const int rb = n <= 32 ? 32 : n <= 64 ? 64 : 128;
+      p.bwd_big = n <= 32 ? k_backward_big<32, T> : n <= 64 ? k_backward_big<64, T> : k_backward_big<128, T>;
+      p.bwd_big_nt = rb * (rb / 32);
+      p.bwd_big_smem = (size_t)(3 * rb + p.bwd_big_nt) * 8;
+      smem_limit_once(p.bwd_big, p.bwd_big_smem * SWB_RHS);
+    }
   }
   // the form of the factors follows the kernel that made them
   const FactorPlan<T> fp = plan_factor<T>(s);
   if (fp.tc) p.op = n;
   if constexpr (sizeof(T) == 8) {
     if (fp.lub.threads) {
+      const int rw = n <= 64 ? 128 : 256;
       p.op = fp.lub.bw;
-      p.fwd_op = true;
+      p.fwd_big = n <= 64 ? k_forward_op<128> : k_forward_op<256>;
+      p.fwd_big_nt = 2 * rw;
+      p.fwd_big_smem = (size_t)(3 * rw + 64) * 8;
+      smem_limit_once(p.fwd_big, p.fwd_big_smem * SWB_RHS);
     }
   }
   return p;
@@ -4519,11 +4384,10 @@ static void forward_levels(DevState& s, const SweepPlan<T>& p, const WorkSet<T>&
   for (int K = 1; K < d.nblock; K *= 2) {
     a.k = K;
     const long np = pairs_at_level(d.nblock, K);
-    if (p.fwd_op) {
-      if constexpr (sizeof(T) == 8) k_forward_op<<<grid_for(np, 1, 148 * 4), FWD_OP_NT, 0, st>>>(a);
-    } else if (p.fwd_pipe)
+    if (p.fwd_big)
+      p.fwd_big<<<grid_for(np, 1, 148 * 32), p.fwd_big_nt, p.fwd_big_smem * std::min(nrhs, SWB_RHS), st>>>(a);
+    else if (p.fwd_pipe)
       p.fwd_pipe<<<grid_for(np, 8, 148 * 2), 256, p.fwd_pipe_smem, st>>>(a, nullptr, nullptr, nullptr, 0);
-    else if (p.fwd_cta) p.fwd_cta<<<grid_for(np, 1, 148 * 8), 256, 0, st>>>(a, nullptr, nullptr);
     else if (p.fwd) p.fwd<<<grid_for(np, 8, 148 * 32), 256, 0, st>>>(a, nullptr, nullptr, nullptr);
     else k_forward_level<T><<<grid_for(np, WARPS_PANEL, 148 * 16), WARPS_PANEL * 32, smem_f, st>>>(a, nullptr, nullptr, nullptr);
     check_launch("k_forward_level");
@@ -4562,7 +4426,8 @@ static void last_and_backward(DevState& s, const SweepPlan<T>& p, const WorkSet<
   for (int k = top_level(d.nblock); (k /= 2) > 0;) {
     a.k = k;
     const long np = pairs_at_level(d.nblock, k);
-    if (p.bwd_cta) p.bwd_cta<<<grid_for(np, 1, 148 * 8), 256, 0, st>>>(a, nullptr, nullptr);
+    if (p.bwd_big)
+      p.bwd_big<<<grid_for(np, 1, 148 * 32), p.bwd_big_nt, p.bwd_big_smem * std::min(nrhs, SWB_RHS), st>>>(a);
     else if (p.bwd) p.bwd<<<grid_for(np, 8, 148 * 32), 256, 0, st>>>(a, nullptr, nullptr, nullptr);
     else k_backward_level<T><<<grid_for(np, WARPS_PANEL, 148 * 16), WARPS_PANEL * 32, smem_b, st>>>(a, nullptr, nullptr, nullptr);
     check_launch("k_backward_level");

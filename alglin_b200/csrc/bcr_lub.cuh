@@ -739,74 +739,3 @@ __device__ int lub_square(LubShared<NT>& sh, double* smem, double* W, int N, int
   }
   return sh.info;
 }
-
-// ---------------------------------------------------------------------------
-// Forward sweep for the operator form of large blocks (T_j, C_j by blocks of
-// op columns): per block one matrix-vector product with the rows at and below
-// it, two threads per row (half the block's columns each) with their loads in
-// flight together.  One CTA per pair.
-// ---------------------------------------------------------------------------
-constexpr int FWD_OP_NT = 512;
-
-__global__ void __launch_bounds__(FWD_OP_NT) k_forward_op(SweepArgs<double> a) {
-  __shared__ double y[LUB_ROWS_MAX], raw[LUB_W], part[LUB_ROWS_MAX];
-  const int tid = threadIdx.x, half = tid >> 8, t = tid & 255;
-  const Dims d = a.d;
-  const int n = d.n, n2 = 2 * n, nr = d.nr, R = n2 + nr, nrhs = a.nrhs, k = a.k, bw = a.op;
-  const long np = pairs_at_level(d.nblock, k);
-  for (long q = blockIdx.x; q < np; q += gridDim.x) {
-    const int j = k + (int)(2L * k * q), jp = j - k;
-    const double* Tj = a.Tm + (size_t)j * szT(d);
-    const unsigned char* Pj = a.P + (size_t)j * szP(d);
-    const double* Cj = a.C + (size_t)j * nr * n;
-    for (int col = 0; col < nrhs; ++col) {
-      double* xc = a.x + (size_t)col * a.ldx;
-      for (int p = tid; p < R; p += FWD_OP_NT) {
-        double v = 0.0;
-        if (p < n2) {
-          const int r = Pj[p];  // original row at this position
-          v = r < n ? xc[(size_t)jp * n + r] : xc[(size_t)j * n + (r - n)];
-        }
-        y[p] = v;
-      }
-      __syncthreads();
-      for (int kb = 0; kb < n; kb += bw) {
-        const int w = n - kb < bw ? n - kb : bw, hw = (w + 1) / 2;
-        for (int c = tid; c < w; c += FWD_OP_NT) raw[c] = y[kb + c];
-        __syncthreads();
-        // rows kb .. R (the border rows last), 256 at a time
-        for (int r0 = kb; r0 < R; r0 += 256) {
-          const int r = r0 + t;
-          const int c0 = half * hw, c1 = half ? w : hw;
-          double s0 = 0.0, s1 = 0.0;
-          if (r < R) {
-            const double* m = r < n2 ? Tj + (size_t)kb * n2 + r : Cj + (size_t)kb * nr + (r - n2);
-            const size_t st = r < n2 ? n2 : nr;
-            const int lim = r < n2 ? r - kb : w;  // strictly left of the diagonal
-            const int ce = c1 < lim ? c1 : lim;
-            for (int c = c0; c < ce; c += 16) {
-              double v[16];
-#pragma unroll
-              for (int u = 0; u < 16; ++u) v[u] = ldg_if(c + u < ce, m + (size_t)(c + u) * st);
-#pragma unroll
-              for (int u = 0; u < 16; u += 2) {
-                s0 = fma(v[u], raw[min(c + u, w - 1)], s0);
-                s1 = fma(v[u + 1], raw[min(c + u + 1, w - 1)], s1);
-              }
-            }
-          }
-          if (half) part[t] = s0 + s1;
-          __syncthreads();
-          if (!half && r < R) y[r] += (s0 + s1) + part[t];
-          __syncthreads();
-        }
-      }
-      for (int p = tid; p < R; p += FWD_OP_NT) {
-        if (p < n) xc[(size_t)j * n + p] = y[p];
-        else if (p < n2) xc[(size_t)jp * n + p - n] = y[p];
-        else a.XB[(size_t)j * nr * nrhs + (size_t)col * nr + (p - n2)] = y[p];
-      }
-      __syncthreads();
-    }
-  }
-}

@@ -85,3 +85,31 @@ def test_large_block_lu(n, nr, nx, nblock):
     qr = max(0, nx - nr)
     s = synth.collocation(nblock, n, qr, qx, nr, nx, seed=n)
     check(s, synth.rhs(s, 3, seed=n + 1), bar=1e-9)
+
+
+@pytest.mark.parametrize("n", [17, 31, 32, 33, 64, 65, 127, 128])
+@pytest.mark.parametrize("nrhs", [1, 8, 9, 17])
+@pytest.mark.parametrize("mode", ["LU", "QRP", "mixed"])
+def test_large_block_sweeps(n, nrhs, mode):
+    """The sweeps for n > 16 at the edges of their runs of 32 columns, of the row
+    counts their threads are built for and of the chunks of right-hand sides
+    (8, after the 16 of a solve), with L and M, with the operator form and with
+    QRP's column map.  Bar: as test_large_block_lu; the mixed path is refined to
+    1e-15 relative residual, which cond(A) <= 3e4 turns into 3e-11."""
+    s = synth.collocation(5, n, 0, 0, 3, 3, seed=n)
+    rhs = synth.rhs(s, nrhs, seed=n + 1)
+    if mode != "mixed":
+        return check(s, rhs, mode, bar=1e-9)
+    o = po.Oracle(s, "LU", "LU")
+    assert o.factorize(), o.last_error()
+    xo = o.solve(rhs)
+    h = B.BorderedCR()
+    h.load_system(s)
+    h.set_precision(B.PRECISION_MIXED)
+    h.set_refinement(1e-15, 10)
+    assert h.factorize(), h.last_error()
+    x = rhs.copy()
+    assert h.solve_n(nrhs, x.reshape(-1), x.shape[1]), h.last_error()
+    assert h.refinement_info()[1] <= 1e-15
+    for c in range(nrhs):
+        assert fwd_err(x[c, :s.ncols], xo[c, :s.ncols]) < 1e-9
