@@ -1744,7 +1744,6 @@ __global__ void __launch_bounds__(2 * N + 32, grp_min_blocks<T, N>())
 // ---------------------------------------------------------------------------
 constexpr int BLK_W = 32;
 constexpr int BLK_ROWS_MAX = 512;  // 2n + nr of the blocked kernel
-constexpr int LAST_BLOCKED_MIN = 64;  // last blocks of this order and above: blocked LU
 
 // W[c*R + rowp[r]] -= sum_m L[m*LD + r] * W[c*R + rowp[k0 + m]] for positions r in
 // [r0, R), c in [c0, NC), m < w; L: the factored block in shared memory (column m,
@@ -3476,6 +3475,85 @@ __device__ void last_fallback_body(Dims d, LastBufs b, StatusWords* st) {
   last_svd(d, b.A2, b, st);
 }
 
+// b <- (L U)^-1 P b with the factors by original row (FACT_LU_ROWS), N <= 512:
+// position r on thread r (the CTA has at least N threads), blocks of 32 columns.
+// Each thread reads its row's 32 elements of a block in one batch, a block ahead
+// of the one being solved, so that the 2 N / 32 steps do not wait for memory
+// (195 us at N = 288 with eight loads at a time, interleaved with their uses).
+__device__ void last_solve_rows(const double* A, const int* piv, int N, double* b, double* tmp) {
+  const int tid = threadIdx.x, bs = blockDim.x, lane = tid & 31;
+  constexpr unsigned FULL = 0xffffffffu;
+  const int nblk = (N + 31) / 32;
+  for (int r = tid; r < N; r += bs) tmp[r] = b[piv[r]];
+  __syncthreads();
+  for (int r = tid; r < N; r += bs) b[r] = tmp[r];
+  const int pr = tid < N ? piv[tid] : 0;
+  double m[32];
+  auto load = [&](int kb, bool lower) {
+#pragma unroll
+    for (int u = 0; u < 32; ++u) {
+      const int c = 32 * kb + u;
+      m[u] = ld_batch(tid < N && c < N && (lower ? c < tid : c >= tid), A + (size_t)c * N + pr);
+    }
+  };
+  load(0, true);
+  __syncthreads();
+  for (int kb = 0; kb < nblk; ++kb) {
+    if (tid / 32 == kb) {  // the warp with the diagonal block
+      const int r = tid;
+      double v = r < N ? b[r] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 31; ++u) {
+        const double vc = __shfl_sync(FULL, v, u);
+        if (lane > u) v = fma(-m[u], vc, v);
+      }
+      if (r < N) b[r] = v;
+    }
+    __syncthreads();
+    if (tid >= 32 * (kb + 1) && tid < N) {
+      double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+      for (int u = 0; u < 32; u += 2) {
+        s0 = fma(m[u], b[min(32 * kb + u, N - 1)], s0);
+        s1 = fma(m[u + 1], b[min(32 * kb + u + 1, N - 1)], s1);
+      }
+      b[tid] -= s0 + s1;
+    }
+    if (kb + 1 < nblk) load(kb + 1, true);
+    else load(nblk - 1, false);
+    __syncthreads();
+  }
+  for (int kb = nblk - 1; kb >= 0; --kb) {
+    if (tid / 32 == kb) {
+      const int r = tid;
+      double ud = 1.0;
+#pragma unroll
+      for (int u = 0; u < 32; ++u)
+        if (u == lane) ud = m[u];
+      double v = r < N ? b[r] : 0.0;
+      const double rdi = r < N ? 1.0 / ud : 0.0;
+#pragma unroll
+      for (int u = 31; u >= 0; --u) {
+        const double xi = __shfl_sync(FULL, v * rdi, u);
+        v = lane == u ? xi : fma(-m[u], lane < u ? xi : 0.0, v);
+      }
+      if (r < N) b[r] = v;
+    }
+    __syncthreads();
+    if (tid < 32 * kb) {
+      double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+      for (int u = 0; u < 32; u += 2) {
+        s0 = fma(m[u], b[min(32 * kb + u, N - 1)], s0);
+        s1 = fma(m[u + 1], b[min(32 * kb + u + 1, N - 1)], s1);
+      }
+      b[tid] -= s0 + s1;
+    }
+    if (kb > 0) load(kb - 1, false);
+    __syncthreads();
+  }
+}
+
 template <typename T>
 __device__ void last_solve_body(Dims d, LastBufs lb, const StatusWords* st, T* x, int ldx, int nrhs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -3484,15 +3562,52 @@ __device__ void last_solve_body(Dims d, LastBufs lb, const StatusWords* st, T* x
   T* b = reinterpret_cast<T*>(smem_raw);
   T* tmp = b + L;
   __shared__ T sv[32];
-  // a diagonal 32 x 32 block of the blocked LU's factors, or the whole L\U of a
-  // small last block (order <= LAST_SMALL, ld order + 1)
+  // the whole L\U of a small last block (order <= LAST_SMALL, ld order + 1)
   __shared__ T big[LAST_SMALL * (LAST_SMALL + 1)];
-  T (*lt)[33] = reinterpret_cast<T (*)[33]>(big);
   const int kind = st->kind;
-  const bool small_lu = kind == FACT_LU && M == N && N <= LAST_SMALL;
-  if (small_lu) {
-    for (int e = tid; e < N * N; e += bs) big[(e / N) * (N + 1) + e % N] = lb.A[e];
+  if ((kind == FACT_LU || kind == FACT_LU_ROWS) && M == N && N <= LAST_SMALL) {
+    // L\U in position order in shared memory; a warp per right-hand side, its
+    // values in registers (lane = rows lane and lane + 32)
+    __shared__ int perm[LAST_SMALL];
+    const bool rows = kind == FACT_LU_ROWS;
+    if (rows) {
+      for (int r = tid; r < N; r += bs) perm[r] = lb.piv[r];
+    } else if (tid == 0) {  // getrf's interchanges
+      for (int r = 0; r < N; ++r) perm[r] = r;
+      for (int i = 0; i < N; ++i) {
+        const int p = lb.piv[i], t = perm[i];
+        perm[i] = perm[p];
+        perm[p] = t;
+      }
+    }
     __syncthreads();
+    for (int e = tid; e < N * N; e += bs) {
+      const int c = e / N, r = e % N;
+      big[c * (N + 1) + r] = lb.A[(size_t)c * N + (rows ? perm[r] : r)];
+    }
+    __syncthreads();
+    const int lane = tid & 31, r0 = lane, r1 = lane + 32, ld = N + 1;
+    const size_t off = (size_t)d.nblock * n;
+    const T d0 = r0 < N ? T(1) / big[r0 * ld + r0] : T(0), d1 = r1 < N ? T(1) / big[r1 * ld + r1] : T(0);
+    for (int c = tid >> 5; c < nrhs; c += bs >> 5) {
+      T* xc = x + (size_t)c * ldx;
+      auto at = [&](int r) -> T& { return r < n ? xc[r] : xc[off + (r - n)]; };
+      T x0 = r0 < N ? at(perm[r0]) : T(0), x1 = r1 < N ? at(perm[r1]) : T(0);
+      __syncwarp();
+      for (int i = 0; i < N; ++i) {
+        const T bi = __shfl_sync(0xffffffffu, i < 32 ? x0 : x1, i & 31);
+        if (r0 > i && r0 < N) x0 = fma(-big[i * ld + r0], bi, x0);
+        if (r1 > i && r1 < N) x1 = fma(-big[i * ld + r1], bi, x1);
+      }
+      for (int i = N - 1; i >= 0; --i) {
+        const T xi = __shfl_sync(0xffffffffu, i < 32 ? x0 * d0 : x1 * d1, i & 31);
+        x0 = r0 == i ? xi : r0 < i ? fma(-big[i * ld + r0], xi, x0) : x0;
+        x1 = r1 == i ? xi : r1 < i ? fma(-big[i * ld + r1], xi, x1) : x1;
+      }
+      if (r0 < N) at(r0) = x0;
+      if (r1 < N) at(r1) = x1;
+    }
+    return;
   }
   const T* A = lb.A;
   const int* piv = lb.piv;
@@ -3544,34 +3659,6 @@ __device__ void last_solve_body(Dims d, LastBufs lb, const StatusWords* st, T* x
         b[i] = s;
       }
       __syncthreads();
-    } else if (small_lu) {
-      // row interchanges, unit-lower and upper solves on one warp, the values in
-      // registers (lane = rows lane and lane + 32) and L\U in shared memory
-      if (tid < 32) {
-        const int lane = tid, r0 = lane, r1 = lane + 32, ld = N + 1;
-        if (lane == 0)
-          for (int i = 0; i < N; ++i) {
-            const int p = piv[i];
-            if (p != i) { T t = b[i]; b[i] = b[p]; b[p] = t; }
-          }
-        __syncwarp();
-        T x0 = r0 < N ? b[r0] : T(0), x1 = r1 < N ? b[r1] : T(0);
-        for (int i = 0; i < N; ++i) {
-          const T bi = __shfl_sync(0xffffffffu, i < 32 ? x0 : x1, i & 31);
-          if (r0 > i && r0 < N) x0 = fma(-big[i * ld + r0], bi, x0);
-          if (r1 > i && r1 < N) x1 = fma(-big[i * ld + r1], bi, x1);
-        }
-        for (int i = N - 1; i >= 0; --i) {
-          const T xi = __shfl_sync(0xffffffffu, i < 32 ? x0 : x1, i & 31) / big[i * ld + i];
-          if (r0 == i) x0 = xi;
-          else if (r0 < i) x0 = fma(-big[i * ld + r0], xi, x0);
-          if (r1 == i) x1 = xi;
-          else if (r1 < i) x1 = fma(-big[i * ld + r1], xi, x1);
-        }
-        if (r0 < N) b[r0] = x0;
-        if (r1 < N) b[r1] = x1;
-      }
-      __syncthreads();
     } else {
       if (kind == FACT_LU || kind == FACT_LUPQ) {
         if (tid == 0)
@@ -3586,45 +3673,7 @@ __device__ void last_solve_body(Dims d, LastBufs lb, const StatusWords* st, T* x
           __syncthreads();
         }
       } else if (kind == FACT_LU_ROWS) {
-        for (int r = tid; r < N; r += bs) tmp[r] = b[piv[r]];
-        __syncthreads();
-        for (int r = tid; r < N; r += bs) b[r] = tmp[r];
-        __syncthreads();
-        // unit lower L by blocks of 32 rows: the diagonal block staged in shared
-        // memory and solved by one warp, the rows below updated with 8 loads in
-        // flight (same operation order as one column at a time)
-        const int lane = tid & 31, warp = tid >> 5;
-        for (int kb = 0; kb < N; kb += 32) {
-          const int w = N - kb < 32 ? N - kb : 32;
-          for (int e = tid; e < 32 * 32; e += bs) {
-            const int c = e >> 5, r = e & 31;
-            lt[c][r] = (c < w && r < w) ? A[(size_t)(kb + c) * N + piv[kb + r]] : T(0);
-          }
-          __syncthreads();
-          if (warp == 0) {
-            T v = lane < w ? b[kb + lane] : T(0);
-            for (int c = 0; c < w; ++c) {
-              const T vc = __shfl_sync(0xffffffffu, v, c);
-              if (lane > c && lane < w) v = fma(-lt[c][lane], vc, v);
-            }
-            if (lane < w) b[kb + lane] = v;
-          }
-          __syncthreads();
-          for (int r = kb + w + tid; r < N; r += bs) {
-            const int pr = piv[r];
-            T sr = b[r];
-            for (int c0 = 0; c0 < w; c0 += 8) {
-              T av[8];
-#pragma unroll
-              for (int u = 0; u < 8; ++u) av[u] = c0 + u < w ? A[(size_t)(kb + c0 + u) * N + pr] : T(0);
-#pragma unroll
-              for (int u = 0; u < 8; ++u)
-                if (c0 + u < w) sr = fma(-av[u], b[kb + c0 + u], sr);
-            }
-            b[r] = sr;
-          }
-          __syncthreads();
-        }
+        last_solve_rows(A, piv, N, b, tmp);
       } else {
         for (int i = 0; i < N; ++i) {
           const T* v = A + (size_t)i * M;
@@ -3639,43 +3688,7 @@ __device__ void last_solve_body(Dims d, LastBufs lb, const StatusWords* st, T* x
         }
       }
       const int lda = (kind == FACT_LU || kind == FACT_LUPQ) ? N : M;
-      if (kind == FACT_LU_ROWS) {
-        // U by blocks of 32 rows from the bottom (row of position r: piv[r]), the
-        // same operation order as one column at a time
-        const int lane = tid & 31, warp = tid >> 5;
-        for (int rb = ((N - 1) / 32) * 32; rb >= 0; rb -= 32) {
-          const int w = N - rb < 32 ? N - rb : 32;
-          for (int e = tid; e < 32 * 32; e += bs) {
-            const int c = e >> 5, r = e & 31;
-            lt[c][r] = (c < w && r < w) ? A[(size_t)(rb + c) * N + piv[rb + r]] : T(0);
-          }
-          __syncthreads();
-          if (warp == 0) {
-            T v = lane < w ? b[rb + lane] : T(0);
-            const T dl = lane < w ? lt[lane][lane] : T(1);
-            for (int ii = w - 1; ii >= 0; --ii) {
-              const T xi = __shfl_sync(0xffffffffu, v / dl, ii);
-              if (lane == ii) v = xi;
-              else if (lane < ii) v = fma(-lt[ii][lane], xi, v);
-            }
-            if (lane < w) b[rb + lane] = v;
-          }
-          __syncthreads();
-          for (int r = tid; r < rb; r += bs) {
-            const int pr = piv[r];
-            T sr = b[r];
-            for (int c1 = w; c1 > 0; c1 -= 8) {  // columns rb + w - 1 down to rb
-              T av[8];
-#pragma unroll
-              for (int u = 0; u < 8; ++u) av[u] = c1 - 1 - u >= 0 ? A[(size_t)(rb + c1 - 1 - u) * N + pr] : T(0);
-#pragma unroll
-              for (int u = 0; u < 8; ++u)
-                if (c1 - 1 - u >= 0) sr = fma(-av[u], b[rb + c1 - 1 - u], sr);
-            }
-            b[r] = sr;
-          }
-          __syncthreads();
-        }
+      if (kind == FACT_LU_ROWS) {  // done above
       } else {
         for (int i = N - 1; i >= 0; --i) {
           const T xi = b[i] / A[(size_t)i * lda + i];
@@ -3734,13 +3747,8 @@ __global__ void __launch_bounds__(512, 1) k_last_lu_blocked(Dims d, LastBufs b, 
 
 __global__ void k_last_fallback(Dims d, LastBufs b, StatusWords* st) { last_fallback_body(d, b, st); }
 
-// LU of a last block of order <= LAST_SMALL on its own (one CTA)
-__global__ void __launch_bounds__(256) k_last_lu_small(Dims d, LastBufs b, StatusWords* st) {
-  last_lu_small<double>(d, b, st);
-}
-
 template <typename T>
-__global__ void k_last_solve(Dims d, LastBufs b, const StatusWords* st, T* x, int ldx, int nrhs) {
+__global__ void __launch_bounds__(512, 1) k_last_solve(Dims d, LastBufs b, const StatusWords* st, T* x, int ldx, int nrhs) {
   last_solve_body<T>(d, b, st, x, ldx, nrhs);
 }
 
@@ -3768,75 +3776,102 @@ __global__ void k_mv_rows(Dims d, const double* D, const double* E, const double
     const double* Dk = D + k * n * n;
     const double* Ek = E + k * n * n;
     const double* Bk = B + k * n * nx;
-    double s = 0;
+    // column by column, eight loads of the matrix in flight (see ld_batch);
+    // x is the same for a block's rows and comes from L1
+    double s = 0.0, sa = 0.0;
+    auto run = [&](const double* M, int cols, const double* v) {
+      for (int c0 = 0; c0 < cols; c0 += 8) {
+        double mv[8], xv[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) mv[u] = ld_batch(c0 + u < cols, M + (size_t)(c0 + u) * n + i);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) xv[u] = ABS ? 0.0 : ld_batch(c0 + u < cols, v + c0 + u);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          s = ABS ? s + fabs(mv[u]) : fma(mv[u], xv[u], s);
+          sa += fabs(mv[u]);
+        }
+      }
+    };
+    run(Dk, n, x + k * n);
+    run(Ek, n, x + (k + 1) * n);
+    run(Bk, nx, x + xb_off);
     if constexpr (ABS) {
-      for (int c = 0; c < n; ++c) s += fabs(Dk[(size_t)c * n + i]) + fabs(Ek[(size_t)c * n + i]);
-      for (int c = 0; c < nx; ++c) s += fabs(Bk[(size_t)c * n + i]);
       res[e] = s;
-    } else if (rowsum) {
-      double sa = 0;
-      for (int c = 0; c < n; ++c) {
-        const double a = Dk[(size_t)c * n + i];
-        s += a * x[k * n + c];
-        sa += fabs(a);
-      }
-      for (int c = 0; c < n; ++c) {
-        const double a = Ek[(size_t)c * n + i];
-        s += a * x[(k + 1) * n + c];
-        sa += fabs(a);
-      }
-      for (int c = 0; c < nx; ++c) {
-        const double a = Bk[(size_t)c * n + i];
-        s += a * x[xb_off + c];
-        sa += fabs(a);
-      }
-      res[e] = (beta == 0.0 ? 0.0 : beta * res[e]) + alpha * s;
-      rowsum[e] = sa;
     } else {
-      for (int c = 0; c < n; ++c) s += Dk[(size_t)c * n + i] * x[k * n + c];
-      for (int c = 0; c < n; ++c) s += Ek[(size_t)c * n + i] * x[(k + 1) * n + c];
-      for (int c = 0; c < nx; ++c) s += Bk[(size_t)c * n + i] * x[xb_off + c];
       res[e] = (beta == 0.0 ? 0.0 : beta * res[e]) + alpha * s;
+      if (rowsum) rowsum[e] = sa;
     }
   }
 }
 
+// C_k x_k per block: 64 elements per CTA round, the columns of each over four
+// threads (eight loads in flight), added in a fixed order
 template <bool ABS>
-__global__ void k_mv_cpart(Dims d, const double* C, const double* x, double* part) {
-  const int n = d.n, nr = d.nr;
+__global__ void __launch_bounds__(256) k_mv_cpart(Dims d, const double* C, const double* x, double* part) {
+  __shared__ double sp[4][64];
+  const int n = d.n, nr = d.nr, t = threadIdx.x & 63, h = threadIdx.x >> 6;
   const size_t total = (size_t)(d.nblock + 1) * nr;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const size_t k = e / nr;
+  const int c_lo = n * h / 4, c_hi = n * (h + 1) / 4;
+  for (size_t e0 = (size_t)blockIdx.x * 64; e0 < total; e0 += (size_t)gridDim.x * 64) {
+    const size_t e = e0 + t, k = e / nr;
     const int r = (int)(e % nr);
+    const bool live = e < total;
     const double* Ck = C + k * nr * n;
-    double s = 0;
-    for (int c = 0; c < n; ++c) s += ABS ? fabs(Ck[(size_t)c * nr + r]) : Ck[(size_t)c * nr + r] * x[k * n + c];
-    part[e] = s;
+    double s = 0.0;
+    for (int c0 = c_lo; c0 < c_hi; c0 += 8) {
+      double cv[8], xv[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) cv[u] = ld_batch(live && c0 + u < c_hi, Ck + (size_t)(c0 + u) * nr + r);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) xv[u] = ABS ? 0.0 : ld_batch(live && c0 + u < c_hi, x + k * n + c0 + u);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s = ABS ? s + fabs(cv[u]) : fma(cv[u], xv[u], s);
+    }
+    sp[h][t] = s;
+    __syncthreads();
+    if (h == 0 && live) part[e] = ((s + sp[1][t]) + sp[2][t]) + sp[3][t];
+    __syncthreads();
   }
 }
 
-// H rows and the nr border rows (Csum = sum_k C_k x_k precomputed)
+// H rows and the nr border rows (Csum = sum_k C_k x_k precomputed): 32 rows per
+// CTA, the columns over its 16 warps, eight loads in flight each, the partial
+// sums added in warp order (one thread per row took 130 us at 144 rows)
+constexpr int MVT_W = 16;
 template <bool ABS>
-__global__ void k_mv_tail(Dims d, const double* H, const double* Cq, const double* F,
+__global__ void __launch_bounds__(32 * MVT_W) k_mv_tail(Dims d, const double* H, const double* Cq, const double* F,
                           const double* Csum, double alpha, const double* x, double beta,
                           double* res) {
+  __shared__ double part[MVT_W][32];
   const int n = d.n, m = n + d.qr, nr = d.nr, qx = d.qx, nx = d.nx, Nc = d.Nc;
   const size_t r0 = (size_t)d.nblock * n;
-  const size_t xN = (size_t)d.nblock * n, xq = (size_t)(d.nblock + 1) * n, xb = xq + qx;
-  for (int r = threadIdx.x; r < m + nr; r += blockDim.x) {
-    double s = 0;
-    if (r < m) {
-      for (int c = 0; c < Nc; ++c) {
-        size_t xi = c < n ? (size_t)c : (c < 2 * n ? xN + (c - n) : xq + (c - 2 * n));
-        s += ABS ? fabs(H[(size_t)c * m + r]) : H[(size_t)c * m + r] * x[xi];
-      }
-    } else {
-      const int rr = r - m;
-      s = Csum[rr];
-      for (int c = 0; c < qx; ++c) s += ABS ? fabs(Cq[(size_t)c * nr + rr]) : Cq[(size_t)c * nr + rr] * x[xq + c];
-      for (int c = 0; c < nx; ++c) s += ABS ? fabs(F[(size_t)c * nr + rr]) : F[(size_t)c * nr + rr] * x[xb + c];
+  const size_t xN = (size_t)d.nblock * n, xq = (size_t)(d.nblock + 1) * n;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = blockIdx.x * 32 + lane;
+  double s = 0.0;
+  // columns of [H0 HN Hq Hp] or, for a border row, of [Cq F] (qx + nx of them)
+  const bool top = r < m, live = r < m + nr;
+  const int cols = top ? Nc : qx + nx;
+  for (int c0 = w; c0 < Nc; c0 += 8 * MVT_W) {
+    double mv[8], xv[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int c = c0 + u * MVT_W, rr = r - m;
+      const bool in = live && c < cols;
+      const double* M = top ? H + (size_t)c * m + r : c < qx ? Cq + (size_t)c * nr + rr : F + (size_t)(c - qx) * nr + rr;
+      const size_t xi = !top ? xq + c : c < n ? (size_t)c : c < 2 * n ? xN + (c - n) : xq + (c - 2 * n);
+      mv[u] = ld_batch(in, M);
+      xv[u] = ABS ? 0.0 : ld_batch(in, x + xi);
     }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s = ABS ? s + fabs(mv[u]) : fma(mv[u], xv[u], s);
+  }
+  part[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && live) {
+    s = top ? 0.0 : Csum[r - m];
+#pragma unroll
+    for (int o = 0; o < MVT_W; ++o) s += part[o][lane];
     const size_t o = r0 + r;
     res[o] = ABS ? s : (beta == 0.0 ? 0.0 : beta * res[o]) + alpha * s;
   }
@@ -4219,14 +4254,11 @@ static void factor_last(DevState& s, const WorkSet<T>& w, cudaStream_t st, bool 
   }
   const LastBufs lb = last_bufs(s);
   const LubPlan lp = lub_plan(d.Nc, d.Nc, true);
-  if (s.sel_last == LAST_LU && d.Nr == d.Nc && d.Nc >= LAST_BLOCKED_MIN && lp.threads) {
+  if (s.sel_last == LAST_LU && d.Nr == d.Nc && lp.threads) {
     auto* kern = lp.depth == 32 ? k_last_lu_blocked<4> : lp.depth == 48 ? k_last_lu_blocked<6> : k_last_lu_blocked<8>;
     smem_limit_once(kern, lp.smem);
     kern<<<1, 512, lp.smem, st>>>(d, lb, s.st, lp.bw);
     check_launch("k_last_lu_blocked");
-  } else if (s.sel_last == LAST_LU && d.Nr == d.Nc && d.Nc <= LAST_SMALL) {
-    k_last_lu_small<<<1, 256, 0, st>>>(d, lb, s.st);
-    check_launch("k_last_lu_small");
   } else {
     k_last_factor<double><<<1, 512, 0, st>>>(d, lb, s.sel_last, s.st);
     check_launch("k_last_factor");
@@ -4400,7 +4432,7 @@ static void last_and_backward(DevState& s, const SweepPlan<T>& p, const WorkSet<
                               int nrhs, cudaStream_t st) {
   const Dims d = s.d;
   const size_t smem_l = 2 * (size_t)(d.Nr > d.Nc ? d.Nr : d.Nc) * 8;
-  k_last_solve<double><<<1, 256, smem_l, st>>>(d, last_bufs(s), s.st, x, ldx, nrhs);
+  k_last_solve<double><<<1, 512, smem_l, st>>>(d, last_bufs(s), s.st, x, ldx, nrhs);
   check_launch("k_last_solve");
   SweepArgs<T> a = sweep_args(s, w, x, ldx, nrhs);
   a.ldw = d.n;
@@ -4601,12 +4633,12 @@ static void mv_t(DevState& s, double alpha, const double* x, double beta, double
   double* Csum = s.Ffin;  // unused when nr == 0
   if (nr > 0) {
     const long tot = (long)(d.nblock + 1) * nr;
-    k_mv_cpart<ABS><<<grid_for(tot, 256, 148 * 8), 256, 0, st>>>(d, s.C0, x, s.mv_part);
+    k_mv_cpart<ABS><<<grid_for(tot, 64, 148 * 8), 256, 0, st>>>(d, s.C0, x, s.mv_part);
     check_launch("k_mv_cpart");
     Csum = s.mv_part + (size_t)(d.nblock + 1) * nr;
     reduce_blocks(s, s.mv_part, 0, d.nblock + 1, nr, nr, nullptr, nr, Csum, nr, st);
   }
-  k_mv_tail<ABS><<<1, 256, 0, st>>>(d, s.H, s.Cq, s.F0, Csum, alpha, x, beta, res);
+  k_mv_tail<ABS><<<(d.n + d.qr + nr + 31) / 32, 32 * MVT_W, 0, st>>>(d, s.H, s.Cq, s.F0, Csum, alpha, x, beta, res);
   check_launch("k_mv_tail");
 }
 
@@ -4615,13 +4647,33 @@ void launch_mv(DevState& s, double alpha, const double* x, double beta, double* 
 }
 
 // out[slot] = max |v_i| over i < len (exact, order independent)
-__global__ void k_absmax(const double* v, long len, unsigned long long* out) {
+// inf-norms of up to three vectors, one per blockIdx.y
+struct AbsMax {
+  const double* v[3];
+  long len[3];
+};
+__global__ void __launch_bounds__(256) k_absmax(AbsMax a, unsigned long long* out) {
+  const double* v = a.v[blockIdx.y];
+  const long len = a.len[blockIdx.y], step = (long)gridDim.x * blockDim.x;
   double m = 0.0;
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (long)gridDim.x * blockDim.x)
-    m = fmax(m, fabs(v[i]));
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += 4 * step) {
+    double t[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) t[u] = ld_batch(i + u * step < len, v + i + u * step);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) m = fmax(m, fabs(t[u]));
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(m));
+  // one atomic per CTA: a few hundred on one address, not a few thousand
+  __shared__ double sm[8];
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int o = 1; o < 8; ++o) m = fmax(m, sm[o]);
+    atomicMax(out + blockIdx.y, (unsigned long long)__double_as_longlong(m));
+  }
 }
 
 __global__ void k_axpy(double* y, const double* x, long len) {
@@ -4642,12 +4694,10 @@ void launch_residual(DevState& s, const double* b, const double* x, double* r, u
   if (rowsum) {
     mv_t<true>(s, 1.0, nullptr, 0.0, rowsum, st, nullptr, true);  // border and last rows
     cudaMemsetAsync(normA, 0, sizeof(unsigned long long), st);
-    k_absmax<<<grid_for(nrows, 256, 148 * 2), 256, 0, st>>>(rowsum, nrows, normA);
+    k_absmax<<<grid_for(nrows, 256, 148 * 2), 256, 0, st>>>(AbsMax{{rowsum}, {nrows}}, normA);
   }
   cudaMemsetAsync(out, 0, 3 * sizeof(unsigned long long), st);
-  k_absmax<<<grid_for(nrows, 256, 148 * 2), 256, 0, st>>>(r, nrows, out);
-  k_absmax<<<grid_for(ncols, 256, 148 * 2), 256, 0, st>>>(x, ncols, out + 1);
-  k_absmax<<<grid_for(nrows, 256, 148 * 2), 256, 0, st>>>(b, nrows, out + 2);
+  k_absmax<<<dim3(grid_for(nrows, 256, 148 * 2), 3), 256, 0, st>>>(AbsMax{{r, x, b}, {nrows, ncols, nrows}}, out);
   check_launch("k_absmax");
 }
 
