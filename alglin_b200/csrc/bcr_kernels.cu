@@ -588,6 +588,12 @@ __global__ void __launch_bounds__(128) k_factor_lu_rows(FactorArgs<T> a0, const 
   rows_body<T, N, NXM, NRM, false>(BATCH ? ab : a0, q0, q1, qs);
 }
 
+template <typename T> __device__ __forceinline__ T rcp_rn(T x);
+template <> __device__ __forceinline__ double rcp_rn<double>(double x) { return __drcp_rn(x); }
+template <> __device__ __forceinline__ float rcp_rn<float>(float x) { return __frcp_rn(x); }
+
+#include "bcr_qr.cuh"
+
 // ---------------------------------------------------------------------------
 // Tensor-core LU pair elimination for n == N (N = 8 or 16), nr <= 8, nx <= 8.
 //
@@ -614,10 +620,6 @@ __global__ void __launch_bounds__(128) k_factor_lu_rows(FactorArgs<T> a0, const 
 // above it; -M L^-1], C_j = -C_j U^-1 L^-1.  The forward sweep applies them as
 // one matrix-vector product (SweepArgs::op).
 // ---------------------------------------------------------------------------
-template <typename T> __device__ __forceinline__ T rcp_rn(T x);
-template <> __device__ __forceinline__ double rcp_rn<double>(double x) { return __drcp_rn(x); }
-template <> __device__ __forceinline__ float rcp_rn<float>(float x) { return __frcp_rn(x); }
-
 // Pivot candidate of one lane: |a| as an integer key (upper word + 1, lower
 // word; NaN below every number, finished rows below everything) and the
 // reciprocal of a by Newton-Raphson steps r <- r + r (1 - a r) from the
@@ -4003,6 +4005,7 @@ struct FactorPlan {
   size_t grp_smem = 0;
   int grp_threads = 0, grp_ctas = 0;
   void (*rows)(FactorArgs<T>, const FactorArgs<T>*, const BatchCta*) = nullptr;             // register LU (n <= 16)
+  void (*qr)(FactorArgs<T>, const FactorArgs<T>*, const BatchCta*) = nullptr;               // warp QR / QRP (n <= 16)
   void (*smem_k)(FactorArgs<T>, const FactorArgs<T>*, const BatchCta*) = nullptr;           // shared-memory kernel
   size_t smem = 0;
   int wpb = 1;
@@ -4094,8 +4097,13 @@ static FactorPlan<T> plan_factor(const DevState& s) {
     else if (n <= 8) p.rows = k_factor_lu_rows<T, 8, 4, 4>;
     else if (n <= 16) p.rows = k_factor_lu_rows<T, 16, 4, 4>;
   }
+  // QR panels in registers; a forced family keeps the shared-memory kernels
+  if (s.sel != SEL_LU && n <= 16 && d.nr <= 8 && n + d.nx <= 32 && s.pair_kernel == PAIR_AUTO) {
+    p.qr = s.sel == SEL_QR ? k_factor_qr_warp<T, false> : k_factor_qr_warp<T, true>;
+    smem_limit_once(p.qr, QrShape<T>::BYTES * 4);
+  }
   const bool smem_fits = per_warp <= SMEM_MAX;
-  if (!p.tc && !p.grp && !p.rows &&
+  if (!p.tc && !p.grp && !p.rows && !p.qr &&
       (use_cta_kernel(d) || s.pair_kernel == PAIR_CTA || !smem_fits) &&
       (s.pair_kernel != PAIR_SMEM || !smem_fits)) {
     p.cta = s.sel == SEL_LU ? k_factor_cta<T, SEL_LU>
@@ -4228,6 +4236,7 @@ static bool factor_levels(DevState& s, const FactorPlan<T>& p, const WorkSet<T>&
     else if (p.grp) p.grp<<<grid_for(np, 1, p.grp_ctas), p.grp_threads, p.grp_smem, st>>>(a, nullptr, nullptr);
     else if (p.tc) p.tc<<<grid_for(np, 4, 148 * 16), 128, p.tc_smem, st>>>(a, nullptr, nullptr);
     else if (p.rows) p.rows<<<grid_for(np, 4, 148 * 16), 128, 0, st>>>(a, nullptr, nullptr);
+    else if (p.qr) p.qr<<<grid_for(np, 4, 148 * 16), 128, QrShape<T>::BYTES * 4, st>>>(a, nullptr, nullptr);
     else p.smem_k<<<grid_for(np, p.wpb, 148 * 16), p.wpb * 32, p.smem, st>>>(a, nullptr, nullptr);
     check_launch("k_factor_level");
     if (nrn) {

@@ -113,3 +113,29 @@ def test_large_block_sweeps(n, nrhs, mode):
     assert h.refinement_info()[1] <= 1e-15
     for c in range(nrhs):
         assert fwd_err(x[c, :s.ncols], xo[c, :s.ncols]) < 1e-9
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 7, 8, 9, 15, 16])
+@pytest.mark.parametrize("nr,nx", [(0, 0), (1, 3), (8, 8), (5, 16)])
+@pytest.mark.parametrize("select", ["QR", "QRP"])
+def test_qr_panels(n, nr, nx, select):
+    """The warp QR kernel from one column to a full warp of rows, with all columns
+    in one pass and in two, and its column map.  cond(A) <= 6e3 (dense SVD)."""
+    s = synth.collocation(9, n, max(0, nx - nr), max(0, nr - nx), nr, nx, seed=n)
+    check(s, synth.rhs(s, 2, seed=n + 1), select, bar=1e-9)
+
+
+@pytest.mark.parametrize("select", ["QR", "QRP"])
+def test_qr_zero_column_is_reported(select):
+    """A panel column that is zero in both its row blocks: R has a zero on its
+    diagonal, the factorization fails, and the library stays usable."""
+    s = synth.collocation(6, 7, 0, 0, 2, 2, seed=3)
+    bad = s.copy()
+    bad.E[2, 4] = 0.0  # column 4 of E_2 and D_3 (stored by columns)
+    bad.D[3, 4] = 0.0
+    h = B.BorderedCR()
+    h.load_system(bad)
+    h.select(select)
+    assert not h.factorize()
+    check(s, synth.rhs(s, 1, seed=4), select)
+
