@@ -716,7 +716,12 @@ __device__ __forceinline__ double ldw(const double* p) { return __ldcg(p); }
 // cg holds columns cg*CPL .. cg*CPL + CPL - 1 of border row r (LPR = 32 / NRM
 // lanes per row), so their eliminations (C_j U^-1, then -C' L^-1) run in the
 // same instructions as everyone else instead of on nr lanes alone.
-template <int N, int NRM, typename T = double>
+//
+// PAD: blocks of order n < N, as the leading part of blocks of order N.  Panel
+// lanes are N apart (TOP row r on lane r, BOTTOM row r on lane N + r); the lanes
+// and columns beyond n hold zeros or are never stored.  Positions are those of
+// the 2n rows; in shared memory the reduced rows start at row N.
+template <int N, int NRM, typename T = double, bool PAD = false>
 __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bool first, T* Wt, int lane,
                                         const TcTree& tr) {
   using S = TcShape<N, T>;
@@ -725,13 +730,13 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
   int* rowof = reinterpret_cast<int*>(Gs + S::GS);
   const Dims d = a.d;
   const int nr = d.nr, nx = d.nx;
-  constexpr int n = N, n2 = 2 * N;
-  constexpr size_t nn = (size_t)N * N;
+  const int n = PAD ? d.n : N, n2 = 2 * n;
+  const size_t nn = (size_t)n * n;
   const size_t nnx = (size_t)n * nx, nrn = (size_t)nr * n, nrnx = (size_t)nr * nx;
   const int nrf = a.nrf;             // fused right-hand sides
-  const int NT = n2 + nx + nrf;      // live trailing columns
-  const bool act = lane < n2, top = lane < n;
-  const int ri = top ? lane : lane - n;
+  const bool top = lane < N;
+  const int ri = lane & (N - 1);
+  const bool act = lane < 2 * N && ri < n;
   const int g = lane >> 2, t = lane & 3;
   const int jp = j - k;
   // block elements: the loaded FP64 matrix at the first level, the working
@@ -756,10 +761,10 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
     const SrcT* Pm = (top ? srcE : srcD) + po;
     const double* Po = (top ? a.E0 : a.D0) + po;
 #pragma unroll
-    for (int c = 0; c < N; ++c) rowA[c] = act ? lds(Pm, Po, (size_t)c * n + ri) : T(0);
+    for (int c = 0; c < N; ++c) rowA[c] = act && (!PAD || c < n) ? lds(Pm, Po, (size_t)c * n + ri) : T(0);
 #pragma unroll
     for (int q = 0; q < CPL; ++q)
-      cb[q] = blive ? lds(srcC, a.C0, (size_t)j * nrn + (size_t)(bc0 + q) * nr + br) : T(0);
+      cb[q] = blive && (!PAD || bc0 + q < n) ? lds(srcC, a.C0, (size_t)j * nrn + (size_t)(bc0 + q) * nr + br) : T(0);
     // C_jpp contributions of the pairs (j - 2K', j - K') of earlier levels,
     // K' = 1, 2, ..., gather: loaded eight levels at a time so that their
     // latencies overlap, then added in level order
@@ -794,44 +799,35 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
         }
       }
     }
-    // trailing columns in the original row order: TOP [D_jp 0 B_jp], BOTTOM [0 E_j B_j]
-    // compile-time trip counts: every load of the pair is issued before the
-    // first one is consumed, so a lone pair pays one memory latency
+    // trailing columns in the original row order: TOP [D_jp 0 B_jp], BOTTOM [0 E_j
+    // B_j] and the fused right-hand sides (TOP x_jp, BOTTOM x_j); columns beyond
+    // them are not set (they feed outputs that are not stored).  Compile-time
+    // trip counts: every load of the pair is issued before the first one is
+    // consumed, so a lone pair pays one memory latency
     const SrcT* Djp = srcD + (size_t)jp * nn;
     const SrcT* Ej = srcE + (size_t)j * nn;
     const double* Djp0 = a.D0 + (size_t)jp * nn;
     const double* Ej0 = a.E0 + (size_t)j * nn;
 #pragma unroll
-    for (int it = 0; it < (int)(nn / 32); ++it) {
-      const int idx = lane + 32 * it;
-      const int r = idx % n, c = idx / n;
-      Wt[r * S::LDW + c] = lds(Djp, Djp0, idx);
-      Wt[(n + r) * S::LDW + c] = lds(Ej, Ej0, idx);
-    }
-    const SrcT* Bjp = srcB + (size_t)jp * nnx;
-    const SrcT* Bj = srcB + (size_t)j * nnx;
-    const double* Bjp0 = a.B0 + (size_t)jp * nnx;
-    const double* Bj0 = a.B0 + (size_t)j * nnx;
-#pragma unroll
-    for (int it = 0; it < (8 * N + 31) / 32; ++it) {
-      const int idx = lane + 32 * it;
-      if (idx < (int)nnx) {
-        const int r = idx % n, c = idx / n;
-        Wt[r * S::LDW + n + c] = lds(Bjp, Bjp0, idx);
-        Wt[(n + r) * S::LDW + n + c] = lds(Bj, Bj0, idx);
+    for (int it = 0; it < N * N / 32; ++it) {
+      const int c = it * (32 / N) + lane / N;
+      if (!PAD || (ri < n && c < n)) {
+        Wt[ri * S::LDW + c] = lds(Djp, Djp0, (size_t)c * n + ri);
+        Wt[(N + ri) * S::LDW + c] = lds(Ej, Ej0, (size_t)c * n + ri);
       }
     }
-    // fused right-hand sides: TOP rows hold x_jp, BOTTOM rows x_j
-    for (int idx = lane; idx < n2 * nrf; idx += 32) {
-      const int r = idx % n2, c = idx / n2;
-      const double* xc = a.x + (size_t)c * a.ldx;
-      Wt[r * S::LDW + n + nx + c] = T(r < n ? ldw(xc + (size_t)jp * n + r) : ldw(xc + (size_t)j * n + r - n));
+    if (act) {
+      T* Wr = Wt + lane * S::LDW + N;
+      const size_t bo = (size_t)(top ? jp : j) * nnx + ri;
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (c < nx) Wr[c] = lds(srcB + bo, a.B0 + bo, (size_t)c * n);
+      const double* xr = a.x + (size_t)(top ? jp : j) * n + ri;
+      for (int c = 0; c < nrf; ++c) Wr[nx + c] = T(ldw(xr + (size_t)c * a.ldx));
     }
-    // zero the padding columns of the live rows (they feed padding outputs only,
-    // but keep them finite)
-    for (int idx = lane; idx < n2 * (S::NTP - NT); idx += 32) {
-      const int r = idx % n2, c = NT + idx / n2;
-      Wt[r * S::LDW + c - n] = T(0);
+    if (PAD) {  // rows of the product that no panel row fills
+      if (lane < 2 * N) rowof[lane] = 0;
+      __syncwarp();
     }
   }
   // ------------------- phase 1: panel LU with the operator rows in place
@@ -840,10 +836,12 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
   // same multiplier updates the X of the earlier columns with the pivot row's
   // X, so one run of N - 1 fused multiply-adds per step yields U, L^-1 (the
   // pivot rows' X, strictly lower), -M L^-1 and -C' L^-1 (see the comment above).
-  int mypos = lane, info = 0;
+  const int pos0 = act ? (top ? ri : n + ri) : 63;
+  int mypos = pos0, info = 0;
   bool done = !act;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
+    if (PAD && i >= n) break;
     // pivot: max |a| over the rows not yet used, ties to the smaller position;
     // every lane forms the reciprocal of its own candidate meanwhile
     unsigned hi, lo, hmax, m;
@@ -913,20 +911,22 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
     T* Tj = a.Tm + (size_t)j * szT(d);
     if (act) {
 #pragma unroll
-      for (int c = 0; c < N; ++c) Tj[(size_t)mypos + (size_t)c * n2] = rowA[c];
-      rowof[mypos] = lane;
-      a.P[(size_t)j * szP(d) + mypos] = (unsigned char)lane;
+      for (int c = 0; c < N; ++c)
+        if (!PAD || c < n) Tj[(size_t)mypos + (size_t)c * n2] = rowA[c];
+      const int gr = mypos < n ? mypos : mypos - n + N;  // row of the product
+      rowof[gr] = lane;
+      a.P[(size_t)j * szP(d) + mypos] = (unsigned char)pos0;
       if (mypos >= n) {
 #pragma unroll
-        for (int c = 0; c < N; c += 2) store2(&Gs[mypos * S::LDG + c], rowA[c], rowA[c + 1]);
+        for (int c = 0; c < N; c += 2) store2(&Gs[gr * S::LDG + c], rowA[c], rowA[c + 1]);
       }
     }
 #pragma unroll
     for (int q = 0; q < CPL; ++q) {
-      if (blive) a.C[(size_t)j * nrn + (size_t)(bc0 + q) * nr + br] = cb[q];
+      if (blive && (!PAD || bc0 + q < n)) a.C[(size_t)j * nrn + (size_t)(bc0 + q) * nr + br] = cb[q];
       // border rows of G (zero for rows >= nr, and rows NRM..7 of the tile)
-      Gs[(n2 + br) * S::LDG + bc0 + q] = blive ? cb[q] : T(0);
-      if constexpr (NRM < 8) Gs[(n2 + NRM + br) * S::LDG + bc0 + q] = T(0);
+      Gs[(2 * N + br) * S::LDG + bc0 + q] = blive ? cb[q] : T(0);
+      if constexpr (NRM < 8) Gs[(2 * N + NRM + br) * S::LDG + bc0 + q] = T(0);
     }
   }
   __syncwarp();
@@ -948,7 +948,7 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
         const int nt = pass * PC + ni;
         const int row = mt * 8 + g;
         T c0 = T(0), c1 = T(0);
-        if (nt < S::NTILES && row >= n && row < n2) {  // (PW)_bot
+        if (nt < S::NTILES && row >= N && row < 2 * N) {  // (PW)_bot
           const int orow = rowof[row];
           c0 = tc_w<N>(Wt, orow, nt * 8 + 2 * t);
           c1 = tc_w<N>(Wt, orow, nt * 8 + 2 * t + 1);
@@ -968,9 +968,9 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
         }
 #pragma unroll
         for (int mt = 0; mt < S::MTILES; ++mt) {
-          if (mt * 8 < n && ks * 4 >= mt * 8 + 8) continue;  // above the diagonal of L^-1
+          if (mt * 8 < N && ks * 4 >= mt * 8 + 8) continue;  // above the diagonal of L^-1
           double afr = Gs[(mt * 8 + g) * S::LDG + ks * 4 + t];
-          if (mt * 8 < n && ks * 4 + 3 >= mt * 8) {
+          if (mt * 8 < N && ks * 4 + 3 >= mt * 8) {
             const int dk = ks * 4 + t - (mt * 8 + g);
             afr = dk < 0 ? afr : dk == 0 ? 1.0 : 0.0;
           }
@@ -994,7 +994,7 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
 #pragma unroll
         for (int mt = 0; mt < S::MTILES; ++mt) {
           T av = Gs[(mt * 8 + g) * S::LDG + kk];
-          if (mt * 8 < n) {
+          if (mt * 8 < N) {
             const int dk = kk - (mt * 8 + g);
             av = dk < 0 ? av : dk == 0 ? T(1) : T(0);
           }
@@ -1022,28 +1022,35 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
             if (nt >= S::NTILES) continue;
             const int col = nt * 8 + 2 * t + hh;
             const T v = acc[mt][ni][hh];
-            if (mt * 8 < n2) {  // panel rows (compile-time per mt)
-              const bool ur = row < n;
-              const int rr = ur ? row : row - n;
+            const int cj = col < N ? col : col < 2 * N ? col - N : col - 2 * N;  // column within its block
+            if (mt * 8 < 2 * N) {  // panel rows (compile-time per mt)
+              const bool ur = mt * 8 < N;
+              const int rr = ur ? row : row - N;
+              if (PAD && rr >= n) continue;
               const size_t blk = ur ? (size_t)j : (size_t)jp;
-              if (col < n) a.D[blk * nn + (size_t)col * n + rr] = v;
-              else if (col < n2) a.E[blk * nn + (size_t)(col - n) * n + rr] = v;
-              else if (col < n2 + nx) a.B[blk * nnx + (size_t)(col - n2) * n + rr] = v;
-              else if (col < NT) a.x[(size_t)(col - n2 - nx) * a.ldx + blk * n + rr] = (double)v;
+              if (nt * 8 < N) {
+                if (!PAD || cj < n) a.D[blk * nn + (size_t)cj * n + rr] = v;
+              } else if (nt * 8 < 2 * N) {
+                if (!PAD || cj < n) a.E[blk * nn + (size_t)cj * n + rr] = v;
+              } else if (cj < nx) {
+                a.B[blk * nnx + (size_t)cj * n + rr] = v;
+              } else if (cj < nx + nrf) {
+                a.x[(size_t)(cj - nx) * a.ldx + blk * n + rr] = (double)v;
+              }
             } else {
-              const int rr = row - n2;
+              const int rr = row - 2 * N;
               if (rr < nr) {
-                if (col < n) {
-                  const size_t o = (size_t)jp * nrn + (size_t)col * nr + rr;
-                  a.C[o] = lds(srcC, a.C0, o) + v;
-                } else if (col < n2) {
-                  a.Rbuf[(size_t)j * nrn + (size_t)(col - n) * nr + rr] = v;
-                } else if (col < n2 + nx) {
+                if (nt * 8 < N) {
+                  const size_t o = (size_t)jp * nrn + (size_t)cj * nr + rr;
+                  if (!PAD || cj < n) a.C[o] = lds(srcC, a.C0, o) + v;
+                } else if (nt * 8 < 2 * N) {
+                  if (!PAD || cj < n) a.Rbuf[(size_t)j * nrn + (size_t)cj * nr + rr] = v;
+                } else if (cj < nx) {
                   // own F update plus the partial sums of the child nodes (tree)
-                  const size_t e = (size_t)(col - n2) * nr + rr;
+                  const size_t e = (size_t)cj * nr + rr;
                   a.Fbuf[(size_t)j * nrnx + e] = (double)v + cs1[hh] + cs2[hh];
-                } else if (col < NT) {
-                  const size_t e = (size_t)(col - n2 - nx) * nr + rr, nrr = (size_t)nr * nrf;
+                } else if (cj < nx + nrf) {
+                  const size_t e = (size_t)(cj - nx) * nr + rr, nrr = (size_t)nr * nrf;
                   a.XB[(size_t)j * nrr + e] = (double)v + cs1[hh] + cs2[hh];
                 }
               }
@@ -1066,7 +1073,7 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
 template <typename T>
 constexpr int tc_min_blocks() { return sizeof(T) == 8 ? 4 : 6; }
 
-template <int N, bool BATCH = false, bool BOOK = false, int NRM = 8, typename T = double>
+template <int N, bool BATCH = false, bool BOOK = false, int NRM = 8, typename T = double, bool PAD = false>
 __global__ void __launch_bounds__(128, tc_min_blocks<T>())
     k_factor_lu_tc(FactorArgs<T> a0, const FactorArgs<T>* tab, const BatchCta* cmap) {
   using S = TcShape<N, T>;
@@ -1084,7 +1091,7 @@ __global__ void __launch_bounds__(128, tc_min_blocks<T>())
       tr.gather = a.k / 2;
       tree_children(j, a.d.nblock, tr.c1, tr.c2);
     }
-    tc_pair<N, NRM, T>(a, j, a.k, a.first != 0, Wt, lane, tr);
+    tc_pair<N, NRM, T, PAD>(a, j, a.k, a.first != 0, Wt, lane, tr);
   }
 }
 
@@ -1180,7 +1187,7 @@ __device__ void tree_root(const FactorArgs<double>& a, const TreeArgs& ta, int r
 // launch replaces two per level, whose fixed cost dominates there.
 constexpr int TOP_WARPS = 16;
 
-template <int N, int NRM>
+template <int N, int NRM, bool PAD = false>
 __global__ void __launch_bounds__(TOP_WARPS * 32, 1) k_factor_top_tc(FactorArgs<double> a, int k_first) {
   using S = TcShape<N>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1188,11 +1195,11 @@ __global__ void __launch_bounds__(TOP_WARPS * 32, 1) k_factor_top_tc(FactorArgs<
   double* Wt = reinterpret_cast<double*>(smem_raw + (size_t)warp * S::BYTES);
   const TcTree none{0, 0, 0};
   const int nb = a.d.nblock;
-  const size_t nrn = (size_t)a.d.nr * N;
+  const size_t nrn = (size_t)a.d.nr * a.d.n;
   for (int k = k_first; k < nb; k *= 2) {
     const long np = pairs_at_level(nb, k);
     for (long q = warp; q < np; q += TOP_WARPS)
-      tc_pair<N, NRM>(a, k + (int)(2L * k * q), k, k == 1, Wt, lane, none);
+      tc_pair<N, NRM, double, PAD>(a, k + (int)(2L * k * q), k, k == 1, Wt, lane, none);
     __syncthreads();
     for (size_t e = threadIdx.x; e < (size_t)np * nrn; e += blockDim.x) {
       const long q = (long)(e / nrn);
@@ -2458,6 +2465,7 @@ __global__ void __launch_bounds__(256, 2) k_forward_rows(SweepArgs<TF> a0, const
     const int n = d.n, nr = d.nr, n2 = 2 * n, nrhs = a.nrhs, k = a.k;
     const bool act = lane < n2;
     constexpr bool lu = LU;
+    const bool op = a0.op != 0;
     for (long q = q0; q < q1; q += qs) {
       const int j = k + (int)(2L * k * q), jp = j - k;
       const TF* Tj = a.Tm + (size_t)j * szT(d);
@@ -2476,7 +2484,17 @@ __global__ void __launch_bounds__(256, 2) k_forward_rows(SweepArgs<TF> a0, const
         double* xc = a.x + (size_t)col * a.ldx;
         const double orig = act ? (lane < n ? xc[(size_t)jp * n + lane] : xc[(size_t)j * n + lane - n]) : 0.0;
         double w = __shfl_sync(FULL, orig, src);
-        if (lu) {
+        const double b = w;
+        if (lu && op) {  // the operator form: one product (see k_forward_pipe)
+          double w2 = 0.0;
+  #pragma unroll
+          for (int i = 0; i < N; i += 2) {
+            const double b0 = __shfl_sync(FULL, b, i), b1 = __shfl_sync(FULL, b, i + 1);
+            if (i < n && lane > i) w = fma(t[i], b0, w);
+            if (i + 1 < n && lane > i + 1) w2 = fma(t[i + 1], b1, w2);
+          }
+          w += w2;
+        } else if (lu) {
   #pragma unroll
           for (int i = 0; i < N; ++i) {
             if (i < n) {
@@ -2498,12 +2516,12 @@ __global__ void __launch_bounds__(256, 2) k_forward_rows(SweepArgs<TF> a0, const
           if (lane < n) xc[(size_t)j * n + lane] = w;
           else xc[(size_t)jp * n + lane - n] = w;
         }
-        const double wt = lane < n ? w : 0.0;
+        const double wt = lane < n ? (lu && op ? b : -w) : 0.0;
   #pragma unroll
         for (int r = 0; r < NRM; ++r) {
           if (r < nr) {
             const double sr = warp_sum(cp[r] * wt);
-            if (lane == 0) a.XB[(size_t)j * nr * nrhs + (size_t)col * nr + r] = -sr;
+            if (lane == 0) a.XB[(size_t)j * nr * nrhs + (size_t)col * nr + r] = sr;
           }
         }
       }
@@ -4013,11 +4031,17 @@ struct FactorPlan {
 };
 
 // the warp-per-pair LU kernel eliminates the pairs of this state (its factors
-// are in operator form, which the forward sweep has to know).  The tree and
-// gather schedules are FP64 only.
+// are in operator form, which the forward sweep has to know).  Orders other than
+// 8 and 16 run as their leading parts: at n = 12, 20,011 blocks, level 1 takes
+// 82 us against 148 in the register kernel (k_factor_lu_rows), a lone pair 11
+// against 16 us; up to n = 4 with borders it takes, that kernel stays.  The tree
+// and gather schedules are FP64 only and unpadded.
 static bool tc_pair_selected(const DevState& s) {
   const Dims d = s.d;
-  if (s.sel != SEL_LU || d.nr > 8 || d.nx > 8 || (d.n != 16 && d.n != 8) || !s.use_tc) return false;
+  if (s.sel != SEL_LU || d.nr > 8 || d.nx > 8 || !s.use_tc) return false;
+  if (d.n != 16 && d.n != 8)  // padded to 8 or 16
+    return d.n < 16 && (s.pair_kernel == PAIR_AUTO || s.pair_kernel == PAIR_TC) &&
+           (d.n > 4 || d.nr > 4 || d.nx > 4);
   return s.pair_kernel == PAIR_AUTO || s.pair_kernel == PAIR_TC ||
          (!s.mixed && (s.pair_kernel == PAIR_TREE || s.pair_kernel == PAIR_TC_GATHER));
 }
@@ -4037,19 +4061,26 @@ static FactorPlan<T> plan_factor(const DevState& s) {
   if (p.smem <= SMEM_MAX) smem_limit_once(p.smem_k, p.smem);
   if constexpr (sizeof(T) == 8) {
     if (tc_pair_selected(s)) {
-      p.tc_smem = tc_smem_per_warp(n) * 4;
+      const int N = n <= 8 ? 8 : 16;
+      p.tc_smem = tc_smem_per_warp(N) * 4;
       // border rows spread over the warp: 8 lanes per row when nr <= 4, else 4
       const bool r4 = d.nr <= 4;
-      if (n == 16) p.tc = r4 ? k_factor_lu_tc<16, false, false, 4> : k_factor_lu_tc<16, false, false, 8>;
+      if (n != N) {
+        if (N == 16) p.tc = r4 ? k_factor_lu_tc<16, false, false, 4, T, true> : k_factor_lu_tc<16, false, false, 8, T, true>;
+        else p.tc = r4 ? k_factor_lu_tc<8, false, false, 4, T, true> : k_factor_lu_tc<8, false, false, 8, T, true>;
+      } else if (n == 16) p.tc = r4 ? k_factor_lu_tc<16, false, false, 4> : k_factor_lu_tc<16, false, false, 8>;
       else p.tc = r4 ? k_factor_lu_tc<8, false, false, 4> : k_factor_lu_tc<8, false, false, 8>;
       smem_limit_once(p.tc, p.tc_smem);
-      p.tc_cols = n == 16 ? TcShape<16>::NTP : TcShape<8>::NTP;
+      p.tc_cols = 2 * n + 8;
       if (s.tree_cnt) {  // single systems (batches keep their own level loop)
-        if (n == 16) p.top = r4 ? k_factor_top_tc<16, 4> : k_factor_top_tc<16, 8>;
+        if (n != N) {
+          if (N == 16) p.top = r4 ? k_factor_top_tc<16, 4, true> : k_factor_top_tc<16, 8, true>;
+          else p.top = r4 ? k_factor_top_tc<8, 4, true> : k_factor_top_tc<8, 8, true>;
+        } else if (n == 16) p.top = r4 ? k_factor_top_tc<16, 4> : k_factor_top_tc<16, 8>;
         else p.top = r4 ? k_factor_top_tc<8, 4> : k_factor_top_tc<8, 8>;
-        smem_limit_once(p.top, tc_smem_per_warp(n) * TOP_WARPS);
+        smem_limit_once(p.top, tc_smem_per_warp(N) * TOP_WARPS);
       }
-      if (s.pair_kernel == PAIR_TC_GATHER && s.tree_cnt && d.nblock >= 2) {
+      if (s.pair_kernel == PAIR_TC_GATHER && n == N && s.tree_cnt && d.nblock >= 2) {
         if (n == 16) p.tcb = r4 ? k_factor_lu_tc<16, false, true, 4> : k_factor_lu_tc<16, false, true, 8>;
         else p.tcb = r4 ? k_factor_lu_tc<8, false, true, 4> : k_factor_lu_tc<8, false, true, 8>;
         p.root = n == 16 ? k_tree_root<16> : k_tree_root<8>;
@@ -4058,7 +4089,7 @@ static FactorPlan<T> plan_factor(const DevState& s) {
       // the tree schedule (single systems with at least one pair), on request:
       // its top levels run one pair per warp along a serial chain, which costs
       // more than the level-by-level launches save at the sizes measured
-      if (s.pair_kernel == PAIR_TREE && s.tree_cnt && d.nblock >= 2) {
+      if (s.pair_kernel == PAIR_TREE && n == N && s.tree_cnt && d.nblock >= 2) {
         if (n == 16) p.tree = r4 ? k_factor_tree_tc<16, 4> : k_factor_tree_tc<16, 8>;
         else p.tree = r4 ? k_factor_tree_tc<8, 4> : k_factor_tree_tc<8, 8>;
         smem_limit_once(p.tree, p.tc_smem);
@@ -4069,12 +4100,16 @@ static FactorPlan<T> plan_factor(const DevState& s) {
     // FP32 factors (mixed path): the same warp-per-pair kernel with FP32
     // products, level by level, no fused right-hand sides
     if (tc_pair_selected(s)) {
-      p.tc_smem = tc_smem_per_warp_t<T>(n) * 4;
+      const int N = n <= 8 ? 8 : 16;
+      p.tc_smem = tc_smem_per_warp_t<T>(N) * 4;
       const bool r4 = d.nr <= 4;
-      if (n == 16) p.tc = r4 ? k_factor_lu_tc<16, false, false, 4, T> : k_factor_lu_tc<16, false, false, 8, T>;
+      if (n != N) {
+        if (N == 16) p.tc = r4 ? k_factor_lu_tc<16, false, false, 4, T, true> : k_factor_lu_tc<16, false, false, 8, T, true>;
+        else p.tc = r4 ? k_factor_lu_tc<8, false, false, 4, T, true> : k_factor_lu_tc<8, false, false, 8, T, true>;
+      } else if (n == 16) p.tc = r4 ? k_factor_lu_tc<16, false, false, 4, T> : k_factor_lu_tc<16, false, false, 8, T>;
       else p.tc = r4 ? k_factor_lu_tc<8, false, false, 4, T> : k_factor_lu_tc<8, false, false, 8, T>;
       smem_limit_once(p.tc, p.tc_smem);
-      p.tc_cols = n == 16 ? TcShape<16, T>::NTP : TcShape<8, T>::NTP;
+      p.tc_cols = 2 * n + 8;
     }
   }
   const bool grp_ok = s.sel == SEL_LU && d.nr <= 8 && d.nx <= 8 &&
@@ -4223,7 +4258,7 @@ static bool factor_levels(DevState& s, const FactorPlan<T>& p, const WorkSet<T>&
     const long np = pairs_at_level(nb, k);
     if constexpr (sizeof(T) == 8) {
       if (p.tc && p.top && np <= TOP_WARPS) {  // this level and every one above it
-        p.top<<<1, TOP_WARPS * 32, tc_smem_per_warp(n) * TOP_WARPS, st>>>(a, k);
+        p.top<<<1, TOP_WARPS * 32, tc_smem_per_warp(n <= 8 ? 8 : 16) * TOP_WARPS, st>>>(a, k);
         check_launch("k_factor_top_tc");
         break;
       }

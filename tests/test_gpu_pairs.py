@@ -139,3 +139,24 @@ def test_qr_zero_column_is_reported(select):
     assert not h.factorize()
     check(s, synth.rhs(s, 1, seed=4), select)
 
+
+@pytest.mark.parametrize("n", [1, 4, 5, 7, 9, 12, 15])
+@pytest.mark.parametrize("nr,nx", [(0, 0), (3, 4), (8, 8)])
+@pytest.mark.parametrize("nblock", [2, 3, 40])
+def test_padded_warp_lu(n, nr, nx, nblock):
+    """Orders between the warp kernel's 8 and 16, as leading parts of such blocks:
+    factorize + solve with the right-hand sides in the factorization (up to 8 - nx)
+    and apart from it.  cond(A) <= 4e4 (dense SVD)."""
+    s = synth.collocation(nblock, n, max(0, nx - nr), max(0, nr - nx), nr, nx, seed=n)
+    check(s, synth.rhs(s, 4, seed=n + 1), bar=1e-9)
+    if nr + max(0, nx - nr) == nx + max(0, nr - nx):
+        rhs = synth.rhs(s, 1, seed=n + 2)
+        o = po.Oracle(s, "LU", "LU")
+        assert o.factorize(), o.last_error()
+        h = B.BorderedCR()
+        h.load_system(s)
+        h.set_precision(B.PRECISION_MIXED)
+        h.set_refinement(1e-15, 10)
+        x = rhs.copy()
+        assert h.factorize_solve(1, x.reshape(-1), x.shape[1]), h.last_error()
+        assert fwd_err(x[0, :s.ncols], o.solve(rhs)[0, :s.ncols]) < 1e-9
