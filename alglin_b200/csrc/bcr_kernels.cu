@@ -76,6 +76,48 @@ __device__ __forceinline__ T ldro(const T* p) {
   else return __ldg(p);
 }
 
+// Element of a batch of loads, 0 where p is false.  volatile keeps the loads of
+// an unrolled batch together: scheduled by the compiler, each one waits for the
+// use of the one before (the same 262 KB read by one CTA: 80,000 cycles from
+// DRAM, against 13,000).
+__device__ __forceinline__ double ld_batch(bool p, const double* a) {
+  double v;
+  asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; mov.f64 %0, 0d0000000000000000; @q ld.global.f64 %0, [%1]; }\n"
+               : "=d"(v)
+               : "l"(a), "r"((unsigned)p));
+  return v;
+}
+__device__ __forceinline__ float ld_batch(bool p, const float* a) {
+  float v;
+  asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; mov.f32 %0, 0f00000000; @q ld.global.f32 %0, [%1]; }\n"
+               : "=f"(v)
+               : "l"(a), "r"((unsigned)p));
+  return v;
+}
+
+// the same through L2 (elements that another CTA of the launch may have written)
+__device__ __forceinline__ double ld_batch_cg(bool p, const double* a) {
+  double v;
+  asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; mov.f64 %0, 0d0000000000000000; @q ld.global.cg.f64 %0, [%1]; }\n"
+               : "=d"(v)
+               : "l"(a), "r"((unsigned)p)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_batch_cg(bool p, const float* a) {
+  float v;
+  asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; mov.f32 %0, 0f00000000; @q ld.global.cg.f32 %0, [%1]; }\n"
+               : "=f"(v)
+               : "l"(a), "r"((unsigned)p)
+               : "memory");
+  return v;
+}
+template <bool COH, typename T>
+__device__ __forceinline__ T ld_batch_c(bool p, const T* a) {
+  if constexpr (COH) return ld_batch_cg(p, a);
+  else return ld_batch(p, a);
+}
+
 // Pair range of one worker (warp or CTA).  Single system: a grid-stride loop
 // over the level's pairs.  Batch: map entry e (by default the CTA's index)
 // holds pairs [q0, q1) of system cmap[e].sys, whose arguments come from the
@@ -1258,14 +1300,23 @@ __global__ void __launch_bounds__(128, 4) k_factor_tree_tc(FactorArgs<double> a,
   }
 }
 
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int K>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(K) : "memory"); }
+
 // ---------------------------------------------------------------------------
-// LU pair kernel for n = 16 and n = 32 in either precision.  One CTA per
-// pair: 2n panel threads (one panel row each, in registers) plus one warp
-// whose first nr lanes hold the border rows C_j.  Three phases as in the
-// tensor-core kernel: register panel LU with the getrf pivot rule (the pivot
-// search spans the panel warps: each publishes its best candidate row and its
-// reciprocal, one barrier per column, double-buffered by column parity); the
-// operator G = [L^-1; -M L^-1; -C' L^-1]; one product G * (P W)_top, on the
+// LU pair kernel for n = 16 and n = 32 in either precision, and for 16 < n < 32
+// padded.  One CTA per pair: 2N panel threads (one panel row each, in registers)
+// plus one warp whose first nr lanes hold the border rows C_j.  As in the
+// warp-per-pair kernel: register panel LU with the getrf pivot rule (the pivot
+// search spans the panel warps: each posts its best candidate row and its
+// reciprocal, one barrier per column, double-buffered by column parity) that
+// keeps the operator G = [L^-1; -M L^-1; -C' L^-1] in the eliminated columns;
+// then one product G * (P W)_top, on the
 // FP64 tensor cores (DMMA 8x8x4) for double, as a 3xTF32 split on the tensor
 // cores for float at n = 32, on the FP32 pipe for float at n = 16.
 // ---------------------------------------------------------------------------
@@ -1505,122 +1556,157 @@ struct GrpProduct<float, 32> {
 template <typename T, int N>
 constexpr int grp_min_blocks() { return N == 32 ? (sizeof(T) == 8 ? 5 : 6) : 4; }
 
-// pairs [q0, q1) step qs of one system and level, one per CTA
-template <typename T, int N, bool COH>
+// 8-byte asynchronous copy to shared memory (completion: cp_async_wait)
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+
+// Pairs [q0, q1) step qs of one system and level, one per CTA.  PAD: blocks of
+// order n < N as the leading part of blocks of order N (see tc_pair).
+//
+// The pivot steps are one rolled loop over rotating registers (a step moves every
+// column one register down and puts the operator's new column at the end, as in
+// lub_panel), so that its code stays in the instruction cache: unrolled, with the
+// triangular solve that the operator then needed, instruction fetch was the
+// largest stall (3.3 of 12 cycles per issue, now 0.5).  The trailing columns
+// arrive by asynchronous copies while the panel is factored.  n = 32, 8,192
+// pairs: FP64 596 -> 509 us, FP32 506 -> 406 us; n = 20 (padded), 10,000 pairs:
+// 728 us in the shared-memory kernel, 492 us.  Bound by the step's chain of
+// reductions and its barrier.
+template <typename T, int N, bool COH, bool PAD = false>
 __device__ __forceinline__ void grp_body(const FactorArgs<T>& a, long q0, long q1, long qs) {
   using S = GrpShape<T, N>;
   constexpr unsigned FULL = 0xffffffffu;
+  constexpr bool ASYNC = sizeof(T) == 8 && !COH;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int s_info;
   T* Wt = reinterpret_cast<T*>(smem_raw);          // [2N][LDW] trailing columns, original rows
-  T* Gs = Wt + 2 * N * S::LDW;                     // [MT][LDG] L rows, then G
-  T* slot = Gs + S::MT * S::LDG;                   // [2][NWP][LDS] candidate pivot row + reciprocal
-  int* hdr = reinterpret_cast<int*>(slot + 2 * S::NWP * S::LDS);  // [2][NWP][4] hi, lo, position, thread
-  int* rowof = hdr + 2 * S::NWP * 4;               // position -> original row
+  T* Gs = Wt + 2 * N * S::LDW;                     // [MT][LDG] operator rows
+  T* slot = Gs + S::MT * S::LDG;                   // [2][NWP][LDS] candidate: reciprocal, then its row from the next column on
+  int* hdr = reinterpret_cast<int*>(slot + 2 * S::NWP * S::LDS);  // [2][NWP][4] |a| (two words), position and thread
+  int* rowof = hdr + 2 * S::NWP * 4;               // row of the product -> panel row
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const Dims d = a.d;
   const int nr = d.nr, nx = d.nx;
-  constexpr int n = N, n2 = 2 * N;
-  constexpr size_t nn = (size_t)N * N;
+  const int n = PAD ? d.n : N, n2 = 2 * n;
+  const size_t nn = (size_t)n * n;
   const size_t nnx = (size_t)n * nx, nrn = (size_t)nr * n, nrnx = (size_t)nr * nx;
   const int k = a.k;
   const bool first = a.first != 0;
-  const bool panel = t < n2;                 // panel row t
-  const bool brow = !panel && t - n2 < nr;   // border row t - 2N
-  const bool top = t < n;
-  const int ri = top ? t : t - n;
+  const bool panel = t < 2 * N;                 // panel row t
+  const bool top = t < N;
+  const int ri = t & (N - 1);
+  const bool act = panel && ri < n;
+  const bool brow = !panel && t - 2 * N < nr;   // border row t - 2N
+  const int pos0 = act ? (top ? ri : n + ri) : 255;
 
   for (long qq = q0; qq < q1; qq += qs) {
     const int j = k + (int)(2L * k * qq), jp = j - k;
     __syncthreads();  // the previous pair's readers of Wt/Gs are done
+    if (t == 0) s_info = 0;
+    if (PAD && t < 2 * N) rowof[t] = 0;  // rows of the product that no panel row fills
     // ------------------------------------------------------------ load
-    // every global load of the pair is issued before the first shared store
-    constexpr int IT = (int)((nn + S::NTH - 1) / S::NTH), IB = (8 * N + S::NTH - 1) / S::NTH;
-    T row[N], vd[IT], ve[IT], vbt[IB], vbb[IB];
-    // the source (loaded FP64 matrix at the first level, working copy after)
-    // is chosen once per pair, so every load below is a plain batched load
+    T row[N];
     auto load = [&](const auto* D, const auto* E, const auto* Bm, const auto* C) {
-      if (panel) {
-        const size_t base = top ? (size_t)jp * nn : (size_t)j * nn;
-        const auto* P = top ? E : D;
+      // trailing columns, compact: TOP rows [D_jp B_jp], BOTTOM rows [E_j B_j]; one
+      // element of both per thread and round
+      constexpr int IT = (N * N + S::NTH - 1) / S::NTH, IB = (8 * N + S::NTH - 1) / S::NTH;
+      if constexpr (ASYNC) {
 #pragma unroll
-        for (int c = 0; c < N; ++c) row[c] = T(ldro<COH>(P + base + (size_t)c * n + ri));
-      } else {
+        for (int it = 0; it < IT; ++it) {
+          const int idx = t + S::NTH * it, r = idx & (N - 1), c = idx / N;
+          if (idx < N * N && (!PAD || (r < n && c < n))) {
+            cp_async8(Wt + r * S::LDW + c, D + (size_t)jp * nn + (size_t)c * n + r);
+            cp_async8(Wt + (N + r) * S::LDW + c, E + (size_t)j * nn + (size_t)c * n + r);
+          }
+        }
 #pragma unroll
-        for (int c = 0; c < N; ++c)
-          row[c] = brow ? T(ldro<COH>(C + (size_t)j * nrn + (size_t)c * nr + (t - n2))) : T(0);
+        for (int it = 0; it < IB; ++it) {
+          const int idx = t + S::NTH * it, r = idx & (N - 1), c = idx / N;
+          if (c < nx && (!PAD || r < n)) {
+            cp_async8(Wt + r * S::LDW + N + c, Bm + (size_t)jp * nnx + (size_t)c * n + r);
+            cp_async8(Wt + (N + r) * S::LDW + N + c, Bm + (size_t)j * nnx + (size_t)c * n + r);
+          }
+        }
+        cp_async_commit();
       }
+      {
+        const auto* P = panel ? (top ? E + (size_t)jp * nn : D + (size_t)j * nn) + ri
+                              : C + (size_t)j * nrn + (t - 2 * N);
+        const int st = panel ? n : nr;
 #pragma unroll
-      for (int it = 0; it < IT; ++it) {
-        const int idx = t + S::NTH * it;
-        const bool in = idx < (int)nn;
-        vd[it] = in ? T(ldro<COH>(D + (size_t)jp * nn + idx)) : T(0);
-        ve[it] = in ? T(ldro<COH>(E + (size_t)j * nn + idx)) : T(0);
+        for (int c = 0; c < N; ++c) row[c] = T(ld_batch_c<COH>((act || brow) && (!PAD || c < n), P + (size_t)c * st));
       }
+      if constexpr (!ASYNC) {
+        constexpr int H = 4;  // rounds in flight
+        for (int i0 = 0; i0 < IT; i0 += H) {
+          T vd[H], ve[H];
 #pragma unroll
-      for (int it = 0; it < IB; ++it) {
-        const int idx = t + S::NTH * it;
-        const bool in = idx < nx * n;
-        vbt[it] = in ? T(ldro<COH>(Bm + (size_t)jp * nnx + idx)) : T(0);
-        vbb[it] = in ? T(ldro<COH>(Bm + (size_t)j * nnx + idx)) : T(0);
+          for (int u = 0; u < H; ++u) {
+            const int idx = t + S::NTH * (i0 + u), r = idx & (N - 1), c = idx / N;
+            const bool in = idx < N * N && (!PAD || (r < n && c < n));
+            vd[u] = T(ld_batch_c<COH>(in, D + (size_t)jp * nn + (size_t)c * n + r));
+            ve[u] = T(ld_batch_c<COH>(in, E + (size_t)j * nn + (size_t)c * n + r));
+          }
+#pragma unroll
+          for (int u = 0; u < H; ++u) {
+            const int idx = t + S::NTH * (i0 + u), r = idx & (N - 1), c = idx / N;
+            if (idx < N * N) {
+              Wt[r * S::LDW + c] = vd[u];
+              Wt[(N + r) * S::LDW + c] = ve[u];
+            }
+          }
+        }
+        T vt[IB], vb[IB];
+#pragma unroll
+        for (int it = 0; it < IB; ++it) {
+          const int idx = t + S::NTH * it, r = idx & (N - 1), c = idx / N;
+          const bool in = c < nx && (!PAD || r < n);
+          vt[it] = T(ld_batch_c<COH>(in, Bm + (size_t)jp * nnx + (size_t)c * n + r));
+          vb[it] = T(ld_batch_c<COH>(in, Bm + (size_t)j * nnx + (size_t)c * n + r));
+        }
+#pragma unroll
+        for (int it = 0; it < IB; ++it) {
+          const int idx = t + S::NTH * it, r = idx & (N - 1), c = idx / N;
+          if (c < 8) {
+            Wt[r * S::LDW + N + c] = vt[it];
+            Wt[(N + r) * S::LDW + N + c] = vb[it];
+          }
+        }
       }
     };
     if (first) load(a.D0, a.E0, a.B0, a.C0);
     else load(a.D, a.E, a.B, a.C);
-
-    // trailing columns, compact: TOP rows [D_jp B_jp], BOTTOM rows [E_j B_j]
-#pragma unroll
-    for (int it = 0; it < IT; ++it) {
-      const int idx = t + S::NTH * it;
-      if (idx < (int)nn) {
-        const int r = idx % n, c = idx / n;
-        Wt[r * S::LDW + c] = vd[it];
-        Wt[(n + r) * S::LDW + c] = ve[it];
-      }
-    }
-#pragma unroll
-    for (int it = 0; it < IB; ++it) {
-      const int idx = t + S::NTH * it;
-      if (idx < 8 * n) {
-        const int r = idx % n, c = idx / n;
-        Wt[r * S::LDW + n + c] = vbt[it];
-        Wt[(n + r) * S::LDW + n + c] = vbb[it];
-      }
-    }
-    // --------------------------------------------------- phase 1: panel LU
-    int mypos = t, info = 0;
-    bool done = !panel;  // border and idle lanes never pivot
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
+    // ------------------- phase 1: panel LU with the operator rows in place
+    int mypos = pos0;
+    bool done = !act, used = false;  // border and idle lanes never pivot
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+      // row[0] is column i
       const int par = i & 1;
+      const T v0 = row[0];
       if (w < S::NWP) {
-        // every lane forms the reciprocal of its own candidate while the pivot
-        // is searched; the winner publishes it with its row
-        const T rc = rcp_rn(row[i]);
         unsigned hi, lo;
-        pivot_key(dev_abs(row[i]), done, hi, lo);
+        T rc;
+        tc_candidate(v0, done, hi, lo, rc);
         const unsigned hmax = __reduce_max_sync(FULL, hi);
-        const unsigned m = __ballot_sync(FULL, hi == hmax && !done);
-        int wl = -1;  // this warp's best candidate lane
-        if (m != 0u) {
-          if (__popc(m) == 1) {
-            wl = __ffs(m) - 1;
-          } else {
-            const bool c1 = hi == hmax && !done;
-            const unsigned lmax = __reduce_max_sync(FULL, c1 ? lo : 0u);
-            const bool cand = c1 && lo == lmax;
-            const unsigned pm = __reduce_min_sync(FULL, cand ? (unsigned)mypos : 0xffffffffu);
-            wl = __ffs(__ballot_sync(FULL, cand && (unsigned)mypos == pm)) - 1;
-          }
+        unsigned lmax = 0u;
+        bool in = hi == hmax && !done;
+        if constexpr (sizeof(T) == 8) {
+          lmax = __reduce_max_sync(FULL, hi == hmax ? lo : 0u);
+          in = in && lo == lmax;
         }
-        int4* h = reinterpret_cast<int4*>(hdr) + par * S::NWP + w;
-        T* sl = slot + (par * S::NWP + w) * S::LDS;
-        if (lane == wl) {
-          *h = make_int4((int)hi, (int)lo, mypos, t);
+        const unsigned best = __reduce_min_sync(FULL, in ? ((unsigned)mypos << 5) | lane : 0xffffffffu);
+        if (hmax != 0u && !tc_plain_pivot<T>(hmax)) rc = v0 != T(0) ? rcp_rn(v0) : T(0);
+        // where no candidate is left (hmax = 0, best all ones) lane 31 posts zeros
+        if ((best & 31u) == (unsigned)lane) {
+          reinterpret_cast<int4*>(hdr)[par * S::NWP + w] =
+              make_int4((int)hmax, (int)lmax, (int)((best >> 5 << 8) | t), 0);
+          T* sl = slot + (par * S::NWP + w) * S::LDS;
+          store2(sl, rc, row[1]);
 #pragma unroll
-          for (int c = (i & ~1); c < N; c += 2) store2(sl + c, row[c], row[c + 1]);
-          sl[N] = rc;
-        } else if (wl < 0 && lane == 0) {
-          *h = make_int4(0, 0, 0x7fffffff, 0);  // no candidate left in this warp
+          for (int c = 2; c < N; c += 2) store2(sl + c, row[c], row[c + 1]);
         }
       }
       __syncthreads();
@@ -1635,95 +1721,92 @@ __device__ __forceinline__ void grp_body(const FactorArgs<T>& a, long q0, long q
           hw = h1;
         }
       }
-      const int pmin = hw.z, p = hw.w;
+      const int p = hw.z & 255, pmin = (hw.z >> 8) & 255;
       const T* u = slot + (par * S::NWP + wb) * S::LDS;
-      const T piv = u[i];
-      if (piv == T(0) && info == 0) info = i + 1;
-      const T rinv = piv != T(0) ? u[N] : T(0);
-      if (panel) {
-        if (!done && mypos == i && t != p) mypos = pmin;
-        if (t == p) mypos = i;
+      mypos = mypos == i ? pmin : mypos;
+      if (t == p) {
+        mypos = i;
+        done = used = true;
+        if (v0 == T(0) && s_info == 0) s_info = i + 1;
       }
-      if ((panel && !done && t != p) || brow) {
-        const T l = row[i] * rinv;
-        row[i] = l;
+      T u0, u1;
+      load2(u, u0, u1);
+      const T l = used ? T(0) : v0 * u0;
+      row[0] = fma(-l, u1, row[1]);
 #pragma unroll
-        for (int c = (i + 1) & ~1; c < N; c += 2) {
-          T u0, u1;
-          load2(u + c, u0, u1);
-          if (c > i) row[c] = fma(-l, u0, row[c]);
-          row[c + 1] = fma(-l, u1, row[c + 1]);
-        }
+      for (int c = 2; c < N; c += 2) {
+        load2(u + c, u0, u1);
+        row[c - 1] = fma(-l, u0, row[c]);
+        row[c] = fma(-l, u1, row[c + 1]);
       }
-      if (t == p) done = true;
+      row[N - 1] = used ? v0 : -l;
     }
-    if (info != 0) {
-      if (t == 0) report(a.st, DEV_ZERO_PIVOT, j, info, k);
+    if (PAD) {  // the rest of the rotation
+#pragma unroll 1
+      for (int i = n; i < N; ++i) {
+        const T v0 = row[0];
+#pragma unroll
+        for (int c = 1; c < N; ++c) row[c - 1] = row[c];
+        row[N - 1] = v0;
+      }
+    }
+    // panel factors T_j in getrf row order (operator form), row map, the border
+    // operator; operator rows for the product (pivot rows: unit lower triangle)
+    __syncthreads();
+    if (s_info != 0) {
+      if (t == 0) report(a.st, DEV_ZERO_PIVOT, j, s_info, k);
+      if constexpr (ASYNC) cp_async_wait<0>();
       continue;
     }
-    // panel factors T_j (L\U and M in getrf row order), row map, C_j U^-1, L rows
-    if (panel) {
+    if (act) {
       T* Tj = a.Tm + (size_t)j * szT(d);
 #pragma unroll
-      for (int c = 0; c < N; ++c) Tj[(size_t)mypos + (size_t)c * n2] = row[c];
-      rowof[mypos] = t;
-      a.P[(size_t)j * szP(d) + mypos] = (unsigned char)t;
-      if (mypos < n) {
+      for (int c = 0; c < N; ++c)
+        if (!PAD || c < n) Tj[(size_t)mypos + (size_t)c * n2] = row[c];
+      const int gr = mypos < n ? mypos : mypos - n + N;
+      rowof[gr] = t;
+      a.P[(size_t)j * szP(d) + mypos] = (unsigned char)pos0;
+      T* G = Gs + gr * S::LDG;
+      const int dg = mypos < n ? mypos : N;  // unit diagonal
 #pragma unroll
-        for (int c = 0; c < N; ++c) Gs[mypos * S::LDG + c] = row[c];
-      }
-    } else if (brow) {
-      T* Cj = a.C + (size_t)j * nrn + (t - n2);
+      for (int c = 0; c < N; c += 2)
+        store2(G + c, c < dg ? row[c] : c == dg ? T(1) : T(0), c + 1 < dg ? row[c + 1] : c + 1 == dg ? T(1) : T(0));
+    } else if (!panel && t - 2 * N < 8) {
+      T* Cj = a.C + (size_t)j * nrn + (t - 2 * N);
+      T* G = Gs + t * S::LDG;
 #pragma unroll
-      for (int c = 0; c < N; ++c) Cj[(size_t)c * nr] = row[c];
-    }
-    __syncthreads();
-    // ------------------------------------ phase 2: operator G (X L = R)
-    // R rows: identity for U-row positions, -M for reduced positions, -C' for border rows
-    {
-      T x[N];
-      const bool unit = panel && mypos < n;
-#pragma unroll
-      for (int c = 0; c < N; ++c) x[c] = unit ? (c == mypos ? T(1) : T(0)) : -row[c];
-      // right-looking: once x[mm] is final, update every x[c], c < mm
-#pragma unroll
-      for (int mm = N - 1; mm > 0; --mm) {
-        const T xm = x[mm];
-        const T* Lrow = Gs + mm * S::LDG;
-#pragma unroll
-        for (int c = 0; c < mm; c += 2) {
-          const T l0 = Lrow[c], l1 = Lrow[c + 1];
-          x[c] = fma(-xm, l0, x[c]);
-          if (c + 1 < mm) x[c + 1] = fma(-xm, l1, x[c + 1]);
-        }
-      }
-      __syncthreads();
-      const int grow = panel ? mypos : n2 + (t - n2);
-      if (panel || t - n2 < 8) {
-#pragma unroll
-        for (int c = 0; c < N; ++c) Gs[grow * S::LDG + c] = (panel || brow) ? x[c] : T(0);
+      for (int c = 0; c < N; ++c) {
+        if (brow && (!PAD || c < n)) Cj[(size_t)c * nr] = row[c];
+        G[c] = brow ? row[c] : T(0);
       }
     }
+    if constexpr (ASYNC) cp_async_wait<0>();
     __syncthreads();
-    // ------------------------------------------ phase 3: G * (P W)_top
+    // ------------------------------------------ phase 2: G * (P W)_top
     GrpProduct<T, N>::run(Wt, Gs, rowof, t, [&](int prow, int col, T v) {
-      if (prow < n2) {
-        const bool ur = prow < n;
-        const int rr = ur ? prow : prow - n;
+      const int cj = col < N ? col : col < 2 * N ? col - N : col - 2 * N;
+      if (prow < 2 * N) {
+        const bool ur = prow < N;
+        const int rr = ur ? prow : prow - N;
         const size_t blk = ur ? (size_t)j : (size_t)jp;
-        if (col < n) a.D[blk * nn + (size_t)col * n + rr] = v;
-        else if (col < n2) a.E[blk * nn + (size_t)(col - n) * n + rr] = v;
-        else if (col < n2 + nx) a.B[blk * nnx + (size_t)(col - n2) * n + rr] = v;
+        if (PAD && rr >= n) return;
+        if (col < N) {
+          if (!PAD || cj < n) a.D[blk * nn + (size_t)cj * n + rr] = v;
+        } else if (col < 2 * N) {
+          if (!PAD || cj < n) a.E[blk * nn + (size_t)cj * n + rr] = v;
+        } else if (cj < nx) {
+          a.B[blk * nnx + (size_t)cj * n + rr] = v;
+        }
       } else {
-        const int rr = prow - n2;
+        const int rr = prow - 2 * N;
         if (rr < nr) {
-          if (col < n) {
-            const size_t o = (size_t)jp * nrn + (size_t)col * nr + rr;
-            a.C[o] = ldsrc_c<COH>(first, a.C0, a.C, o) + v;
-          } else if (col < n2) {
-            a.Rbuf[(size_t)j * nrn + (size_t)(col - n) * nr + rr] = v;
-          } else if (col < n2 + nx) {
-            a.Fbuf[(size_t)j * nrnx + (size_t)(col - n2) * nr + rr] = (double)v;
+          if (col < N) {
+            const size_t o = (size_t)jp * nrn + (size_t)cj * nr + rr;
+            if (!PAD || cj < n) a.C[o] = ldsrc_c<COH>(first, a.C0, a.C, o) + v;
+          } else if (col < 2 * N) {
+            if (!PAD || cj < n) a.Rbuf[(size_t)j * nrn + (size_t)cj * nr + rr] = v;
+          } else if (cj < nx) {
+            a.Fbuf[(size_t)j * nrnx + (size_t)cj * nr + rr] = (double)v;
           }
         }
       }
@@ -1731,13 +1814,13 @@ __device__ __forceinline__ void grp_body(const FactorArgs<T>& a, long q0, long q
   }
 }
 
-template <typename T, int N, bool BATCH = false>
+template <typename T, int N, bool BATCH = false, bool PAD = false>
 __global__ void __launch_bounds__(2 * N + 32, grp_min_blocks<T, N>())
     k_factor_lu_grp(FactorArgs<T> a0, const FactorArgs<T>* tab, const BatchCta* cmap) {
   FactorArgs<T> ab;  // this CTA's system (batch only)
   long q0, q1, qs;
   pair_range<BATCH>(a0, tab, cmap, 1, 0, ab, q0, q1, qs);
-  grp_body<T, N, false>(BATCH ? ab : a0, q0, q1, qs);
+  grp_body<T, N, false, PAD>(BATCH ? ab : a0, q0, q1, qs);
 }
 
 // ---------------------------------------------------------------------------
@@ -2205,25 +2288,6 @@ __global__ void __launch_bounds__(256) k_factor_cta(FactorArgs<T> a, T* slab, si
   }
 }
 
-// Element of a batch of loads, 0 where p is false.  volatile keeps the loads of
-// an unrolled batch together: scheduled by the compiler, each one waits for the
-// use of the one before (the same 262 KB read by one CTA: 80,000 cycles from
-// DRAM, against 13,000).
-__device__ __forceinline__ double ld_batch(bool p, const double* a) {
-  double v;
-  asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; mov.f64 %0, 0d0000000000000000; @q ld.global.f64 %0, [%1]; }\n"
-               : "=d"(v)
-               : "l"(a), "r"((unsigned)p));
-  return v;
-}
-__device__ __forceinline__ float ld_batch(bool p, const float* a) {
-  float v;
-  asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; mov.f32 %0, 0f00000000; @q ld.global.f32 %0, [%1]; }\n"
-               : "=f"(v)
-               : "l"(a), "r"((unsigned)p));
-  return v;
-}
-
 // copy of loaded FP64 blocks into the working precision
 template <typename T>
 __global__ void k_convert_blocks(const double* src, T* dst, size_t count) {
@@ -2613,14 +2677,6 @@ struct BwdBuf {
   static constexpr size_t BYTES = (size_t)2 * WORDS * sizeof(T);  // two buffers
 };
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int K>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(K) : "memory"); }
-
 // the factors of pair q (level stride k) into one buffer (every lane issues
 // its share), in 16-byte chunks of V elements; for n = 8, 16 every block (D',
 // E', B', the U columns of T) starts and ends on a 16-byte boundary in FP64
@@ -2989,12 +3045,14 @@ __global__ void __launch_bounds__(256, 2) k_forward_pipe(SweepArgs<T> a0, const 
 // 32 + i (forward) or U-row i (backward); x values are exchanged by shuffles
 // and every factor element is read once, coalesced
 // ---------------------------------------------------------------------------
+// Factors in operator form (k_factor_lu_grp): one product with the permuted rows,
+// 16 columns of both rows read in one batch, up to four right-hand sides on each.
 template <typename TF, int NRM, bool BATCH = false>
 __global__ void __launch_bounds__(256, 2) k_forward_rows32(SweepArgs<TF> a0, const SweepArgs<TF>* tab,
                                                            const BatchCta* cmap, const long* ecnt) {
   for_entries<BATCH>(ecnt, [&](long entry) {
     constexpr unsigned FULL = 0xffffffffu;
-    constexpr int n = 32, n2 = 64;
+    constexpr int n = 32, n2 = 64, RH = 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     SweepArgs<TF> ab;  // this CTA's system (batch only)
     long q0, q1, qs;
@@ -3007,32 +3065,63 @@ __global__ void __launch_bounds__(256, 2) k_forward_rows32(SweepArgs<TF> a0, con
       const TF* Tj = a.Tm + (size_t)j * szT(d);
       const unsigned char* Pj = a.P + (size_t)j * szP(d);
       const int s0 = Pj[lane], s1 = Pj[n + lane];  // original rows at positions lane, 32 + lane
-      double cp[NRM];
       const TF* Cj = a.C + (size_t)j * nr * n;
-  #pragma unroll
-      for (int r = 0; r < NRM; ++r) cp[r] = r < nr ? double(Cj[(size_t)lane * nr + r]) : 0.0;
-      for (int col = 0; col < nrhs; ++col) {
-        double* xc = a.x + (size_t)col * a.ldx;
-        const double ot = xc[(size_t)jp * n + lane], ob = xc[(size_t)j * n + lane];
-        const double a0t = __shfl_sync(FULL, ot, s0 & 31), a0b = __shfl_sync(FULL, ob, s0 & 31);
-        const double a1t = __shfl_sync(FULL, ot, s1 & 31), a1b = __shfl_sync(FULL, ob, s1 & 31);
-        double w0 = s0 < n ? a0t : a0b, w1 = s1 < n ? a1t : a1b;
-  #pragma unroll
-        for (int i = 0; i < n; ++i) {
-          const double wi = __shfl_sync(FULL, w0, i);
-          const double t0 = double(Tj[(size_t)i * n2 + lane]), t1 = double(Tj[(size_t)i * n2 + n + lane]);
-          if (lane > i) w0 = fma(-t0, wi, w0);
-          w1 = fma(-t1, wi, w1);
-        }
-        xc[(size_t)j * n + lane] = w0;
-        xc[(size_t)jp * n + lane] = w1;
-  #pragma unroll
-        for (int r = 0; r < NRM; ++r) {
-          if (r < nr) {
-            const double sr = warp_sum(cp[r] * w0);
-            if (lane == 0) a.XB[(size_t)j * nr * nrhs + (size_t)col * nr + r] = -sr;
+      for (int col0 = 0; col0 < nrhs; col0 += RH) {
+        const int nc = min(RH, nrhs - col0);
+        double* xc = a.x + (size_t)col0 * a.ldx;
+        double b[RH], w0[RH], w1[RH];
+        TF t0[16], t1[16], cp[NRM];
+        auto load = [&](int c0) {
+#pragma unroll
+          for (int u = 0; u < 16; ++u) {
+            t0[u] = ld_batch(lane > c0 + u, Tj + (size_t)(c0 + u) * n2 + lane);
+            t1[u] = ld_batch(true, Tj + (size_t)(c0 + u) * n2 + n + lane);
           }
+        };
+        load(0);
+#pragma unroll
+        for (int r = 0; r < NRM; ++r) cp[r] = ld_batch(r < nr, Cj + (size_t)lane * nr + r);
+        double ot[RH], ob[RH];
+#pragma unroll
+        for (int c = 0; c < RH; ++c) {
+          ot[c] = ld_batch(c < nc, xc + (size_t)c * a.ldx + (size_t)jp * n + lane);
+          ob[c] = ld_batch(c < nc, xc + (size_t)c * a.ldx + (size_t)j * n + lane);
         }
+#pragma unroll
+        for (int c = 0; c < RH; ++c)
+          if (c < nc) {
+            const double a0t = __shfl_sync(FULL, ot[c], s0 & 31), a0b = __shfl_sync(FULL, ob[c], s0 & 31);
+            const double a1t = __shfl_sync(FULL, ot[c], s1 & 31), a1b = __shfl_sync(FULL, ob[c], s1 & 31);
+            w0[c] = b[c] = s0 < n ? a0t : a0b;
+            w1[c] = s1 < n ? a1t : a1b;
+          }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+          for (int c = 0; c < RH; ++c)
+            if (c < nc) {
+#pragma unroll
+              for (int u = 0; u < 16; ++u) {
+                const double bi = __shfl_sync(FULL, b[c], 16 * h + u);
+                w0[c] = fma(double(t0[u]), bi, w0[c]);
+                w1[c] = fma(double(t1[u]), bi, w1[c]);
+              }
+            }
+          if (h == 0) load(16);
+        }
+#pragma unroll
+        for (int c = 0; c < RH; ++c)
+          if (c < nc) {
+            xc[(size_t)c * a.ldx + (size_t)j * n + lane] = w0[c];
+            xc[(size_t)c * a.ldx + (size_t)jp * n + lane] = w1[c];
+#pragma unroll
+            for (int r = 0; r < NRM; ++r) {
+              if (r < nr) {
+                const double sr = warp_sum(double(cp[r]) * b[c]);
+                if (lane == 0) a.XB[(size_t)j * nr * nrhs + (size_t)(col0 + c) * nr + r] = sr;
+              }
+            }
+          }
       }
     }
   });
@@ -3043,7 +3132,7 @@ __global__ void __launch_bounds__(256, 2) k_backward_rows32(SweepArgs<TF> a0, co
                                                             const BatchCta* cmap, const long* ecnt) {
   for_entries<BATCH>(ecnt, [&](long entry) {
     constexpr unsigned FULL = 0xffffffffu;
-    constexpr int n = 32, n2 = 64;
+    constexpr int n = 32, n2 = 64, RH = 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     SweepArgs<TF> ab;  // this CTA's system (batch only)
     long q0, q1, qs;
@@ -3053,36 +3142,73 @@ __global__ void __launch_bounds__(256, 2) k_backward_rows32(SweepArgs<TF> a0, co
     const int nx = d.nx, nb = d.nblock, nrhs = a.nrhs, k = a.k;
     const bool qrp = a.sel == SEL_QRP;
     const size_t xb_off = (size_t)(nb + 1) * n + d.qx;
-    constexpr size_t nn = (size_t)n * n;
     for (long q = q0; q < q1; q += qs) {
       const int j = k + (int)(2L * k * q), jp = j - k, jpp = min(j + k, nb);
-      const TF* Dj = a.D + (size_t)j * nn;
-      const TF* Ej = a.E + (size_t)j * nn;
+      const TF* Dj = a.D + (size_t)j * n * n;
+      const TF* Ej = a.E + (size_t)j * n * n;
       const TF* Bj = a.B + (size_t)j * n * nx;
       const TF* Tj = a.Tm + (size_t)j * szT(d);
-      const double rdi = 1.0 / double(Tj[(size_t)lane * n2 + lane]);
       const int dst = qrp ? (int)a.P[(size_t)j * szP(d) + n2 + lane] : lane;
-      for (int col = 0; col < nrhs; ++col) {
-        double* xc = a.x + (size_t)col * a.ldx;
-        const double xjp = xc[(size_t)jp * n + lane], xjpp = xc[(size_t)jpp * n + lane];
-        const double xj = xc[(size_t)j * n + lane];
-        double s0 = 0.0, s1 = 0.0;
-  #pragma unroll
-        for (int c = 0; c < n; ++c) {
-          s0 = fma(double(Dj[(size_t)c * n + lane]), __shfl_sync(FULL, xjp, c), s0);
-          s1 = fma(double(Ej[(size_t)c * n + lane]), __shfl_sync(FULL, xjpp, c), s1);
+      for (int col0 = 0; col0 < nrhs; col0 += RH) {
+        const int nc = min(RH, nrhs - col0);
+        double* xc = a.x + (size_t)col0 * a.ldx;
+        TF m[32];
+        auto load = [&](const TF* M, int ld, int from) {  // columns from `from` on
+#pragma unroll
+          for (int c = 0; c < 32; ++c) m[c] = ld_batch(c >= from, M + (size_t)c * ld + lane);
+        };
+        load(Dj, n, 0);
+        TF bb[NXM];
+#pragma unroll
+        for (int c = 0; c < NXM; ++c) bb[c] = ld_batch(c < nx, Bj + (size_t)c * n + lane);
+        double xa[RH], xz[RH], y[RH];
+#pragma unroll
+        for (int c = 0; c < RH; ++c) {
+          xa[c] = ld_batch(c < nc, xc + (size_t)c * a.ldx + (size_t)jp * n + lane);
+          xz[c] = ld_batch(c < nc, xc + (size_t)c * a.ldx + (size_t)jpp * n + lane);
+          y[c] = ld_batch(c < nc, xc + (size_t)c * a.ldx + (size_t)j * n + lane);
         }
-  #pragma unroll
-        for (int c = 0; c < NXM; ++c)
-          if (c < nx) s0 = fma(double(Bj[(size_t)c * n + lane]), xc[xb_off + c], s0);
-        double y = xj - (s0 + s1);
-  #pragma unroll
-        for (int ii = n - 1; ii >= 0; --ii) {
-          const double xi = __shfl_sync(FULL, y * rdi, ii);
-          if (lane == ii) y = xi;
-          else if (lane < ii) y = fma(-double(Tj[(size_t)ii * n2 + lane]), xi, y);
-        }
-        xc[(size_t)j * n + dst] = y;
+        auto subtract = [&](const double (&x)[RH]) {  // y -= M x
+#pragma unroll
+          for (int c = 0; c < RH; ++c)
+            if (c < nc) {
+              double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+              for (int u = 0; u < 32; u += 2) {
+                s0 = fma(double(m[u]), __shfl_sync(FULL, x[c], u), s0);
+                s1 = fma(double(m[u + 1]), __shfl_sync(FULL, x[c], u + 1), s1);
+              }
+              y[c] -= s0 + s1;
+            }
+        };
+        subtract(xa);
+        load(Ej, n, 0);
+#pragma unroll
+        for (int c = 0; c < RH; ++c)
+          if (c < nc) {
+            double s = 0.0;
+#pragma unroll
+            for (int e = 0; e < NXM; ++e) s = fma(double(bb[e]), e < nx ? xc[(size_t)c * a.ldx + xb_off + e] : 0.0, s);
+            y[c] -= s;
+          }
+        subtract(xz);
+        load(Tj, n2, lane);  // U, on and right of the diagonal
+        double ud = 1.0;
+#pragma unroll
+        for (int c = 0; c < 32; ++c)
+          if (c == lane) ud = double(m[c]);
+        const double rdi = 1.0 / ud;
+#pragma unroll
+        for (int c = 0; c < RH; ++c)
+          if (c < nc) {
+            double v = y[c];
+#pragma unroll
+            for (int u = 31; u >= 0; --u) {
+              const double xi = __shfl_sync(FULL, v * rdi, u);
+              v = lane == u ? xi : fma(-double(m[u]), lane < u ? xi : 0.0, v);
+            }
+            xc[(size_t)c * a.ldx + (size_t)j * n + dst] = v;
+          }
       }
     }
   });
@@ -4112,17 +4238,18 @@ static FactorPlan<T> plan_factor(const DevState& s) {
       p.tc_cols = 2 * n + 8;
     }
   }
+  // orders between 16 and 32 run as the leading part of a block of order 32
   const bool grp_ok = s.sel == SEL_LU && d.nr <= 8 && d.nx <= 8 &&
-                      (n == 32 || (n == 16 && (sizeof(T) == 4 || s.pair_kernel == PAIR_GRP)));
+                      ((n > 16 && n <= 32) || (n == 16 && (sizeof(T) == 4 || s.pair_kernel == PAIR_GRP)));
   if (!p.tc && grp_ok && (s.pair_kernel == PAIR_AUTO || s.pair_kernel == PAIR_GRP)) {
-    if (n == 32) {
-      p.grp = k_factor_lu_grp<T, 32>;
+    if (n > 16) {
+      p.grp = n == 32 ? k_factor_lu_grp<T, 32> : k_factor_lu_grp<T, 32, false, true>;
       p.grp_smem = GrpShape<T, 32>::BYTES;
     } else {
       p.grp = k_factor_lu_grp<T, 16>;
       p.grp_smem = GrpShape<T, 16>::BYTES;
     }
-    p.grp_threads = 2 * n + 32;
+    p.grp_threads = (n > 16 ? 64 : 32) + 32;
     smem_limit_once(p.grp, p.grp_smem);
     p.grp_ctas = 148 * resident_ctas(p.grp, p.grp_threads, p.grp_smem);
   }
@@ -4408,12 +4535,23 @@ static SweepPlan<T> plan_sweeps(const DevState& s) {
   }
   // the form of the factors follows the kernel that made them
   const FactorPlan<T> fp = plan_factor<T>(s);
-  if (fp.tc) p.op = n;
+  if (fp.tc || fp.grp) p.op = n;
+  if (n == 32 && s.sel == SEL_LU && !fp.grp) {  // L and M
+    p.fwd = nullptr;
+    p.fwd_big = k_forward_lm<64, T>;
+    p.fwd_big_nt = 64;
+    p.fwd_big_smem = 64 * 8;
+  }
+  if (n > 16 && n < 32 && fp.grp) {
+    p.fwd_big = k_forward_op<64, T>;
+    p.fwd_big_nt = 128;
+    p.fwd_big_smem = (size_t)(3 * 64 + 64) * 8;
+  }
   if constexpr (sizeof(T) == 8) {
     if (fp.lub.threads) {
       const int rw = n <= 64 ? 128 : 256;
       p.op = fp.lub.bw;
-      p.fwd_big = n <= 64 ? k_forward_op<128> : k_forward_op<256>;
+      p.fwd_big = n <= 64 ? k_forward_op<128, T> : k_forward_op<256, T>;
       p.fwd_big_nt = 2 * rw;
       p.fwd_big_smem = (size_t)(3 * rw + 64) * 8;
       smem_limit_once(p.fwd_big, p.fwd_big_smem * SWB_RHS);
@@ -5613,7 +5751,7 @@ static void batch_sweeps_rows(BatchClass& c, cudaStream_t st, bool forward, int 
   const bool r4 = c.nrm <= 4, x4 = c.nxm <= 4;
   SweepArgs<T> a0{};
   a0.k = 1 << L;
-  a0.op = c.fam == PAIR_TC ? c.n : 0;
+  a0.op = c.fam == PAIR_TC || c.fam == PAIR_GRP ? c.n : 0;
   if constexpr (N == 8 || N == 16) {
     if (c.n == N) {  // pipelined: a fixed grid walks the level's map entries
       const long nent = c.scnt[L];

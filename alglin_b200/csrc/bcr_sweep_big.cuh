@@ -78,10 +78,10 @@ __device__ __forceinline__ void fwd_border(const SweepArgs<T>& a, int j, int col
 }
 
 // Forward sweep with factors in operator form by blocks of op <= 64 columns
-// (k_factor_lu_lub): two threads per row, each with 32 of the block's columns.
+// (k_factor_lu_lub; padded k_factor_lu_grp): two threads per row, each with 32 of the block's columns.
 // RW: rows, at least 2n.
-template <int RW>
-__global__ void __launch_bounds__(2 * RW, 256 / RW) k_forward_op(SweepArgs<double> a) {
+template <int RW, typename T>
+__global__ void __launch_bounds__(2 * RW, RW == 64 ? 4 : 256 / RW) k_forward_op(SweepArgs<T> a) {
   constexpr int NT = 2 * RW;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double(*y)[RW] = reinterpret_cast<double(*)[RW]>(smem_raw);
@@ -94,10 +94,10 @@ __global__ void __launch_bounds__(2 * RW, 256 / RW) k_forward_op(SweepArgs<doubl
   const long np = pairs_at_level(d.nblock, k);
   for (long q = blockIdx.x; q < np; q += gridDim.x) {
     const int j = k + (int)(2L * k * q), jp = j - k;
-    const double* Tj = a.Tm + (size_t)j * szT(d);
+    const T* Tj = a.Tm + (size_t)j * szT(d);
     for (int col0 = 0; col0 < a.nrhs; col0 += SWB_RHS) {
       const int nc = min(SWB_RHS, a.nrhs - col0);
-      double m[32];
+      T m[32];
       auto load = [&](int kb) {  // strictly left of the diagonal
         const int lim = min(min(bw, n - kb), r - kb);
 #pragma unroll

@@ -160,3 +160,31 @@ def test_padded_warp_lu(n, nr, nx, nblock):
         x = rhs.copy()
         assert h.factorize_solve(1, x.reshape(-1), x.shape[1]), h.last_error()
         assert fwd_err(x[0, :s.ncols], o.solve(rhs)[0, :s.ncols]) < 1e-9
+
+
+@pytest.mark.parametrize("n", [17, 24, 31, 32])
+@pytest.mark.parametrize("nr,nx", [(0, 0), (1, 8), (8, 2)])
+@pytest.mark.parametrize("nblock", [2, 29])
+def test_padded_cta_lu(n, nr, nx, nblock):
+    """Orders between 16 and 32 as leading parts of the CTA kernel's blocks.
+    cond(A) <= 2e5 (dense SVD), 2e5 * 2^-53 * 64 rows."""
+    s = synth.collocation(nblock, n, max(0, nx - nr), max(0, nr - nx), nr, nx, seed=n)
+    check(s, synth.rhs(s, 5, seed=n + 1), bar=1e-9)
+
+
+@pytest.mark.parametrize("n", [12, 20, 32])
+def test_zero_pivot_in_the_warp_and_cta_kernels(n):
+    """A zero column in both row blocks of a pair: getrf's INFO, and the handle's
+    next matrix is factored correctly."""
+    s = synth.collocation(6, n, 0, 0, 2, 2, seed=3)
+    bad = s.copy()
+    bad.E[2, 5] = 0.0
+    bad.D[3, 5] = 0.0
+    h = B.BorderedCR()
+    h.load_system(bad)
+    h.select("LU")
+    assert not h.factorize()
+    assert "INFO = 6" in h.last_error()
+    h.load_system(s)
+    assert h.factorize(), h.last_error()
+    check(s, synth.rhs(s, 1, seed=4))
