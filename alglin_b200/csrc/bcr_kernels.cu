@@ -798,7 +798,7 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
   const bool blive = br < nr;
   T rowA[N], cb[CPL];
   double cs1[2] = {0.0, 0.0}, cs2[2] = {0.0, 0.0};  // children's F / xb sums (tree)
-  {
+  auto load_panel = [&]() {
     const size_t po = top ? (size_t)jp * nn : (size_t)j * nn;
     const SrcT* Pm = (top ? srcE : srcD) + po;
     const double* Po = (top ? a.E0 : a.D0) + po;
@@ -825,6 +825,9 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
 #pragma unroll
         for (int q = 0; q < CPL; ++q) cb[q] += v[e][q];
     }
+  };
+  load_panel();
+  {
     // the children's F / xb partial sums of the two border-tile elements this
     // lane holds in the product (row 2N + g, columns 2N + 2t + {0, 1})
     if ((tr.c1 | tr.c2) && g < nr) {
@@ -878,73 +881,88 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
   // same multiplier updates the X of the earlier columns with the pivot row's
   // X, so one run of N - 1 fused multiply-adds per step yields U, L^-1 (the
   // pivot rows' X, strictly lower), -M L^-1 and -C' L^-1 (see the comment above).
+  // The registers rotate: rowA[0] is column i, a step moves every column one
+  // register down and puts X_r[i] at the end, so that the steps are one rolled
+  // loop that stays in the instruction cache (column c is at (c - i) mod N).
+  // The pivot is found by reductions: the largest |a| (upper, then lower word),
+  // then the smallest (position, lane).  Reciprocals of zero, tiny or huge pivots
+  // need the correctly rounded routine, whose branch would wait for the search at
+  // each step: such a pivot is only noted, and the panel run again with it.
   const int pos0 = act ? (top ? ri : n + ri) : 63;
   int mypos = pos0, info = 0;
-  bool done = !act;
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    if (PAD && i >= n) break;
-    // pivot: max |a| over the rows not yet used, ties to the smaller position;
-    // every lane forms the reciprocal of its own candidate meanwhile
-    unsigned hi, lo, hmax, m;
-    T rc;
-    tc_candidate(rowA[i], done, hi, lo, rc);
-    hmax = __reduce_max_sync(FULL, hi);
-    if constexpr (sizeof(T) == 8) {
-      lo = hi == hmax ? lo : 0u;
-      const unsigned lmax = __reduce_max_sync(FULL, lo);
-      m = __ballot_sync(FULL, hi == hmax && lo == lmax);
-    } else {
-      m = __ballot_sync(FULL, hi == hmax);
-    }
-    if (__popc(m) != 1 || !tc_plain_pivot<T>(hmax)) {  // exact tie, or zero, tiny, huge or no number
-      const unsigned pm = __reduce_min_sync(FULL, (m >> lane) & 1u ? (unsigned)mypos : 0xffffffffu);
-      m = __ballot_sync(FULL, ((m >> lane) & 1u) && (unsigned)mypos == pm);
-      rc = rcp_rn(rowA[i]);
-      const T pv = __shfl_sync(FULL, rowA[i], __ffs(m) - 1);
-      if (pv == T(0)) {
-        if (info == 0) info = i + 1;
-        rc = T(0);
+  bool done = !act, bad = false;
+  for (int attempt = 0;; ++attempt) {
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+      const T v0 = rowA[0];
+      unsigned hi, lo;
+      T rc;
+      tc_candidate(v0, done, hi, lo, rc);
+      const unsigned hmax = __reduce_max_sync(FULL, hi);
+      bool in = hi == hmax;
+      if constexpr (sizeof(T) == 8) {
+        const unsigned lmax = __reduce_max_sync(FULL, in ? lo : 0u);
+        in = in && lo == lmax;
       }
-    }
-    const int p = __ffs(m) - 1;
-    const int pmin = __shfl_sync(FULL, mypos, p);
-    const bool isp = lane == p;
-    mypos = isp ? i : (mypos == i ? pmin : mypos);
-    T* prow = Gs + i * S::LDG;  // the pivot row [X | U], then its reciprocal
-    if (isp) {
-      prow[N] = rc;
+      const unsigned best = __reduce_min_sync(FULL, in ? ((unsigned)mypos << 5) | lane : 0xffffffffu);
+      const int p = (int)(best & 31u), pmin = (int)(best >> 5);
+      bad = bad || !tc_plain_pivot<T>(hmax);
+      if (attempt) {
+        if (!tc_plain_pivot<T>(hmax)) rc = v0 != T(0) ? rcp_rn(v0) : T(0);
+        if (info == 0 && __shfl_sync(FULL, v0, p) == T(0)) info = i + 1;
+      }
+      const bool isp = lane == p;
+      mypos = isp ? i : (mypos == i ? pmin : mypos);
+      T* prow = Gs + i * S::LDG;  // the reciprocal, then the pivot row from column i + 1 on
+      if (isp) {
+        store2(&prow[0], rc, rowA[1]);
 #pragma unroll
-      for (int c = 0; c < N; c += 2) store2(&prow[c], rowA[c], rowA[c + 1]);
-    }
-    __syncwarp();
-    done = done || isp;
-    const T rinv = prow[N];
-    const T l = done ? T(0) : rowA[i] * rinv;
-    // the next column first: its search is what the next step waits for
-    if (i + 1 < N) rowA[i + 1] = fma(-l, prow[i + 1], rowA[i + 1]);
-#pragma unroll
-    for (int c = 0; c < N; c += 2) {
+        for (int c = 2; c < N; c += 2) store2(&prow[c], rowA[c], rowA[c + 1]);
+      }
+      __syncwarp();
+      done = done || isp;
       T u0, u1;
-      load2(&prow[c], u0, u1);
-      if (c != i && c != i + 1) rowA[c] = fma(-l, u0, rowA[c]);
-      if (c + 1 != i && c + 1 != i + 1) rowA[c + 1] = fma(-l, u1, rowA[c + 1]);
-    }
-    if (!done) rowA[i] = -l;
-    {  // border rows: multiplier from the lane holding column i of the row
-      const T ci = __shfl_sync(FULL, cb[i % CPL], (lane & ~(LPR - 1)) | (i / CPL));
-      const T lb = ci * rinv;
+      load2(&prow[0], u0, u1);
+      const T rinv = u0;
+      const T l = done ? T(0) : v0 * rinv;
+      rowA[0] = fma(-l, u1, rowA[1]);
 #pragma unroll
-      for (int q = 0; q < CPL; ++q) {
-        const T v = fma(-lb, prow[bc0 + q], cb[q]);
-        cb[q] = (q == i % CPL && bc0 + q == i) ? -lb : v;
+      for (int c = 2; c < N; c += 2) {
+        load2(&prow[c], u0, u1);
+        rowA[c - 1] = fma(-l, u0, rowA[c]);
+        rowA[c] = fma(-l, u1, rowA[c + 1]);
+      }
+      rowA[N - 1] = done ? v0 : -l;
+      {  // border rows: multiplier from the lane holding column i of the row
+        T ci = cb[0];
+#pragma unroll
+        for (int q = 1; q < CPL; ++q) ci = (i & (CPL - 1)) == q ? cb[q] : ci;
+        const T lb = __shfl_sync(FULL, ci, (lane & ~(LPR - 1)) | (i / CPL)) * rinv;
+#pragma unroll
+        for (int q = 0; q < CPL; ++q) {
+          const int at = (bc0 + q - i) & (N - 1);
+          cb[q] = at == 0 ? -lb : fma(-lb, prow[at], cb[q]);
+        }
       }
     }
+    if (!bad || attempt) break;
+    load_panel();
+    mypos = pos0;
+    done = !act;
   }
   if (info != 0) {
     if (lane == 0) report(a.st, DEV_ZERO_PIVOT, j, info, k);
     __syncwarp();
     return false;
+  }
+  if (PAD) {  // the rest of the rotation
+#pragma unroll 1
+    for (int i = n; i < N; ++i) {
+      const T v0 = rowA[0];
+#pragma unroll
+      for (int c = 1; c < N; ++c) rowA[c - 1] = rowA[c];
+      rowA[N - 1] = v0;
+    }
   }
   // panel factors T_j in getrf row order (operator form: [L^-1 \ U; -M L^-1],
   // the unit diagonal of L^-1 not stored), pivots, the border operator
@@ -1011,11 +1029,10 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
 #pragma unroll
         for (int mt = 0; mt < S::MTILES; ++mt) {
           if (mt * 8 < N && ks * 4 >= mt * 8 + 8) continue;  // above the diagonal of L^-1
-          double afr = Gs[(mt * 8 + g) * S::LDG + ks * 4 + t];
-          if (mt * 8 < N && ks * 4 + 3 >= mt * 8) {
-            const int dk = ks * 4 + t - (mt * 8 + g);
-            afr = dk < 0 ? afr : dk == 0 ? 1.0 : 0.0;
-          }
+          // (row r of L^-1 is stored from column r on, see phase 1)
+          const int dk = ks * 4 + t - (mt * 8 + g);
+          double afr = Gs[(mt * 8 + g) * S::LDG + (mt * 8 < N ? dk & (N - 1) : ks * 4 + t)];
+          if (mt * 8 < N && ks * 4 + 3 >= mt * 8) afr = dk < 0 ? afr : dk == 0 ? 1.0 : 0.0;
 #pragma unroll
           for (int ni = 0; ni < PC; ++ni)
             if (pass * PC + ni < S::NTILES) dmma_8x8x4(acc[mt][ni][0], acc[mt][ni][1], afr, bfr[ni]);
@@ -1035,11 +1052,9 @@ __device__ __forceinline__ bool tc_pair(const FactorArgs<T>& a, int j, int k, bo
         }
 #pragma unroll
         for (int mt = 0; mt < S::MTILES; ++mt) {
-          T av = Gs[(mt * 8 + g) * S::LDG + kk];
-          if (mt * 8 < N) {
-            const int dk = kk - (mt * 8 + g);
-            av = dk < 0 ? av : dk == 0 ? T(1) : T(0);
-          }
+          const int dk = kk - (mt * 8 + g);
+          T av = Gs[(mt * 8 + g) * S::LDG + (mt * 8 < N ? dk & (N - 1) : kk)];
+          if (mt * 8 < N) av = dk < 0 ? av : dk == 0 ? T(1) : T(0);
 #pragma unroll
           for (int ni = 0; ni < PC; ++ni) {
             acc[mt][ni][0] = fma(av, bv[ni][0], acc[mt][ni][0]);
@@ -1608,6 +1623,13 @@ __device__ __forceinline__ void grp_body(const FactorArgs<T>& a, long q0, long q
     if (PAD && t < 2 * N) rowof[t] = 0;  // rows of the product that no panel row fills
     // ------------------------------------------------------------ load
     T row[N];
+    auto load_rows = [&](const auto* D, const auto* E, const auto* C) {
+      const auto* P = panel ? (top ? E + (size_t)jp * nn : D + (size_t)j * nn) + ri
+                            : C + (size_t)j * nrn + (t - 2 * N);
+      const int st = panel ? n : nr;
+#pragma unroll
+      for (int c = 0; c < N; ++c) row[c] = T(ld_batch_c<COH>((act || brow) && (!PAD || c < n), P + (size_t)c * st));
+    };
     auto load = [&](const auto* D, const auto* E, const auto* Bm, const auto* C) {
       // trailing columns, compact: TOP rows [D_jp B_jp], BOTTOM rows [E_j B_j]; one
       // element of both per thread and round
@@ -1631,13 +1653,7 @@ __device__ __forceinline__ void grp_body(const FactorArgs<T>& a, long q0, long q
         }
         cp_async_commit();
       }
-      {
-        const auto* P = panel ? (top ? E + (size_t)jp * nn : D + (size_t)j * nn) + ri
-                              : C + (size_t)j * nrn + (t - 2 * N);
-        const int st = panel ? n : nr;
-#pragma unroll
-        for (int c = 0; c < N; ++c) row[c] = T(ld_batch_c<COH>((act || brow) && (!PAD || c < n), P + (size_t)c * st));
-      }
+      load_rows(D, E, C);
       if constexpr (!ASYNC) {
         constexpr int H = 4;  // rounds in flight
         for (int i0 = 0; i0 < IT; i0 += H) {
@@ -1679,8 +1695,11 @@ __device__ __forceinline__ void grp_body(const FactorArgs<T>& a, long q0, long q
     if (first) load(a.D0, a.E0, a.B0, a.C0);
     else load(a.D, a.E, a.B, a.C);
     // ------------------- phase 1: panel LU with the operator rows in place
+    // (zero, tiny and huge pivots are only noted, and the panel run again with
+    // their reciprocals: see tc_pair)
     int mypos = pos0;
-    bool done = !act, used = false;  // border and idle lanes never pivot
+    bool done = !act, used = false, bad = false;  // border and idle lanes never pivot
+    for (int attempt = 0;; ++attempt) {
 #pragma unroll 1
     for (int i = 0; i < n; ++i) {
       // row[0] is column i
@@ -1698,7 +1717,7 @@ __device__ __forceinline__ void grp_body(const FactorArgs<T>& a, long q0, long q
           in = in && lo == lmax;
         }
         const unsigned best = __reduce_min_sync(FULL, in ? ((unsigned)mypos << 5) | lane : 0xffffffffu);
-        if (hmax != 0u && !tc_plain_pivot<T>(hmax)) rc = v0 != T(0) ? rcp_rn(v0) : T(0);
+        if (attempt && hmax != 0u && !tc_plain_pivot<T>(hmax)) rc = v0 != T(0) ? rcp_rn(v0) : T(0);
         // where no candidate is left (hmax = 0, best all ones) lane 31 posts zeros
         if ((best & 31u) == (unsigned)lane) {
           reinterpret_cast<int4*>(hdr)[par * S::NWP + w] =
@@ -1721,13 +1740,14 @@ __device__ __forceinline__ void grp_body(const FactorArgs<T>& a, long q0, long q
           hw = h1;
         }
       }
+      bad = bad || !tc_plain_pivot<T>((unsigned)hw.x);
       const int p = hw.z & 255, pmin = (hw.z >> 8) & 255;
       const T* u = slot + (par * S::NWP + wb) * S::LDS;
       mypos = mypos == i ? pmin : mypos;
       if (t == p) {
         mypos = i;
         done = used = true;
-        if (v0 == T(0) && s_info == 0) s_info = i + 1;
+        if (attempt && v0 == T(0) && s_info == 0) s_info = i + 1;
       }
       T u0, u1;
       load2(u, u0, u1);
@@ -1740,6 +1760,14 @@ __device__ __forceinline__ void grp_body(const FactorArgs<T>& a, long q0, long q
         row[c] = fma(-l, u1, row[c + 1]);
       }
       row[N - 1] = used ? v0 : -l;
+    }
+      if (!bad || attempt) break;
+      if (first) load_rows(a.D0, a.E0, a.C0);
+      else load_rows(a.D, a.E, a.C);
+      mypos = pos0;
+      done = !act;
+      used = false;
+      __syncthreads();  // the last step's readers of the slots are done
     }
     if (PAD) {  // the rest of the rotation
 #pragma unroll 1

@@ -152,14 +152,20 @@ __device__ void lub_panel(LubShared<NT>& sh, double* Pb, int ld, double* Xb, dou
     if (warp < nwa) {
       const bool before = used;  // a pivot of an earlier sub-block
       int own = SB;
+      const int pos_in = mypos;
+      const bool done_in = done;
       double v[SB];
-#pragma unroll
-      for (int c = 0; c < SB; ++c) v[c] = Pb[(size_t)min(c0 + c, w - 1) * ld + tid];
       const int steps = min(SB, w - c0);
       const unsigned hdr0 = (unsigned)__cvta_generic_to_shared(&sh.hdr[0][warp]);
       const unsigned val0 = (unsigned)__cvta_generic_to_shared(&sh.val[0][warp][0]);
       constexpr unsigned HS = sizeof(sh.hdr[0]), VS = sizeof(sh.val[0]);
       const int hl = lane < nwa ? lane : 0;
+      // zero, tiny and huge pivots are only noted, and the sub-block run again with
+      // their correctly rounded reciprocals (see tc_pair)
+      for (int attempt = 0;; ++attempt) {
+        bool bad = false;
+#pragma unroll
+        for (int c = 0; c < SB; ++c) v[c] = Pb[(size_t)min(c0 + c, w - 1) * ld + tid];
 #pragma unroll 1
       for (int i = 0; i < steps; ++i) {
         // v[0] is column i; a step moves every column one register down and the
@@ -175,7 +181,7 @@ __device__ void lub_panel(LubShared<NT>& sh, double* Pb, int ld, double* Xb, dou
         const unsigned lmax = __reduce_max_sync(FULL, lo);
         const bool in = hi == hmax && lo == lmax && !done;
         const unsigned best = __reduce_min_sync(FULL, in ? ((unsigned)mypos << 5) | lane : 0xffffffffu);
-        if (hmax != 0u && !tc_plain_pivot<double>(hmax)) rc = v0 != 0.0 ? __drcp_rn(v0) : 0.0;
+        if (attempt && hmax != 0u && !tc_plain_pivot<double>(hmax)) rc = v0 != 0.0 ? __drcp_rn(v0) : 0.0;
         // the warp's candidate; where none is left (hmax = 0, best all ones) lane 31
         // posts zeros
         sts_candidate((best & 31u) == (unsigned)lane, hdr0 + par * HS, hmax, lmax, (best >> 5 << 9) | tid,
@@ -186,6 +192,7 @@ __device__ void lub_panel(LubShared<NT>& sh, double* Pb, int ld, double* Xb, dou
         const unsigned bl = __reduce_max_sync(FULL, (unsigned)h.x == bh ? (unsigned)h.y : 0u);
         const unsigned pt =
             __reduce_min_sync(FULL, (unsigned)h.x == bh && (unsigned)h.y == bl ? (unsigned)h.z : 0xffffffffu);
+        bad = bad || !tc_plain_pivot<double>(bh);
         const int p = (int)(pt & 511u), pmin = (int)(pt >> 9);
         const double* sv = sh.val[par][p >> 5];
         double u[SB];
@@ -193,7 +200,7 @@ __device__ void lub_panel(LubShared<NT>& sh, double* Pb, int ld, double* Xb, dou
         for (int c = 0; c < SB; c += 2) load2(&sv[c], u[c], u[c + 1]);
         mypos = mypos == gi ? pmin : mypos;
         if (tid == p) {
-          if (v0 == 0.0 && sh.info == 0) sh.info = gi + 1;
+          if (attempt && v0 == 0.0 && sh.info == 0) sh.info = gi + 1;
           mypos = gi;
           done = used = true;
           own = i;
@@ -204,6 +211,13 @@ __device__ void lub_panel(LubShared<NT>& sh, double* Pb, int ld, double* Xb, dou
 #pragma unroll
         for (int c = 1; c < SB; ++c) v[c - 1] = fma(-l, u[c], v[c]);
         v[SB - 1] = used ? v0 : -l;
+      }
+        if (!bad || attempt) break;
+        mypos = pos_in;
+        done = done_in;
+        used = before;
+        own = SB;
+        lub_bar(nwa * 32);  // the last step's readers of the candidates are done
       }
 #pragma unroll 1
       for (int i = steps; i < SB; ++i) {  // a partial sub-block: the rest of the rotation
