@@ -2714,7 +2714,8 @@ __device__ __forceinline__ void bwd_stage(const SweepArgs<T>& a, int k, long q, 
   using Bf = BwdBuf<N, NXM, T>;
   constexpr int V = 16 / (int)sizeof(T);
   const Dims d = a.d;
-  const int n = d.n, nx = d.nx;
+  constexpr int n = N;
+  const int nx = d.nx;
   const int j = k + (int)(2L * k * q);
   const T* Dj = a.D + (size_t)j * n * n;
   const T* Ej = a.E + (size_t)j * n * n;
@@ -2779,6 +2780,103 @@ struct PipeItems {
   }
 };
 
+// Eight right-hand sides of one pair of the backward sweep (FP64): the products
+// D' X_jp, E' X_jpp and B' X_b on the tensor cores, then the triangle with four
+// columns per half warp.  buf: the pair's staged factors (overwritten).
+//
+// One column at a time, 50 shuffles and as many multiply-adds repeat for every
+// column, and the triangle's chain of N shuffles is walked once per column: 8
+// right-hand sides of 30,000 blocks of order 16 took 128 us at level 1, and take
+// 47 us here; the factor's 16.6 MB pass is 3 us of that.  Taken from two
+// right-hand sides on, where it already is the faster one (the whole solve of
+// that size: 389 to 318 us for 2, 487 to 323 us for 3, 780 to 490 us with the
+// factorization for 8); a single one stays with the scalar code, which does an
+// eighth of the work.
+template <int N, int NXM>
+__device__ __forceinline__ void bwd_multi(const SweepArgs<double>& a, int j, int jp, int jpp, double* buf, int lane) {
+  using Bf = BwdBuf<N, NXM, double>;
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int MT = N / 8, KS = N / 4;
+  const Dims d = a.d;
+  const int nx = d.nx, nrhs = a.nrhs, g = lane >> 2, q = lane & 3, i = lane & 15, hb = lane >> 4;
+  const size_t xb_off = (size_t)(d.nblock + 1) * N + d.qx;
+  const bool rowok = i < N;
+  double u[N];
+#pragma unroll
+  for (int c = 0; c < N; ++c) u[c] = rowok ? buf[2 * Bf::DE + Bf::BB + c * N + i] : 0.0;
+  double ud = 1.0;
+#pragma unroll
+  for (int c = 0; c < N; ++c)
+    if (c == i) ud = u[c];
+  const double rdi = rowok ? 1.0 / ud : 0.0;
+  const int dst = a.sel == SEL_QRP && rowok ? (int)a.P[(size_t)j * szP(d) + 2 * N + i] : i;
+  // -[D' E' B'] as A fragments, kept for all chunks of columns
+  double fd[MT][KS], fe[MT][KS], fb[MT][2];
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) {
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      fd[mt][ks] = -buf[(4 * ks + q) * N + 8 * mt + g];
+      fe[mt][ks] = -buf[Bf::DE + (4 * ks + q) * N + 8 * mt + g];
+    }
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks) {
+      const int c = 4 * ks + q;
+      fb[mt][ks] = c < nx ? -buf[2 * Bf::DE + (c < NXM ? c : 0) * N + 8 * mt + g] : 0.0;
+    }
+  }
+  for (int c0 = 0; c0 < nrhs; c0 += 8) {
+    const int nc = min(8, nrhs - c0);
+    double* xc = a.x + (size_t)c0 * a.ldx;
+    double bd[KS], be[KS], bb[2], acc[MT][2];
+    const double* xg = xc + (size_t)min(g, nc - 1) * a.ldx;
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      bd[ks] = ld_batch(g < nc, xg + (size_t)jp * N + 4 * ks + q);
+      be[ks] = ld_batch(g < nc, xg + (size_t)jpp * N + 4 * ks + q);
+    }
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks) bb[ks] = ld_batch(g < nc && 4 * ks + q < nx, xg + xb_off + 4 * ks + q);
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        acc[mt][h] = ld_batch(2 * q + h < nc, xc + (size_t)min(2 * q + h, nc - 1) * a.ldx + (size_t)j * N + 8 * mt + g);
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        dmma_8x8x4(acc[mt][0], acc[mt][1], fd[mt][ks], bd[ks]);
+        dmma_8x8x4(acc[mt][0], acc[mt][1], fe[mt][ks], be[ks]);
+      }
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) dmma_8x8x4(acc[mt][0], acc[mt][1], fb[mt][ks], bb[ks]);
+    // to lane = row through the buffer's first block
+    __syncwarp();
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) buf[(2 * q + h) * N + 8 * mt + g] = acc[mt][h];
+    __syncwarp();
+    double y[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y[e] = rowok ? buf[(4 * hb + e) * N + i] : 0.0;
+#pragma unroll
+    for (int ii = N - 1; ii >= 0; --ii) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const double xi = __shfl_sync(FULL, y[e] * rdi, (lane & 16) | ii);
+        y[e] = i == ii ? xi : i < ii ? fma(-u[ii], xi, y[e]) : y[e];
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (rowok && 4 * hb + e < nc) xc[(size_t)(4 * hb + e) * a.ldx + (size_t)j * N + dst] = y[e];
+  }
+}
+
 template <int N, int NXM, typename T = double, bool BATCH = false>
 __global__ void __launch_bounds__(256, 2) k_backward_pipe(SweepArgs<T> a0, const SweepArgs<T>* tab,
                                                           const BatchCta* map, const long* ecnt, long nent) {
@@ -2806,7 +2904,8 @@ __global__ void __launch_bounds__(256, 2) k_backward_pipe(SweepArgs<T> a0, const
     if (have) {
       const SweepArgs<T>& a = items.args(sys);
       const Dims d = a.d;
-      const int n = d.n, nx = d.nx, nb = d.nblock, nrhs = a.nrhs;
+      constexpr int n = N;
+      const int nx = d.nx, nb = d.nblock, nrhs = a.nrhs;
       const bool hi = lane >= 16, rowok = i < n;
       const bool qrp = a.sel == SEL_QRP;
       const size_t xb_off = (size_t)(nb + 1) * n + d.qx;
@@ -2820,47 +2919,53 @@ __global__ void __launch_bounds__(256, 2) k_backward_pipe(SweepArgs<T> a0, const
       const int dst = (qrp && !hi && rowok) ? (int)a.P[(size_t)j * szP(d) + 2 * n + i] : i;
       cp_async_wait<1>();  // this pair's factors (the next pair's may still be in flight)
       __syncwarp();
-      const T* buf = bufs + cur * Bf::WORDS;
-      double m[N], u[N], bb[NXM];
+      T* buf = bufs + cur * Bf::WORDS;
+      const bool multi = sizeof(T) == 8 && nrhs > 1;
+      if constexpr (sizeof(T) == 8) {
+        if (multi) bwd_multi<N, NXM>(a, j, jp, jpp, buf, lane);
+      }
+      if (!multi) {
+        double m[N], u[N], bb[NXM];
 #pragma unroll
-      for (int c = 0; c < N; ++c) m[c] = (rowok && c < n) ? buf[(hi ? Bf::DE : 0) + c * n + i] : 0.0;
+        for (int c = 0; c < N; ++c) m[c] = (rowok && c < n) ? buf[(hi ? Bf::DE : 0) + c * n + i] : 0.0;
 #pragma unroll
-      for (int c = 0; c < N; ++c) u[c] = (!hi && rowok && c < n) ? buf[2 * Bf::DE + Bf::BB + c * n + i] : 0.0;
+        for (int c = 0; c < N; ++c) u[c] = (!hi && rowok && c < n) ? buf[2 * Bf::DE + Bf::BB + c * n + i] : 0.0;
 #pragma unroll
-      for (int c = 0; c < NXM; ++c) bb[c] = (!hi && rowok && c < nx) ? buf[2 * Bf::DE + c * n + i] : 0.0;
-      double ud = 1.0;
+        for (int c = 0; c < NXM; ++c) bb[c] = (!hi && rowok && c < nx) ? buf[2 * Bf::DE + c * n + i] : 0.0;
+        double ud = 1.0;
 #pragma unroll
-      for (int c = 0; c < N; ++c)
-        if (c == i) ud = u[c];
-      const double rdi = (!hi && rowok) ? 1.0 / ud : 0.0;
-      for (int col = 0; col < nrhs; ++col) {
-        double* xc = a.x + (size_t)col * a.ldx;
-        const double xv = col == 0 ? xv0 : (rowok ? (hi ? xc[(size_t)jpp * n + i] : xc[(size_t)jp * n + i]) : 0.0);
-        const double xj = col == 0 ? xj0 : ((!hi && rowok) ? xc[(size_t)j * n + i] : 0.0);
-        double xbv[NXM];
+        for (int c = 0; c < N; ++c)
+          if (c == i) ud = u[c];
+        const double rdi = (!hi && rowok) ? 1.0 / ud : 0.0;
+        for (int col = 0; col < nrhs; ++col) {
+          double* xc = a.x + (size_t)col * a.ldx;
+          const double xv = col == 0 ? xv0 : (rowok ? (hi ? xc[(size_t)jpp * n + i] : xc[(size_t)jp * n + i]) : 0.0);
+          const double xj = col == 0 ? xj0 : ((!hi && rowok) ? xc[(size_t)j * n + i] : 0.0);
+          double xbv[NXM];
 #pragma unroll
-        for (int c = 0; c < NXM; ++c) xbv[c] = c < nx ? xc[xb_off + c] : 0.0;
-        double sacc = 0.0;
+          for (int c = 0; c < NXM; ++c) xbv[c] = c < nx ? xc[xb_off + c] : 0.0;
+          double sacc = 0.0;
 #pragma unroll
-        for (int c = 0; c < N; ++c) {
-          if (c < n) {
-            const double xcv = __shfl_sync(FULL, xv, (lane & 16) | c);
-            sacc = fma(m[c], xcv, sacc);
+          for (int c = 0; c < N; ++c) {
+            if (c < n) {
+              const double xcv = __shfl_sync(FULL, xv, (lane & 16) | c);
+              sacc = fma(m[c], xcv, sacc);
+            }
           }
-        }
-        sacc += __shfl_xor_sync(FULL, sacc, 16);
+          sacc += __shfl_xor_sync(FULL, sacc, 16);
 #pragma unroll
-        for (int c = 0; c < NXM; ++c) sacc = fma(bb[c], xbv[c], sacc);
-        double y = xj - sacc;
+          for (int c = 0; c < NXM; ++c) sacc = fma(bb[c], xbv[c], sacc);
+          double y = xj - sacc;
 #pragma unroll
-        for (int ii = N - 1; ii >= 0; --ii) {
-          if (ii < n) {
-            const double xi = __shfl_sync(FULL, y * rdi, ii);
-            if (i == ii) y = xi;
-            else if (i < ii) y = fma(-u[ii], xi, y);
+          for (int ii = N - 1; ii >= 0; --ii) {
+            if (ii < n) {
+              const double xi = __shfl_sync(FULL, y * rdi, ii);
+              if (i == ii) y = xi;
+              else if (i < ii) y = fma(-u[ii], xi, y);
+            }
           }
+          if (!hi && rowok) xc[(size_t)j * n + dst] = y;
         }
-        if (!hi && rowok) xc[(size_t)j * n + dst] = y;
       }
     }
     __syncwarp();  // every lane is done with this buffer before it is refilled
@@ -2964,12 +3069,73 @@ __device__ __forceinline__ void fwd_stage(const SweepArgs<T>& a, int k, long q, 
   using Bf = FwdBuf<N, NRM, T>;
   constexpr int V = 16 / (int)sizeof(T);
   const Dims d = a.d;
-  const int n = d.n, nr = d.nr;
+  constexpr int n = N;
+  const int nr = d.nr;
   const int j = k + (int)(2L * k * q);
   const T* Tj = a.Tm + (size_t)j * szT(d);
   const T* Cj = a.C + (size_t)j * nr * n;
   for (int c = lane; c < 2 * n * n / V; c += 32) cp_async16(buf + V * c, Tj + V * c);
   for (int c = lane; c < n * nr / V; c += 32) cp_async16(buf + Bf::TT + V * c, Cj + V * c);
+}
+
+// Eight right-hand sides of one pair of the forward sweep (FP64, operator form):
+// one product [L^-1; -M L^-1; -C' L^-1] X on the tensor cores (see bwd_multi).
+// src: the original row at position `lane`; buf: the pair's staged T_j and C_j.
+template <int N, int NRM>
+__device__ __forceinline__ void fwd_multi(const SweepArgs<double>& a, int j, int jp, int src, const double* buf,
+                                          int lane) {
+  using Bf = FwdBuf<N, NRM, double>;
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int MT = 2 * N / 8, KS = N / 4;
+  const Dims d = a.d;
+  const int nr = d.nr, nrhs = a.nrhs, g = lane >> 2, q = lane & 3;
+  double f[MT + 1][KS];
+#pragma unroll
+  for (int ks = 0; ks < KS; ++ks) {
+    const int c = 4 * ks + q;
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      const double v = buf[c * 2 * N + 8 * mt + g];
+      f[mt][ks] = 8 * mt + g > c ? v : 0.0;  // strictly below the diagonal; the rest of row k is U
+    }
+    f[MT][ks] = g < nr ? buf[Bf::TT + c * nr + (g < nr ? g : 0)] : 0.0;
+  }
+  // the vector element at this lane's rows
+  auto at = [&](int r, int c) { return a.x + (size_t)c * a.ldx + (r < N ? (size_t)jp * N + r : (size_t)j * N + r - N); };
+  int rk[KS], rm[MT];
+#pragma unroll
+  for (int ks = 0; ks < KS; ++ks) rk[ks] = __shfl_sync(FULL, src, 4 * ks + q);
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) rm[mt] = __shfl_sync(FULL, src, 8 * mt + g);
+  for (int c0 = 0; c0 < nrhs; c0 += 8) {
+    const int nc = min(8, nrhs - c0);
+    double b[KS], acc[MT + 1][2];
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) b[ks] = ld_batch(g < nc, at(rk[ks], c0 + min(g, nc - 1)));
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) acc[mt][h] = ld_batch(2 * q + h < nc, at(rm[mt], c0 + min(2 * q + h, nc - 1)));
+    acc[MT][0] = acc[MT][1] = 0.0;
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+      for (int mt = 0; mt <= MT; ++mt) dmma_8x8x4(acc[mt][0], acc[mt][1], f[mt][ks], b[ks]);
+    __syncwarp();  // every lane's reads are done
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (2 * q + h < nc) {
+        const int c = c0 + 2 * q + h;
+        double* xc = a.x + (size_t)c * a.ldx;
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          const int r = 8 * mt + g;
+          if (8 * mt < N) xc[(size_t)j * N + r] = acc[mt][h];
+          else xc[(size_t)jp * N + r - N] = acc[mt][h];
+        }
+        if (g < nr) a.XB[(size_t)j * nr * nrhs + (size_t)c * nr + g] = acc[MT][h];
+      }
+  }
 }
 
 template <int N, int NRM, typename T = double, bool BATCH = false>
@@ -3011,7 +3177,8 @@ __global__ void __launch_bounds__(256, 2) k_forward_pipe(SweepArgs<T> a0, const 
     if (have) {
       const SweepArgs<T>& a = items.args(sys);
       const Dims d = a.d;
-      const int n = d.n, nr = d.nr, n2 = 2 * n, nrhs = a.nrhs;
+      constexpr int n = N, n2 = 2 * N;
+      const int nr = d.nr, nrhs = a.nrhs;
       const bool act = lane < n2;
       const int j = k + (int)(2L * k * q), jp = j - k;
       // the first right-hand side's values, loaded while the factors arrive
@@ -3019,42 +3186,48 @@ __global__ void __launch_bounds__(256, 2) k_forward_pipe(SweepArgs<T> a0, const 
       cp_async_wait<1>();  // this pair's factors (the next pair's may still be in flight)
       __syncwarp();
       const T* buf = bufs + cur * Bf::WORDS;
-      double t[N], cp[NRM];
+      const bool multi = sizeof(T) == 8 && op && nrhs > 1;
+      if constexpr (sizeof(T) == 8) {
+        if (multi) fwd_multi<N, NRM>(a, j, jp, src, buf, lane);
+      }
+      if (!multi) {
+        double t[N], cp[NRM];
 #pragma unroll
-      for (int c = 0; c < N; ++c) t[c] = (act && (!op || lane > c)) ? double(buf[c * n2 + lane]) : 0.0;
+        for (int c = 0; c < N; ++c) t[c] = (act && (!op || lane > c)) ? double(buf[c * n2 + lane]) : 0.0;
 #pragma unroll
-      for (int r = 0; r < NRM; ++r) cp[r] = (lane < n && r < nr) ? double(buf[Bf::TT + lane * nr + r]) : 0.0;
-      for (int col = 0; col < nrhs; ++col) {
-        double* xc = a.x + (size_t)col * a.ldx;
-        const double orig =
-            col == 0 ? orig0 : (act ? (lane < n ? xc[(size_t)jp * n + lane] : xc[(size_t)j * n + lane - n]) : 0.0);
-        const double b = __shfl_sync(FULL, orig, src);
-        double w = b, w2 = 0.0;
-        if (op) {  // one product with the operator: no serial chain
+        for (int r = 0; r < NRM; ++r) cp[r] = (lane < n && r < nr) ? double(buf[Bf::TT + lane * nr + r]) : 0.0;
+        for (int col = 0; col < nrhs; ++col) {
+          double* xc = a.x + (size_t)col * a.ldx;
+          const double orig =
+              col == 0 ? orig0 : (act ? (lane < n ? xc[(size_t)jp * n + lane] : xc[(size_t)j * n + lane - n]) : 0.0);
+          const double b = __shfl_sync(FULL, orig, src);
+          double w = b, w2 = 0.0;
+          if (op) {  // one product with the operator: no serial chain
 #pragma unroll
-          for (int i = 0; i < N; i += 2) {
-            w = fma(t[i], __shfl_sync(FULL, b, i), w);
-            w2 = fma(t[i + 1], __shfl_sync(FULL, b, i + 1), w2);
+            for (int i = 0; i < N; i += 2) {
+              w = fma(t[i], __shfl_sync(FULL, b, i), w);
+              w2 = fma(t[i + 1], __shfl_sync(FULL, b, i + 1), w2);
+            }
+            w += w2;
+          } else {
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+              const double wi = __shfl_sync(FULL, w, i);
+              if (lane > i && act) w = fma(-t[i], wi, w);
+            }
           }
-          w += w2;
-        } else {
-#pragma unroll
-          for (int i = 0; i < N; ++i) {
-            const double wi = __shfl_sync(FULL, w, i);
-            if (lane > i && act) w = fma(-t[i], wi, w);
+          if (act) {
+            if (lane < n) xc[(size_t)j * n + lane] = w;
+            else xc[(size_t)jp * n + lane - n] = w;
           }
-        }
-        if (act) {
-          if (lane < n) xc[(size_t)j * n + lane] = w;
-          else xc[(size_t)jp * n + lane - n] = w;
-        }
-        // operator form: -C' L^-1 times the permuted rows; else -C' times y
-        const double wt = lane < n ? (op ? b : -w) : 0.0;
+          // operator form: -C' L^-1 times the permuted rows; else -C' times y
+          const double wt = lane < n ? (op ? b : -w) : 0.0;
 #pragma unroll
-        for (int r = 0; r < NRM; ++r) {
-          if (r < nr) {
-            const double sr = warp_sum(cp[r] * wt);
-            if (lane == 0) a.XB[(size_t)j * nr * nrhs + (size_t)col * nr + r] = sr;
+          for (int r = 0; r < NRM; ++r) {
+            if (r < nr) {
+              const double sr = warp_sum(cp[r] * wt);
+              if (lane == 0) a.XB[(size_t)j * nr * nrhs + (size_t)col * nr + r] = sr;
+            }
           }
         }
       }
@@ -4650,9 +4823,11 @@ static void last_and_backward(DevState& s, const SweepPlan<T>& p, const WorkSet<
   if (p.bwd_pipe) {
     // the levels with at most 16 pairs (the top) in one CTA, then one
     // pipelined launch per level below
+    // (several right-hand sides: all levels, whose kernel takes eight at once)
     int k = top_level(d.nblock) / 2, k_split = 0;
-    for (int kk = k; kk > 0; kk /= 2)
-      if (pairs_at_level(d.nblock, kk) > 16) { k_split = kk; break; }
+    if (sizeof(T) == 8 && nrhs > 1) k_split = k;
+    for (int kk = k; kk > 0 && !k_split; kk /= 2)
+      if (pairs_at_level(d.nblock, kk) > 16) k_split = kk;
     if (k > k_split) {
       p.bwd_top<<<1, 512, 0, st>>>(a, k, k_split * 2 > 0 ? k_split * 2 : 1);
       check_launch("k_backward_top");

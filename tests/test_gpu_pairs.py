@@ -188,3 +188,15 @@ def test_zero_pivot_in_the_warp_and_cta_kernels(n):
     h.load_system(s)
     assert h.factorize(), h.last_error()
     check(s, synth.rhs(s, 1, seed=4))
+
+
+@pytest.mark.parametrize("n", [8, 16])
+@pytest.mark.parametrize("nrhs", [2, 7, 8, 9, 17])
+@pytest.mark.parametrize("nblock,nr,nx", [(1, 0, 0), (2, 1, 3), (37, 5, 4), (200, 8, 8)])
+@pytest.mark.parametrize("select", ["LU", "QR", "QRP"])
+def test_sweeps_of_several_right_hand_sides(n, nrhs, nblock, nr, nx, select):
+    """The sweeps that take eight right-hand sides of a pair at once: a part of a
+    chunk, a whole one, a remainder of one; borders of zero, of less than the
+    products' four columns, and of eight.  cond(A) <= 6e3 (dense SVD)."""
+    s = synth.collocation(nblock, n, max(0, nx - nr), max(0, nr - nx), nr, nx, seed=n)
+    check(s, synth.rhs(s, nrhs, seed=n + 1), select)
