@@ -20,6 +20,9 @@
 //      per thread reads the U rows four times as often, and the 4-cycle return of
 //      a 16-byte broadcast bounds it.  Row interchanges are a position map, no row
 //      moves.  n = 128, 512 pairs: 1,157 -> 890 us; a lone pair 213 -> 182 us.
+//      X goes to global memory by position without its zero halves: the scattered
+//      4-byte stores cost a sector each (32,000 cycles of a pair, 18,000 without
+//      the zeros).
 //   2. Z = L11^-1 (the inverse of the unit lower triangle of the n pivot rows),
 //      by 32 x 32 diagonal inverses and block forward substitution.
 //   3. with Xt the n pivot rows and Xb the other n rows of the trailing
@@ -37,6 +40,11 @@
 // buffers; tcgen05.commit arrives on the buffer's mbarrier when the MMAs that
 // read it are done.  Every wait on an mbarrier is bounded (about a second):
 // on expiry the kernel reports DEV_TIMEOUT, frees its tensor memory and ends.
+//
+// A lone pair of n = 128 takes 166 us (213 before the panel and the product code
+// were rewritten), 320,000 cycles: 106,000 pivot steps, 48,000 block updates of the
+// panel, 31,000 the inverse, 34,000 + 47,000 the two products (address arithmetic,
+// staging and the border rows, not the tensor cores), the rest copies.
 // ---------------------------------------------------------------------------
 #include "bcr_umma_layout.cuh"
 
@@ -135,7 +143,9 @@ __device__ __forceinline__ void um_batched(int cnt, Ld ld, St st) {
 }
 
 // One product D[128 x Npad] = A[128 x Kpad] * B[Kpad x Npad] with the B operand
-// staged 16 K-rows at a time by all threads from src(c, m) (m the K index).
+// staged 16 K-rows at a time by all threads from src(c, m, in) (m the K index;
+// the address of the element, which is read if `in` is set and zero otherwise;
+// in must be false for c >= Npad).
 // A (hi, lo) must be in shared memory and fenced.  Returns false on a timeout.
 template <typename Src, typename Obs>
 __device__ bool umma_product(const UmmaLayout& L, unsigned char* sm, uint64_t* bars, uint32_t (&par)[2],
@@ -144,13 +154,19 @@ __device__ bool umma_product(const UmmaLayout& L, unsigned char* sm, uint64_t* b
   const int S = L.Kpad / 16;
   const uint32_t sA = smem_u32(sm);
   const int cnt = 16 * L.Npad;  // <= UM_PF * UM_NT
+  // thread: K index m0 of every stage, columns c0, c0 + UM_NT / 16, ...
+  const int m0 = tid & 15, c0 = tid >> 4;
+  const uint32_t ob = umma_b_off(c0, m0, L.LBO_B);
+  static_assert(UM_NT / 16 % 8 == 0, "a thread's columns lie whole core matrices apart");
+  constexpr uint32_t OBU = UM_NT / 16 / 8 * 128;
   // the next stage's elements are loaded one stage ahead, into registers
   float pv[UM_PF];
   auto load_stage = [&](int s) {
 #pragma unroll
     for (int u = 0; u < UM_PF; ++u) {
-      const int e = tid + u * UM_NT;
-      pv[u] = e < cnt ? src(e >> 4, 16 * s + (e & 15)) : 0.0f;
+      bool in = false;
+      const float* g = src(c0 + u * (UM_NT / 16), 16 * s + m0, in);
+      pv[u] = ld_batch_cg(in, g);
     }
   };
   load_stage(0);
@@ -169,7 +185,7 @@ __device__ bool umma_product(const UmmaLayout& L, unsigned char* sm, uint64_t* b
         const int e = tid + u * UM_NT;
         if (e < cnt) {
           const float h = tf32_hi(pv[u]);
-          const uint32_t o = umma_b_off(e >> 4, e & 15, L.LBO_B);
+          const uint32_t o = ob + u * OBU;
           *reinterpret_cast<float*>(bh + o) = h;
           *reinterpret_cast<float*>(bl + o) = pv[u] - h;
         }
@@ -181,25 +197,22 @@ __device__ bool umma_product(const UmmaLayout& L, unsigned char* sm, uint64_t* b
     if (tid == 0) {
       tc_fence_after();
       const uint32_t sB = smem_u32(sm + L.offB + (unsigned)b * 2u * L.szBhalf);
+      // operands in 16-byte units relative to the first one of the stage
+      const uint64_t ah0 = umma_sdesc(sA + (uint32_t)(4 * s) * 2048u, 2048, 128), al0 = ah0 + (L.szAhalf >> 4);
+      const uint64_t bh0 = umma_sdesc(sB, (uint32_t)L.LBO_B, 128), bl0 = bh0 + (L.szBhalf >> 4);
 #pragma unroll
       for (int ks = 0; ks < 2; ++ks) {
-        const int kg = 16 * s + 8 * ks;
-        const uint32_t ao = (uint32_t)(kg >> 2) * 2048u;
-        const uint64_t ah = umma_sdesc(sA + ao, 2048, 128);
-        const uint64_t al = umma_sdesc(sA + L.szAhalf + ao, 2048, 128);
-        const uint32_t bo = (uint32_t)(2 * ks) * (uint32_t)L.LBO_B;
+        const uint64_t ah = ah0 + (uint64_t)(ks * 256), al = al0 + (uint64_t)(ks * 256);
+#pragma unroll
         for (int ch = 0; ch < 2; ++ch) {
           const int nw = ch ? L.N1 : L.N0;
           if (nw == 0) continue;
-          const int c0 = ch ? L.N0 : 0;
-          const uint32_t co = (uint32_t)(c0 >> 3) * 128u;
-          const uint64_t bdh = umma_sdesc(sB + bo + co, (uint32_t)L.LBO_B, 128);
-          const uint64_t bdl = umma_sdesc(sB + L.szBhalf + bo + co, (uint32_t)L.LBO_B, 128);
+          const uint64_t bo = (uint64_t)((2 * ks * L.LBO_B + (ch ? L.N0 * 16 : 0)) >> 4);
           const uint32_t id = umma_idesc_tf32(128, nw);
-          const uint32_t dt = tmem + (uint32_t)c0;
-          umma_tf32(dt, ah, bdh, id, (s > 0 || ks > 0) ? 1u : 0u);
-          umma_tf32(dt, al, bdh, id, 1u);
-          umma_tf32(dt, ah, bdl, id, 1u);
+          const uint32_t dt = tmem + (uint32_t)(ch ? L.N0 : 0);
+          umma_tf32(dt, ah, bh0 + bo, id, (s > 0 || ks > 0) ? 1u : 0u);
+          umma_tf32(dt, al, bh0 + bo, id, 1u);
+          umma_tf32(dt, ah, bl0 + bo, id, 1u);
         }
       }
       umma_commit(&bars[b]);
@@ -230,6 +243,24 @@ __device__ void umma_stage_a(const UmmaLayout& L, unsigned char* sm, Src a) {
   fence_async_smem();
 }
 
+// the same from rows of shared memory, ld floats apart (16-byte aligned)
+__device__ __forceinline__ void umma_stage_a_rows(const UmmaLayout& L, unsigned char* sm, const float* Z, int ld, int n) {
+#pragma unroll 4
+  for (int e = threadIdx.x; e < 32 * L.Kpad; e += UM_NT) {
+    const int i = e & 127, k4 = 4 * (e >> 7);
+    float4 v = *reinterpret_cast<const float4*>(Z + (i < n ? i : 0) * ld + k4);
+    v.x = i < n && k4 < n ? v.x : 0.0f;
+    v.y = i < n && k4 + 1 < n ? v.y : 0.0f;
+    v.z = i < n && k4 + 2 < n ? v.z : 0.0f;
+    v.w = i < n && k4 + 3 < n ? v.w : 0.0f;
+    const float4 h = make_float4(tf32_hi(v.x), tf32_hi(v.y), tf32_hi(v.z), tf32_hi(v.w));
+    const uint32_t o = umma_a_off(i, k4);
+    *reinterpret_cast<float4*>(sm + o) = h;
+    *reinterpret_cast<float4*>(sm + L.szAhalf + o) = make_float4(v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w);
+  }
+  fence_async_smem();
+}
+
 // one row of cnt elements, element c at src[c * stride], into dst[0, round_up(cnt, 16))
 // (16-byte aligned; zero past cnt), the 16 loads of a group issued together
 template <typename S>
@@ -243,15 +274,15 @@ __device__ __forceinline__ void um_load_row(const S* src, int stride, int cnt, f
       *reinterpret_cast<float4*>(dst + c0 + 4 * u) = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
   }
 }
-// cnt elements src[c * stride] (zeros when src is null) to dst[c * dstride]
+// cnt elements src[c * stride] to dst[c * dstride]
 template <typename S>
 __device__ __forceinline__ void um_copy_col(const S* src, int stride, int cnt, float* dst, int dstride) {
-  for (int c0 = 0; c0 < cnt; c0 += 16) {
-    float v[16];
+  for (int c0 = 0; c0 < cnt; c0 += 32) {
+    float v[32];
 #pragma unroll
-    for (int u = 0; u < 16; ++u) v[u] = float(ld_batch(src && c0 + u < cnt, src + (size_t)(c0 + u) * stride));
+    for (int u = 0; u < 32; ++u) v[u] = float(ld_batch(c0 + u < cnt, src + (size_t)(c0 + u) * stride));
 #pragma unroll
-    for (int u = 0; u < 16; ++u)
+    for (int u = 0; u < 32; ++u)
       if (c0 + u < cnt) dst[(size_t)(c0 + u) * dstride] = v[u];
   }
 }
@@ -305,7 +336,12 @@ __global__ void __launch_bounds__(UM_NT, 1) k_factor_lu_umma(FactorArgs<float> a
     float* const Ej = a.E + oj;
     float* const Bj = a.B + (size_t)j * nnx;
     // column c of the pair's U-row [D'_j E'_j B'_j] (n rows)
-    auto ucol = [&](int c) -> float* { return c < n ? Dj + (size_t)c * n : c < n2 ? Ej + (size_t)(c - n) * n : Bj + (size_t)(c - n2) * n; };
+    auto ucol = [&](int c) -> float* {
+      float* const base = c < n ? Dj : c < n2 ? Ej : Bj;
+      return base + (c - (c < n ? 0 : c < n2 ? n : n2)) * n;
+    };
+    // X = [D_jp 0 B_jp; 0 E_j B_j] by position: the zero halves are not stored
+    auto x_stored = [&](int p, int c) { return c < Nc && (c >= n2 || (c < n) == (s_perm[p] < n)); };
     // ------------------------------------------------------------ panel load
     if (tid == 0) s_info = 0;
     // row t of [E_jp; D_j; C_j] by thread t
@@ -489,9 +525,7 @@ __global__ void __launch_bounds__(UM_NT, 1) k_factor_lu_umma(FactorArgs<float> a
       const int r = tid % n;
       if (tid < n) {
         if (first) um_copy_col(a.D0 + ojp + r, n, n, xd, n2); else um_copy_col(a.D + ojp + r, n, n, xd, n2);
-        um_copy_col((const float*)nullptr, n, n, xd + (size_t)n * n2, n2);
       } else {
-        um_copy_col((const float*)nullptr, n, n, xd, n2);
         // E'_j is written here later: plain loads
         if (first) um_copy_col(a.E0 + oj + r, n, n, xd + (size_t)n * n2, n2); else um_copy_col(Ej + r, n, n, xd + (size_t)n * n2, n2);
       }
@@ -524,7 +558,13 @@ __global__ void __launch_bounds__(UM_NT, 1) k_factor_lu_umma(FactorArgs<float> a
             v = (r == c) ? 1.0f : 0.0f;
             const float* Lr = P + s_perm[gr] * LDP + a32;
 #pragma unroll
-            for (int m = 0; m < r; ++m) v = fmaf(-Lr[m], z[m], v);
+            for (int m = 0; m < r; m += 4) {
+              const float4 l = *reinterpret_cast<const float4*>(Lr + m);
+              v = fmaf(-l.x, z[m], v);
+              if (m + 1 < r) v = fmaf(-l.y, z[m + 1], v);
+              if (m + 2 < r) v = fmaf(-l.z, z[m + 2], v);
+              if (m + 3 < r) v = fmaf(-l.w, z[m + 3], v);
+            }
           }
           z[r] = v;
         }
@@ -537,48 +577,74 @@ __global__ void __launch_bounds__(UM_NT, 1) k_factor_lu_umma(FactorArgs<float> a
         for (int t = zt; t < 16 * (r0 / 4); t += 128) {
           const int rr = 2 * (t & 15), cc = 4 * (t >> 4);
           const int g0 = r0 + rr, g1 = g0 + 1;
-          const float* L0 = g0 < n ? P + s_perm[g0] * LDP : nullptr;
-          const float* L1 = g1 < n ? P + s_perm[g1] * LDP : nullptr;
+          const float* L0 = P + s_perm[g0 < n ? g0 : 0] * LDP;
+          const float* L1 = P + s_perm[g1 < n ? g1 : 0] * LDP;
           float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
-          for (int m = cc; m < r0; ++m) {  // Z[m][cc..cc+3] = 0 for m < cc
-            const float4 zv = *reinterpret_cast<const float4*>(Zf + m * LDP + cc);
-            const float l0 = L0 ? L0[m] : 0.0f, l1 = L1 ? L1[m] : 0.0f;
-            s0.x = fmaf(l0, zv.x, s0.x); s0.y = fmaf(l0, zv.y, s0.y);
-            s0.z = fmaf(l0, zv.z, s0.z); s0.w = fmaf(l0, zv.w, s0.w);
-            s1.x = fmaf(l1, zv.x, s1.x); s1.y = fmaf(l1, zv.y, s1.y);
-            s1.z = fmaf(l1, zv.z, s1.z); s1.w = fmaf(l1, zv.w, s1.w);
+#pragma unroll 2
+          for (int m = cc; m < r0; m += 4) {  // Z[m][cc..cc+3] = 0 for m < cc
+            const float4 l0 = *reinterpret_cast<const float4*>(L0 + m), l1 = *reinterpret_cast<const float4*>(L1 + m);
+            const float a0[4] = {l0.x, l0.y, l0.z, l0.w}, a1[4] = {l1.x, l1.y, l1.z, l1.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const float4 zv = *reinterpret_cast<const float4*>(Zf + (m + u) * LDP + cc);
+              s0.x = fmaf(a0[u], zv.x, s0.x); s0.y = fmaf(a0[u], zv.y, s0.y);
+              s0.z = fmaf(a0[u], zv.z, s0.z); s0.w = fmaf(a0[u], zv.w, s0.w);
+              s1.x = fmaf(a1[u], zv.x, s1.x); s1.y = fmaf(a1[u], zv.y, s1.y);
+              s1.z = fmaf(a1[u], zv.z, s1.z); s1.w = fmaf(a1[u], zv.w, s1.w);
+            }
           }
+          if (g0 >= n) s0 = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (g1 >= n) s1 = make_float4(0.f, 0.f, 0.f, 0.f);
           *reinterpret_cast<float4*>(Zf + g0 * LDP + cc) = s0;
           *reinterpret_cast<float4*>(Zf + g1 * LDP + cc) = s1;
         }
         asm volatile("bar.sync 2, 128;" ::: "memory");
-        // Zf[r0:r0+32, 0:r0] = -Z_bb * (that), in place, one column per thread
-        for (int c = zt; c < r0; c += 128) {
-          float y[32];
+        // Zf[r0:r0+32, 0:r0] = -Z_bb * (that), in place: all tiles, then the stores
+        float4 o[3][2];
 #pragma unroll
-          for (int r = 0; r < 32; ++r) y[r] = Zf[(r0 + r) * LDP + c];
+        for (int x = 0; x < 3; ++x) {  // 16 * (r0 / 4) <= 3 * 128 tiles
+          const int t = zt + 128 * x;
+          if (t < 16 * (r0 / 4)) {
+            const int g0 = r0 + 2 * (t & 15), cc = 4 * (t >> 4);
+            float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
+#pragma unroll 2
+            for (int m = r0; m <= g0 + 1; m += 4) {  // Z_bb is zero right of its diagonal
+              const float4 l0 = *reinterpret_cast<const float4*>(Zf + g0 * LDP + m);
+              const float4 l1 = *reinterpret_cast<const float4*>(Zf + (g0 + 1) * LDP + m);
+              const float a0[4] = {l0.x, l0.y, l0.z, l0.w}, a1[4] = {l1.x, l1.y, l1.z, l1.w};
 #pragma unroll
-          for (int r = 31; r >= 0; --r) {
-            const float* Zr = Zf + (r0 + r) * LDP + r0;
-            float s = 0.0f;
-#pragma unroll
-            for (int m = 0; m <= r; ++m) s = fmaf(Zr[m], y[m], s);
-            y[r] = -s;
+              for (int u = 0; u < 4; ++u) {
+                const float4 zv = *reinterpret_cast<const float4*>(Zf + (m + u) * LDP + cc);
+                s0.x = fmaf(a0[u], zv.x, s0.x); s0.y = fmaf(a0[u], zv.y, s0.y);
+                s0.z = fmaf(a0[u], zv.z, s0.z); s0.w = fmaf(a0[u], zv.w, s0.w);
+                s1.x = fmaf(a1[u], zv.x, s1.x); s1.y = fmaf(a1[u], zv.y, s1.y);
+                s1.z = fmaf(a1[u], zv.z, s1.z); s1.w = fmaf(a1[u], zv.w, s1.w);
+              }
+            }
+            o[x][0] = make_float4(-s0.x, -s0.y, -s0.z, -s0.w);
+            o[x][1] = make_float4(-s1.x, -s1.y, -s1.z, -s1.w);
           }
+        }
+        asm volatile("bar.sync 2, 128;" ::: "memory");
 #pragma unroll
-          for (int r = 0; r < 32; ++r) Zf[(r0 + r) * LDP + c] = y[r];
+        for (int x = 0; x < 3; ++x) {
+          const int t = zt + 128 * x;
+          if (t < 16 * (r0 / 4)) {
+            float* dst = Zf + (r0 + 2 * (t & 15)) * LDP + 4 * (t >> 4);
+            *reinterpret_cast<float4*>(dst) = o[x][0];
+            *reinterpret_cast<float4*>(dst + LDP) = o[x][1];
+          }
         }
         asm volatile("bar.sync 2, 128;" ::: "memory");
       }
     }
     __syncthreads();
     // ------------------------------------------------ U12 = Z Xt (tensor cores)
-    umma_stage_a(L, smem_raw, [&](int i, int kk) {
-      return (i < n && kk < n) ? Zf[i * LDP + kk] : 0.0f;
-    });
+    umma_stage_a_rows(L, smem_raw, Zf, LDP, n);
     __syncthreads();
-    bool ok = umma_product(L, smem_raw, s_bar, par, tmem, [&](int c, int m) {
-      return (m < n && c < Nc) ? Xs[(size_t)c * n2 + m] : 0.0f;
+    bool ok = umma_product(L, smem_raw, s_bar, par, tmem, [&](int c, int m, bool& in) -> const float* {
+      in = m < n && x_stored(m, c);
+      return Xs + (c * n2 + m);
     }, [](int, const unsigned char*) {});
     if (!ok) {
       if (tid == 0) report(a.st, DEV_TIMEOUT, j, 0, k);
@@ -609,7 +675,7 @@ __global__ void __launch_bounds__(UM_NT, 1) k_factor_lu_umma(FactorArgs<float> a
     __syncthreads();
     // ------------------------------------------- Xb - L21 U12 (tensor cores)
     umma_stage_a(L, smem_raw, [&](int i, int kk) {
-      return (i < n && kk < n) ? Tj[(size_t)kk * n2 + n + i] : 0.0f;
+      return ld_batch_cg(i < n && kk < n, Tj + (size_t)kk * n2 + n + i);
     });
     __syncthreads();
     // the border rows' -Lc U12 on the CUDA cores from the staged U12 rows, one
@@ -617,30 +683,32 @@ __global__ void __launch_bounds__(UM_NT, 1) k_factor_lu_umma(FactorArgs<float> a
     float bacc[UM_NRMAX];
 #pragma unroll
     for (int r = 0; r < UM_NRMAX; ++r) bacc[r] = 0.0f;
-    ok = umma_product(L, smem_raw, s_bar, par, tmem, [&](int c, int m) {
-      return (m < n && c < Nc) ? ucol(c)[m] : 0.0f;
+    ok = umma_product(L, smem_raw, s_bar, par, tmem, [&](int c, int m, bool& in) -> const float* {
+      in = m < n && c < Nc;
+      return ucol(c) + m;
     }, [&](int s, const unsigned char* bh) {
       if (nr == 0 || tid >= Nc) return;
+      float u[16];
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
         const uint32_t o = umma_b_off(tid, 4 * g, L.LBO_B);
         const float4 h4 = *reinterpret_cast<const float4*>(bh + o);
         const float4 l4 = *reinterpret_cast<const float4*>(bh + L.szBhalf + o);
-        const float u[4] = {h4.x + l4.x, h4.y + l4.y, h4.z + l4.z, h4.w + l4.w};
+        u[4 * g] = h4.x + l4.x; u[4 * g + 1] = h4.y + l4.y; u[4 * g + 2] = h4.z + l4.z; u[4 * g + 3] = h4.w + l4.w;
+      }
+      // past n the staged rows are zeros: any row of Lc will do
+      const float* lc0 = Lc + 16 * s * UM_NRMAX;
+      const int last = min(15, n - 1 - 16 * s);
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const int m = 16 * s + 4 * g + t;
-          if (m < n) {
-            const float4* l4p = reinterpret_cast<const float4*>(Lc + m * UM_NRMAX);
+      for (int r4 = 0; r4 < UM_NRMAX / 4; ++r4) {
+        if (4 * r4 < nr) {
 #pragma unroll
-            for (int r4 = 0; r4 < UM_NRMAX / 4; ++r4) {
-              if (4 * r4 >= nr) break;
-              const float4 lc = l4p[r4];
-              bacc[4 * r4] = fmaf(lc.x, u[t], bacc[4 * r4]);
-              bacc[4 * r4 + 1] = fmaf(lc.y, u[t], bacc[4 * r4 + 1]);
-              bacc[4 * r4 + 2] = fmaf(lc.z, u[t], bacc[4 * r4 + 2]);
-              bacc[4 * r4 + 3] = fmaf(lc.w, u[t], bacc[4 * r4 + 3]);
-            }
+          for (int t = 0; t < 16; ++t) {
+            const float4 lc = *reinterpret_cast<const float4*>(lc0 + min(t, last) * UM_NRMAX + 4 * r4);
+            bacc[4 * r4] = fmaf(lc.x, u[t], bacc[4 * r4]);
+            bacc[4 * r4 + 1] = fmaf(lc.y, u[t], bacc[4 * r4 + 1]);
+            bacc[4 * r4 + 2] = fmaf(lc.z, u[t], bacc[4 * r4 + 2]);
+            bacc[4 * r4 + 3] = fmaf(lc.w, u[t], bacc[4 * r4 + 3]);
           }
         }
       }
@@ -651,13 +719,18 @@ __global__ void __launch_bounds__(UM_NT, 1) k_factor_lu_umma(FactorArgs<float> a
     }
     if (nr > 0 && tid < Nc) {
       const int c = tid;
+      const size_t oc0 = (size_t)jp * nrn + (size_t)(c < n ? c : 0) * nr;
+      float cjp[UM_NRMAX];
+#pragma unroll
+      for (int r = 0; r < UM_NRMAX; ++r) {
+        const bool in = r < nr && c < n;
+        cjp[r] = first ? float(ld_batch(in, a.C0 + oc0 + r)) : ld_batch(in, a.C + oc0 + r);
+      }
 #pragma unroll
       for (int r = 0; r < UM_NRMAX; ++r) {
         if (r < nr) {
           if (c < n) {
-            const size_t oc = (size_t)jp * nrn + r + (size_t)c * nr;
-            const float cjp = first ? float(a.C0[oc]) : a.C[oc];
-            a.C[oc] = cjp - bacc[r];
+            a.C[oc0 + r] = cjp[r] - bacc[r];
           } else if (c < n2) {
             a.Rbuf[(size_t)j * nrn + r + (size_t)(c - n) * nr] = -bacc[r];
           } else {
@@ -672,23 +745,35 @@ __global__ void __launch_bounds__(UM_NT, 1) k_factor_lu_umma(FactorArgs<float> a
       float* const Ejp = a.E + ojp;
       float* const Bjp = a.B + (size_t)jp * nnx;
       const int qd = warp & 3, grp = warp >> 2, i = 32 * qd + lane;
+      const float* const xr = Xs + n + i;
+      const bool top = i < n && s_perm[n + i] < n;  // a row of [D_jp 0 B_jp]
       for (int pc = grp; pc < L.Npad / 16; pc += UM_NW / 4) {
         float v[16];
         float xb[16];
+        const int cb = 16 * pc;
+        const bool whole = (n & 15) == 0 && cb + 16 <= Nc;  // the piece lies in one of D'_jp, E'_jp, B'_jp
+        if (whole) {
+          const bool in = i < n && (cb >= n2 || (cb < n) == top);
 #pragma unroll
-        for (int jj = 0; jj < 16; ++jj) {
-          const int c = 16 * pc + jj;
-          xb[jj] = (i < n && c < Nc) ? Xs[(size_t)c * n2 + n + i] : 0.0f;
+          for (int jj = 0; jj < 16; ++jj) xb[jj] = ld_batch_cg(in, xr + (cb + jj) * n2);
+        } else {
+#pragma unroll
+          for (int jj = 0; jj < 16; ++jj) {
+            const int c = cb + jj;
+            xb[jj] = ld_batch_cg(i < n && c < Nc && (c >= n2 || (c < n) == top), xr + c * n2);
+          }
         }
         tmem_ld16(tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)(16 * pc), v);
         if (i < n) {
+          auto rcol = [&](int c) { return c < n ? Djp + c * n : c < n2 ? Ejp + (c - n) * n : Bjp + (c - n2) * n; };
+          if (whole) {
+            float* col = rcol(cb) + i;
 #pragma unroll
-          for (int jj = 0; jj < 16; ++jj) {
-            const int c = 16 * pc + jj;
-            if (c >= Nc) continue;
-            const float y = xb[jj] - v[jj];
-            float* col = c < n ? Djp + (size_t)c * n : c < n2 ? Ejp + (size_t)(c - n) * n : Bjp + (size_t)(c - n2) * n;
-            col[i] = y;
+            for (int jj = 0; jj < 16; ++jj) col[(size_t)jj * n] = xb[jj] - v[jj];
+          } else {
+#pragma unroll
+            for (int jj = 0; jj < 16; ++jj)
+              if (cb + jj < Nc) rcol(cb + jj)[i] = xb[jj] - v[jj];
           }
         }
       }

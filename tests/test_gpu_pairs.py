@@ -200,3 +200,25 @@ def test_sweeps_of_several_right_hand_sides(n, nrhs, nblock, nr, nx, select):
     products' four columns, and of eight.  cond(A) <= 6e3 (dense SVD)."""
     s = synth.collocation(nblock, n, max(0, nx - nr), max(0, nr - nx), nr, nx, seed=n)
     check(s, synth.rhs(s, nrhs, seed=n + 1), select)
+
+
+@pytest.mark.parametrize("n", [33, 40, 95, 128])
+@pytest.mark.parametrize("nblock,nr,nx", [(2, 0, 0), (3, 1, 1), (40, 16, 16), (5, 13, 4)])
+def test_large_block_fp32_panels(n, nblock, nr, nx):
+    """The tensor-core pair kernel's panel with a partial last block, border rows
+    in a warp of their own and in one with pivot rows, and its products with no
+    borders and the most.  Bar: test_large_block_sweeps' for the mixed path."""
+    s = synth.collocation(nblock, n, max(0, nx - nr), max(0, nr - nx), nr, nx, seed=n)
+    rhs = synth.rhs(s, 2, seed=n + 1)
+    o = po.Oracle(s, "LU", "LU")
+    assert o.factorize(), o.last_error()
+    xo = o.solve(rhs)
+    h = B.BorderedCR()
+    h.load_system(s)
+    h.set_precision(B.PRECISION_MIXED)
+    h.set_refinement(1e-15, 10)
+    assert h.factorize(), h.last_error()
+    x = rhs.copy()
+    assert h.solve_n(2, x.reshape(-1), x.shape[1]), h.last_error()
+    for c in range(2):
+        assert fwd_err(x[c, :s.ncols], xo[c, :s.ncols]) < 1e-9
