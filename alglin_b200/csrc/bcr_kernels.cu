@@ -4330,6 +4330,48 @@ static LubKernel lub_kernel(const LubPlan& p) {
   return p.depth == 32 ? k_factor_lu_lub<512, 4> : p.depth == 48 ? k_factor_lu_lub<512, 6> : k_factor_lu_lub<512, 8>;
 }
 
+// Clusters of 2, 4 and 8 CTAs of k_factor_lu_lub that are resident at once (a
+// cluster lies within one of the GPU's processing clusters, so that of 8 CTAs
+// fewer than 148 / 8 fit); asked for once per thread and shape.
+static void lub_clusters(LubPlan& p) {
+  static_assert(LUB_SLICES_MAX == 8, "one entry per cluster size");
+  struct Entry {
+    LubKernel kernel;
+    size_t smem;
+    int nc[3];
+  };
+  thread_local Entry cache[16];
+  thread_local int used = 0;
+  const LubKernel kernel = lub_kernel(p);
+  int slot = 0;
+  while (slot < std::min(used, 16) && (cache[slot].kernel != kernel || cache[slot].smem != p.smem)) ++slot;
+  if (slot == std::min(used, 16)) {
+    slot = used++ % 16;
+    if (used == 32) used = 16;
+    Entry& en = cache[slot];
+    en.kernel = kernel;
+    en.smem = p.smem;
+    for (int i = 0; i < 3; ++i) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(1024);
+      cfg.blockDim = dim3((unsigned)p.threads);
+      cfg.dynamicSmemBytes = p.smem;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = 2u << i;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      en.nc[i] = 0;
+      if (cudaOccupancyMaxActiveClusters(&en.nc[i], kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        en.nc[i] = 0;
+      }
+    }
+  }
+  for (int i = 0; i < 3; ++i) p.clusters[i] = cache[slot].nc[i];
+}
+
 template <typename T>
 struct FactorPlan {
   void (*cta)(FactorArgs<T>, T*, size_t) = nullptr;  // CTA per pair (large n)
@@ -4473,7 +4515,10 @@ static FactorPlan<T> plan_factor(const DevState& s) {
           : s.sel == SEL_QR ? k_factor_cta<T, SEL_QR> : k_factor_cta<T, SEL_QRP>;
     if constexpr (sizeof(T) == 8) {
       p.lub = s.sel == SEL_LU ? lub_plan(2 * n + d.nr, n, false) : LubPlan{};
-      if (p.lub.threads) smem_limit_once(lub_kernel(p.lub), p.lub.smem);
+      if (p.lub.threads) {
+        smem_limit_once(lub_kernel(p.lub), p.lub.smem);
+        lub_clusters(p.lub);
+      }
     } else {
       const size_t bsm = (size_t)BLK_W * (2 * n + d.nr) * sizeof(T);
       if (s.sel == SEL_LU && n <= 128 && 2 * n + d.nr <= BLK_ROWS_MAX && bsm <= SMEM_MAX) {
@@ -4500,15 +4545,17 @@ static int fusable_rhs(const DevState& s, const FactorPlan<T>& p, int nrhs) {
   return 2 * s.d.n + s.d.nx + nrhs <= p.tc_cols ? nrhs : 0;
 }
 
-// One level of k_factor_lu_lub.  Where the level has fewer pairs than CTAs fit
-// on the GPU, the trailing columns of a pair are split over a cluster of 2, 4 or
-// 8 CTAs (at least 24 columns each: every CTA repeats the panel).
+// One level of k_factor_lu_lub.  Where the level has few pairs, the trailing
+// columns of a pair are split over a cluster of 2, 4 or 8 CTAs (at least 24
+// columns each: every CTA repeats the panel), as long as all clusters are
+// resident at once: 16 pairs of n = 128 in clusters of 8 took two waves, 341 us,
+// and take 212 us in clusters of 4.
 static void launch_lub(const FactorArgs<double>& a, double* slab, size_t slab_elems, const LubPlan& p, long np,
                        cudaStream_t st) {
   const long ctas = 148L * (512 / p.threads);
   const int trail = 2 * a.d.n + a.d.nx;
   int slices = 1;
-  while (slices < LUB_SLICES_MAX && np * slices * 2 <= ctas && trail >= slices * 2 * 24) slices *= 2;
+  for (int i = 0; i < 3 && np <= p.clusters[i] && trail >= slices * 2 * 24; ++i) slices *= 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(slices > 1 ? np * slices : std::min(np, ctas)));
   cfg.blockDim = dim3((unsigned)p.threads);

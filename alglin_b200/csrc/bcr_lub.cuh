@@ -56,6 +56,7 @@ __host__ __device__ inline size_t lub_smem(int rows, int depth) {
 struct LubPlan {
   int threads = 0, bw = 0, depth = 0;
   size_t smem = 0;
+  int clusters[3] = {0, 0, 0};  // clusters of 2, 4 and 8 CTAs resident at once
 };
 inline LubPlan lub_plan(int rows, int npiv, bool alone) {
   LubPlan p;
