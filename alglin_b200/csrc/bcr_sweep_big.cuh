@@ -144,13 +144,17 @@ __global__ void __launch_bounds__(2 * RW, RW == 64 ? 4 : 256 / RW) k_forward_op(
 }
 
 // Forward sweep with L and M (FP32 factors): a thread per row and run of 32
-// columns.  RW: rows, at least 2n; RW / 64 runs.
+// columns.  RW: rows, at least 2n; RW / 64 runs.  The triangles' elements wait in
+// shared memory as doubles, each for the lane that wrote it: 1,024 threads leave
+// 64 registers, and the 31 converted values of the serial part were spilled (a
+// lone pair of n = 128: 22 -> 16 us).
 template <int RW, typename T>
 __global__ void __launch_bounds__(RW * (RW / 64), 1) k_forward_lm(SweepArgs<T> a) {
   constexpr int NT = RW * (RW / 64);
   constexpr unsigned FULL = 0xffffffffu;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double(*y)[RW] = reinterpret_cast<double(*)[RW]>(smem_raw);
+  __shared__ double tri[RW / 64][32][32];  // [triangle][column][row]
   const int tid = threadIdx.x, h = tid / RW, r = tid % RW, lane = tid & 31;
   const Dims d = a.d;
   const int n = d.n, n2 = 2 * n, k = a.k;
@@ -164,6 +168,10 @@ __global__ void __launch_bounds__(RW * (RW / 64), 1) k_forward_lm(SweepArgs<T> a
       const int c = 32 * h + u;
       m[u] = ld_batch(r < n2 && c < n && c < r, Tj + (size_t)c * n2 + r);
     }
+    if (r / 32 == h) {
+#pragma unroll
+      for (int u = 0; u < 32; ++u) tri[h][u][lane] = -double(m[u]);
+    }
     for (int col0 = 0; col0 < a.nrhs; col0 += SWB_RHS) {
       const int nc = min(SWB_RHS, a.nrhs - col0);
       fwd_gather<RW, NT>(a, j, jp, col0, nc, y);
@@ -172,10 +180,10 @@ __global__ void __launch_bounds__(RW * (RW / 64), 1) k_forward_lm(SweepArgs<T> a
         if (h == b && r / 32 == b) {  // the warp of the diagonal block
           for (int c = 0; c < nc; ++c) {
             double v = y[c][r];
-#pragma unroll
+#pragma unroll 8
             for (int u = 0; u < 31; ++u) {
               const double vc = __shfl_sync(FULL, v, u);
-              v = fma(-double(m[u]), lane > u ? vc : 0.0, v);
+              v = fma(tri[b][u][lane], lane > u ? vc : 0.0, v);
             }
             // rows below n of a partial last block are updated here too
             y[c][r] = v;
