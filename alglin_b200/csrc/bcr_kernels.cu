@@ -2782,7 +2782,8 @@ struct PipeItems {
 
 // Eight right-hand sides of one pair of the backward sweep (FP64): the products
 // D' X_jp, E' X_jpp and B' X_b on the tensor cores, then the triangle with four
-// columns per half warp.  buf: the pair's staged factors (overwritten).
+// columns per half warp.  buf: the pair's staged factors (overwritten).  COH: x
+// may have been written earlier in this launch.
 //
 // One column at a time, 50 shuffles and as many multiply-adds repeat for every
 // column, and the triangle's chain of N shuffles is walked once per column: 8
@@ -2792,7 +2793,7 @@ struct PipeItems {
 // that size: 389 to 318 us for 2, 487 to 323 us for 3, 780 to 490 us with the
 // factorization for 8); a single one stays with the scalar code, which does an
 // eighth of the work.
-template <int N, int NXM>
+template <int N, int NXM, bool COH>
 __device__ __forceinline__ void bwd_multi(const SweepArgs<double>& a, int j, int jp, int jpp, double* buf, int lane) {
   using Bf = BwdBuf<N, NXM, double>;
   constexpr unsigned FULL = 0xffffffffu;
@@ -2832,16 +2833,16 @@ __device__ __forceinline__ void bwd_multi(const SweepArgs<double>& a, int j, int
     const double* xg = xc + (size_t)min(g, nc - 1) * a.ldx;
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks) {
-      bd[ks] = ld_batch(g < nc, xg + (size_t)jp * N + 4 * ks + q);
-      be[ks] = ld_batch(g < nc, xg + (size_t)jpp * N + 4 * ks + q);
+      bd[ks] = ld_batch_c<COH>(g < nc, xg + (size_t)jp * N + 4 * ks + q);
+      be[ks] = ld_batch_c<COH>(g < nc, xg + (size_t)jpp * N + 4 * ks + q);
     }
 #pragma unroll
-    for (int ks = 0; ks < 2; ++ks) bb[ks] = ld_batch(g < nc && 4 * ks + q < nx, xg + xb_off + 4 * ks + q);
+    for (int ks = 0; ks < 2; ++ks) bb[ks] = ld_batch_c<COH>(g < nc && 4 * ks + q < nx, xg + xb_off + 4 * ks + q);
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int h = 0; h < 2; ++h)
-        acc[mt][h] = ld_batch(2 * q + h < nc, xc + (size_t)min(2 * q + h, nc - 1) * a.ldx + (size_t)j * N + 8 * mt + g);
+        acc[mt][h] = ld_batch_c<COH>(2 * q + h < nc, xc + (size_t)min(2 * q + h, nc - 1) * a.ldx + (size_t)j * N + 8 * mt + g);
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks)
 #pragma unroll
@@ -2922,7 +2923,7 @@ __global__ void __launch_bounds__(256, 2) k_backward_pipe(SweepArgs<T> a0, const
       T* buf = bufs + cur * Bf::WORDS;
       const bool multi = sizeof(T) == 8 && nrhs > 1;
       if constexpr (sizeof(T) == 8) {
-        if (multi) bwd_multi<N, NXM>(a, j, jp, jpp, buf, lane);
+        if (multi) bwd_multi<N, NXM, false>(a, j, jp, jpp, buf, lane);
       }
       if (!multi) {
         double m[N], u[N], bb[NXM];
@@ -2990,6 +2991,26 @@ __global__ void __launch_bounds__(512, 1) k_backward_top(SweepArgs<T> a, int k_t
   const bool hi = lane >= 16, rowok = i < n;
   const bool qrp = a.sel == SEL_QRP;
   const size_t xb_off = (size_t)(nb + 1) * n + d.qx;
+  if constexpr (sizeof(T) == 8) {
+    if (nrhs > 1) {  // eight right-hand sides at once (the launch brings BwdBuf::WORDS per warp)
+      extern __shared__ __align__(16) unsigned char smem_raw[];
+      T* buf = reinterpret_cast<T*>(smem_raw) + (size_t)warp * BwdBuf<N, NXM, T>::WORDS;
+      for (int k = k_top; k >= k_min && k > 0; k /= 2) {
+        const long np = pairs_at_level(nb, k);
+        for (long q = warp; q < np; q += 16) {
+          const int j = k + (int)(2L * k * q);
+          bwd_stage<N, NXM, T>(a, k, q, buf, lane);
+          cp_async_commit();
+          cp_async_wait<0>();
+          __syncwarp();
+          bwd_multi<N, NXM, true>(a, j, j - k, min(j + k, nb), buf, lane);
+          __syncwarp();
+        }
+        __syncthreads();
+      }
+      return;
+    }
+  }
   for (int k = k_top; k >= k_min && k > 0; k /= 2) {
     const long np = pairs_at_level(nb, k);
     for (long q = warp; q < np; q += 16) {
@@ -4715,6 +4736,7 @@ struct SweepPlan {
   void (*bwd_pipe)(SweepArgs<T>, const SweepArgs<T>*, const BatchCta*, const long*, long) = nullptr;
   size_t bwd_pipe_smem = 0;
   void (*bwd_top)(SweepArgs<T>, int, int) = nullptr;
+  size_t bwd_top_smem = 0;  // with several right-hand sides
   // CTA per pair (16 < n, see bcr_sweep_big.cuh): threads, shared memory per right-hand side
   void (*fwd_big)(SweepArgs<T>) = nullptr;
   void (*bwd_big)(SweepArgs<T>) = nullptr;
@@ -4761,6 +4783,8 @@ static SweepPlan<T> plan_sweeps(const DevState& s) {
       p.bwd_top = x4 ? k_backward_top<8, 4, T> : k_backward_top<8, 8, T>;
     }
     smem_limit_once(p.bwd_pipe, p.bwd_pipe_smem);
+    if (sizeof(T) == 8) p.bwd_top_smem = p.bwd_pipe_smem;  // one buffer for each of twice the warps
+    smem_limit_once(p.bwd_top, p.bwd_top_smem);
   }
   if (n == 32) {
     if (s.sel == SEL_LU && d.nr <= 8) p.fwd = d.nr <= 4 ? k_forward_rows32<T, 4> : k_forward_rows32<T, 8>;
@@ -4869,14 +4893,14 @@ static void last_and_backward(DevState& s, const SweepPlan<T>& p, const WorkSet<
   const size_t smem_b = (size_t)d.n * 8 * WARPS_PANEL;
   if (p.bwd_pipe) {
     // the levels with at most 16 pairs (the top) in one CTA, then one
-    // pipelined launch per level below
-    // (several right-hand sides: all levels, whose kernel takes eight at once)
+    // pipelined launch per level below.  (With several right-hand sides too: one
+    // launch per level at the top made an uncaptured solve of 64 blocks wait for
+    // its launches, 46 against 37 us at n = 8 with 2 right-hand sides.)
     int k = top_level(d.nblock) / 2, k_split = 0;
-    if (sizeof(T) == 8 && nrhs > 1) k_split = k;
     for (int kk = k; kk > 0 && !k_split; kk /= 2)
       if (pairs_at_level(d.nblock, kk) > 16) k_split = kk;
     if (k > k_split) {
-      p.bwd_top<<<1, 512, 0, st>>>(a, k, k_split * 2 > 0 ? k_split * 2 : 1);
+      p.bwd_top<<<1, 512, nrhs > 1 ? p.bwd_top_smem : 0, st>>>(a, k, k_split * 2 > 0 ? k_split * 2 : 1);
       check_launch("k_backward_top");
     }
     for (int kk = k_split; kk > 0; kk /= 2) {
