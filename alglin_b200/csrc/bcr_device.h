@@ -98,6 +98,7 @@ struct BatchClass {
   int nsys = 0;
   int fam = PAIR_AUTO;   // PAIR_TC, PAIR_GRP or PAIR_ROWS
   int mixed = 0;         // FP32 working blocks (refined by the caller)
+  int op = 0;            // form of the factors last written (SweepArgs::op): it stays with them when fam changes
   int chunk = 8;         // pairs per CTA of the factorization launches
   int n = 0, nrm = 0, nxm = 0, levels = 0, nrhs = 1;
   size_t last_smem = 0;

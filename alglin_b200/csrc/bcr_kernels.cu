@@ -6008,6 +6008,7 @@ static void batch_factorize_t(BatchClass& c, cudaStream_t st) {
 
 void batch_factorize(BatchClass& c, cudaStream_t st) {
   if (c.nsys == 0) return;
+  c.op = c.fam == PAIR_TC || c.fam == PAIR_GRP ? c.n : 0;
   if (c.mixed) batch_factorize_t<float>(c, st);
   else batch_factorize_t<double>(c, st);
 }
@@ -6025,7 +6026,7 @@ static void batch_sweeps_rows(BatchClass& c, cudaStream_t st, bool forward, int 
   const bool r4 = c.nrm <= 4, x4 = c.nxm <= 4;
   SweepArgs<T> a0{};
   a0.k = 1 << L;
-  a0.op = c.fam == PAIR_TC || c.fam == PAIR_GRP ? c.n : 0;
+  a0.op = c.op;
   if constexpr (N == 8 || N == 16) {
     if (c.n == N) {  // pipelined: a fixed grid walks the level's map entries
       const long nent = c.scnt[L];
