@@ -193,7 +193,7 @@ struct bcr_handle_s {
     A(dalloc(z.Rbuf, nb * nr * n)); A(dalloc(z.Fbuf, nb * nr * nx));
     z.xb_cap = 16;
     A(dalloc(z.XB, nb * nr * 16));
-    z.part_cap = 97 * (int)std::max<size_t>(256, nr);  // at most 97 parts of 256 sums, or of one column (reduce_blocks)
+    z.part_cap = 97 * 256;  // at most 97 parts of 256 sums (reduce_blocks)
     A(dalloc(z.part, (size_t)z.part_cap));
     A(dalloc(z.Ffin, std::max<size_t>(nr * nx, 1)));
     A(dalloc(z.Hl, (size_t)d.Nr * d.Nc)); A(dalloc(z.tau_l, Lmax)); A(dalloc(z.piv_l, 2 * Lmax));

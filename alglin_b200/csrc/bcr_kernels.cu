@@ -4294,35 +4294,37 @@ static void check_launch(const char* what) {
   }
 }
 
-// sums of per-block m-vectors, m = h x cols (column-major, height h <= 256);
-// column groups of at most 256 elements are reduced one after the other
+// sums of per-block m-vectors, m = h x cols (column-major, height h), in pieces of
+// at most 256 elements, one after the other: groups of whole columns, or for
+// h > 256 the rows of one column
 static void reduce_blocks(DevState& s, const double* buf, long first, long count, int m, int h,
                           const double* base, int ldb, double* out, int ldo, cudaStream_t st) {
   if (m <= 0 || h <= 0) return;
-  const int cols = m / h, cw = h <= 256 ? 256 / h : 1;
+  const int cols = m / h, cw = h <= 256 ? 256 / h : 1, hw = std::min(h, 256);
   // about 96 parts: enough CTAs to have the sums in flight, few enough for the
   // one CTA that adds the parts (16,383 sums of 64 elements took 46 us in 16
   // parts of 1,024); whole rounds of the CTA's 256 / (column height) groups
-  const long unit = std::max(1, 256 / (std::min(cols, cw) * h)) * 8;
+  const long unit = 256 / (std::min(cols, cw) * hw) * 8;
   const long chunk = std::max(unit, (count / 96 + unit) / unit * unit);
   const int nparts = count > 0 ? (int)((count + chunk - 1) / chunk) : 0;
-  for (int c0 = 0; c0 < cols; c0 += cw) {
-    const int cn = cols - c0 < cw ? cols - c0 : cw, mm = cn * h;
-    const double* bb = buf + (size_t)c0 * h;
-    const double* ba = base ? base + (size_t)c0 * ldb : nullptr;
-    double* oo = out + (size_t)c0 * ldo;
-    if (nparts > 1) {
-      k_reduce_tree<double><<<nparts, 256, 0, st>>>(bb, m, first, count, mm, chunk, s.part, nullptr, h,
-                                                    0, nullptr, 0);
+  for (int c0 = 0; c0 < cols; c0 += cw)
+    for (int r0 = 0; r0 < h; r0 += hw) {
+      const int hn = std::min(hw, h - r0), mm = std::min(cw, cols - c0) * hn;
+      const double* bb = buf + (size_t)c0 * h + r0;
+      const double* ba = base ? base + (size_t)c0 * ldb + r0 : nullptr;
+      double* oo = out + (size_t)c0 * ldo + r0;
+      if (nparts > 1) {
+        k_reduce_tree<double><<<nparts, 256, 0, st>>>(bb, m, first, count, mm, chunk, s.part, nullptr, hn,
+                                                      0, nullptr, 0);
+        check_launch("k_reduce_tree");
+        k_reduce_tree<double><<<1, 256, 0, st>>>(s.part, mm, 0, nparts, mm, nparts, nullptr, ba, hn, ldb,
+                                                 oo, ldo);
+      } else {
+        k_reduce_tree<double><<<1, 256, 0, st>>>(bb, m, first, count, mm, chunk, nullptr, ba, hn, ldb, oo,
+                                                 ldo);
+      }
       check_launch("k_reduce_tree");
-      k_reduce_tree<double><<<1, 256, 0, st>>>(s.part, mm, 0, nparts, mm, nparts, nullptr, ba, h, ldb,
-                                               oo, ldo);
-    } else {
-      k_reduce_tree<double><<<1, 256, 0, st>>>(bb, m, first, count, mm, chunk, nullptr, ba, h, ldb, oo,
-                                               ldo);
     }
-    check_launch("k_reduce_tree");
-  }
 }
 
 // ---------------------------------------------------------------------------
