@@ -3922,6 +3922,9 @@ __device__ void last_solve_rows(const double* A, const int* piv, int N, double* 
   }
 }
 
+// shared memory that a launch may ask for without raising the kernel's limit: 48 KB
+// less the 34 KB that last_solve_body holds statically
+constexpr size_t LAST_SOLVE_UNASKED = 14 * 1024;
 template <typename T>
 __device__ void last_solve_body(Dims d, LastBufs lb, const StatusWords* st, T* x, int ldx, int nrhs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -4251,8 +4254,8 @@ __global__ void __launch_bounds__(32 * MVT_W) k_mv_tail(Dims d, const double* H,
 // Raise a kernel's dynamic shared-memory limit once per process and kernel;
 // later calls (for instance inside a CUDA graph capture) only launch.
 template <typename K>
-static void smem_limit_once(K* kernel, size_t bytes) {
-  if (bytes <= 32 * 1024) return;  // 48 KB less what a kernel may hold statically
+static void smem_limit_once(K* kernel, size_t bytes, size_t unasked = 32 * 1024) {
+  if (bytes <= unasked) return;  // 48 KB less what a kernel may hold statically
   static const void* keys[64];
   static size_t done[64];
   static int used = 0;
@@ -4888,6 +4891,7 @@ static void last_and_backward(DevState& s, const SweepPlan<T>& p, const WorkSet<
                               int nrhs, cudaStream_t st) {
   const Dims d = s.d;
   const size_t smem_l = 2 * (size_t)(d.Nr > d.Nc ? d.Nr : d.Nc) * 8;
+  smem_limit_once(k_last_solve<double>, smem_l, LAST_SOLVE_UNASKED);
   k_last_solve<double><<<1, 512, smem_l, st>>>(d, last_bufs(s), s.st, x, ldx, nrhs);
   check_launch("k_last_solve");
   SweepArgs<T> a = sweep_args(s, w, x, ldx, nrhs);
@@ -6101,6 +6105,7 @@ static void batch_solve_t(BatchClass& c, cudaStream_t st, bool compact) {
   const LastDesc* ld = static_cast<const LastDesc*>(c.ld);
   for (int L = 0; L < c.levels; ++L) batch_sweep_level<T>(c, st, true, L, compact);
   kb_reduce_xb<<<c.nsys, 256, 0, st>>>(ld, c.nrhs);
+  smem_limit_once(kb_last_solve, c.last_smem, LAST_SOLVE_UNASKED);
   kb_last_solve<<<c.nsys, 256, c.last_smem, st>>>(ld, c.nrhs);
   for (int L = c.levels - 1; L >= 0; --L) batch_sweep_level<T>(c, st, false, L, compact);
   check_launch("batched solve");

@@ -1,0 +1,45 @@
+"""GPU tests of last blocks of every size, against the CPU oracle or a solution
+that is known."""
+import numpy as np
+import pytest
+
+from alglin_b200 import bcr as B
+from alglin_b200 import synth
+from oracle import pyoracle as po
+from tests._util import fwd_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("order", [960, 961, 976, 977, 1100])
+@pytest.mark.parametrize("last", ["LU", "QR"])
+@pytest.mark.parametrize("batch", [False, True])
+def test_last_blocks_of_about_a_thousand_rows(order, last, batch):
+    """Last blocks whose two work vectors do not fit in what a kernel may use of
+    shared memory without asking (orders of 961 and above).  cond(A) <= 3e3 (dense
+    SVD), 3e3 * 2^-53 * 1,100 rows = 4e-10: bar 1e-9."""
+    n = 4
+    q = order - 2 * n
+    s = synth.collocation(5, n, q, q, 0, 0, seed=order)
+    for i in range(q):
+        s.H[2 * n + i, n + i] += 40.0
+    rhs = synth.rhs(s, 1, seed=3)
+    o = po.Oracle(s, "LU", last)
+    assert o.factorize(), o.last_error()
+    want = o.solve(rhs)
+    h = B.BorderedCR()
+    h.load_system(s)
+    h.select("LU")
+    h.select_last(last)
+    x = rhs.copy()
+    if batch:
+        bt = B.Batch([h])
+        bt.prepare()
+        assert bt.factorize(), bt.last_error()
+        xs = [x[0]]
+        assert bt.solve(xs), bt.last_error()
+        x = np.array(xs)
+    else:
+        assert h.factorize(), h.last_error()
+        assert h.solve_n(1, x.reshape(-1), x.shape[1]), h.last_error()
+    assert fwd_err(x[0, :s.ncols], want[0, :s.ncols]) < 1e-9
