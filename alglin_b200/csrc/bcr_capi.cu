@@ -306,7 +306,7 @@ struct bcr_handle_s {
     int rc = prepare_launch();
     if (rc) return rc;
     enqueue_factorize();
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = bcr::launch_error();
     if (e != cudaSuccess) return cuda_fail(e, "factorize launch");
     pending_status = true;
     factorized = true;  // provisional until the status word is read
@@ -323,7 +323,7 @@ struct bcr_handle_s {
       if (nrhs > 0 && (rc = save_rhs(nrhs, dx, ld))) return rc;
       if (nrhs > 0) bcr::launch_factorize_solve(s, dx, ld, nrhs, stream);  // x0 with the factors
       else enqueue_factorize();
-      cudaError_t e = cudaGetLastError();
+      cudaError_t e = bcr::launch_error();
       if (e != cudaSuccess) return cuda_fail(e, "factorize launch");
       pending_status = true;
       factorized = true;
@@ -332,7 +332,7 @@ struct bcr_handle_s {
     }
     if (nrhs == 0) bcr::launch_factorize(s, stream);
     else bcr::launch_factorize_solve(s, dx, ld, nrhs, stream);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = bcr::launch_error();
     if (e != cudaSuccess) return cuda_fail(e, "factorize_solve launch");
     pending_status = true;
     factorized = true;
@@ -442,7 +442,7 @@ struct bcr_handle_s {
       ++it;
     }
     ir_iters = it;
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = bcr::launch_error();
     if (e != cudaSuccess) return cuda_fail(e, "refinement launch");
     return BCR_OK;
   }
@@ -459,7 +459,7 @@ struct bcr_handle_s {
       return solve_mixed(nrhs, dx, ld, fixed);
     }
     bcr::launch_solve(s, dx, ld, nrhs, stream);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = bcr::launch_error();
     if (e != cudaSuccess) return cuda_fail(e, "solve launch");
     return BCR_OK;
   }
@@ -967,8 +967,10 @@ static int mv_host(bcr_handle h, double alpha, const double* x, double beta, dou
   cudaMemcpyAsync(h->dX, x, nc * 8, cudaMemcpyHostToDevice, h->stream);
   if (beta != 0.0) cudaMemcpyAsync(h->dY, res, nrw * 8, cudaMemcpyHostToDevice, h->stream);
   bcr::launch_mv(h->s, alpha, h->dX, beta, h->dY, h->stream);
+  cudaError_t e = bcr::launch_error();
+  if (e != cudaSuccess) return h->cuda_fail(e, "Mv launch");
   cudaMemcpyAsync(res, h->dY, nrw * 8, cudaMemcpyDeviceToHost, h->stream);
-  cudaError_t e = cudaStreamSynchronize(h->stream);
+  e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return h->cuda_fail(e, "Mv");
   return BCR_OK;
 }
@@ -1153,7 +1155,7 @@ int bcr_factorize_solve(bcr_handle h, int nrhs, double* rhs, int ldRhs) {
       h->factorized = false;
       if (bcr::launch_upload_factorize_solve(h->s, hm, h->dX, (int)Lx, nrhs, h->stream, h->copy_stream,
                                              h->chunk_ev, bcr_handle_s::NCHUNK_EV)) {
-        cudaError_t e = cudaGetLastError();
+        cudaError_t e = bcr::launch_error();
         if (e != cudaSuccess) return h->cuda_fail(e, "factorize_solve launch");
         h->dirty = false;
         h->pending_status = true;
@@ -1194,7 +1196,7 @@ int bcr_mv_device(bcr_handle h, double alpha, const double* d_x, double beta, do
   if (rc) return rc;
   if (h->dirty && (rc = h->upload())) return rc;
   bcr::launch_mv(h->s, alpha, d_x, beta, d_res, h->stream);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = bcr::launch_error();
   return e == cudaSuccess ? BCR_OK : h->cuda_fail(e, "Mv launch");
 }
 
@@ -1255,7 +1257,9 @@ int bcr_graph_capture(bcr_handle h, int what, int nrhs, double* d_x, int ld, con
   h->ir_pending = false;
   cudaGraph_t graph = nullptr;
   e = cudaStreamEndCapture(h->stream, &graph);
-  if (e != cudaSuccess) { cudaGetLastError(); return h->cuda_fail(e, "cudaStreamEndCapture"); }
+  const cudaError_t launched = bcr::launch_error();
+  if (e != cudaSuccess) return h->cuda_fail(e, "cudaStreamEndCapture");
+  if (!rc && launched != cudaSuccess) rc = h->cuda_fail(launched, "graph capture");
   if (rc) { cudaGraphDestroy(graph); return rc; }
   e = cudaGraphInstantiate(&h->graphs[what], graph, 0);
   cudaGraphDestroy(graph);
@@ -1553,14 +1557,14 @@ struct bcr_batch_s {
     }
     cudaMemcpyAsync(d_x, d_sol, x_elems * 8, cudaMemcpyDeviceToDevice, stream);
     ir_iters = it;
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = bcr::launch_error();
     return e == cudaSuccess ? BCR_OK : cuda_fail(e, "batch refinement");
   }
   // the solve step after a factorization, on the rhs region (b kept in d_b)
   int solve_step(int fixed) {
     if (!mixed()) {
       enqueue_solve();
-      cudaError_t e = cudaGetLastError();
+      cudaError_t e = bcr::launch_error();
       return e == cudaSuccess ? BCR_OK : cuda_fail(e, "batch solve");
     }
     return solve_mixed(fixed, true);
@@ -1791,7 +1795,8 @@ int bcr_batch_s::tune_class(size_t ci) {
       cudaEventRecord(e0, stream);
       for (int r = 0; r < 3; ++r) bcr::batch_factorize(c, stream);
       cudaEventRecord(e1, stream);
-      cudaError_t e = cudaEventSynchronize(e1);
+      cudaError_t e = bcr::launch_error();
+      if (e == cudaSuccess) e = cudaEventSynchronize(e1);
       if (e != cudaSuccess) return cuda_fail(e, "batch autotune");
       float ms = 0.f;
       cudaEventElapsedTime(&ms, e0, e1);
@@ -1963,7 +1968,7 @@ int bcr_batch_upload(bcr_batch b) {
 int bcr_batch_factorize(bcr_batch b) {
   B_READY(b);
   b->enqueue_factorize();
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = bcr::launch_error();
   if (e != cudaSuccess) return b->cuda_fail(e, "batch factorize");
   return b->read_status();
 }
@@ -2014,7 +2019,7 @@ int bcr_batch_factorize_solve(bcr_batch b, double* const* x) {
     if ((rc = b->solve_step(-1))) return rc;
   } else {
     b->enqueue_solve();
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = bcr::launch_error();
     if (e != cudaSuccess) return b->cuda_fail(e, "batch factorize_solve");
     if ((rc = b->read_status())) return rc;
   }
@@ -2062,7 +2067,9 @@ int bcr_batch_graph_capture(bcr_batch b) {
   b->ir_pending = false;
   cudaGraph_t g = nullptr;
   e = cudaStreamEndCapture(b->stream, &g);
-  if (e != cudaSuccess) { cudaGetLastError(); return b->cuda_fail(e, "cudaStreamEndCapture"); }
+  const cudaError_t launched = bcr::launch_error();
+  if (e != cudaSuccess) return b->cuda_fail(e, "cudaStreamEndCapture");
+  if (!rc && launched != cudaSuccess) rc = b->cuda_fail(launched, "graph capture");
   if (rc) { cudaGraphDestroy(g); return rc; }
   e = cudaGraphInstantiate(&b->graph, g, 0);
   cudaGraphDestroy(g);

@@ -55,6 +55,10 @@ struct DevState {
 bool use_cta_kernel(const Dims& d);
 size_t cta_slab_elems(const Dims& d);
 
+// the error of the first launch that failed in this thread since the last call of
+// this function, or any other pending error; every caller of the launchers asks
+cudaError_t launch_error();
+
 // factorization of every cyclic-reduction level plus the last block
 void launch_factorize(DevState& s, cudaStream_t st);
 // x: device, column-major (ldx x nrhs); in place, reference semantics

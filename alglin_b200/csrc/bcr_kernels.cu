@@ -4290,11 +4290,21 @@ static int grid_for(long work_items, int per_cta, int cap) {
   return (int)g;
 }
 
+// the first failed launch of this thread since launch_error() was last asked
+static thread_local cudaError_t first_launch_error = cudaSuccess;
+
 static void check_launch(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     fprintf(stderr, "alglin_b200: launch of %s failed: %s\n", what, cudaGetErrorString(e));
+    if (first_launch_error == cudaSuccess) first_launch_error = e;
   }
+}
+
+cudaError_t launch_error() {
+  const cudaError_t e = first_launch_error, last = cudaGetLastError();
+  first_launch_error = cudaSuccess;
+  return e != cudaSuccess ? e : last;
 }
 
 // sums of per-block m-vectors, m = h x cols (column-major, height h), in pieces of

@@ -43,3 +43,23 @@ def test_last_blocks_of_about_a_thousand_rows(order, last, batch):
         assert h.factorize(), h.last_error()
         assert h.solve_n(1, x.reshape(-1), x.shape[1]), h.last_error()
     assert fwd_err(x[0, :s.ncols], want[0, :s.ncols]) < 1e-9
+
+
+def test_a_launch_that_does_not_fit_is_an_error():
+    """A last block whose two work vectors are larger than an SM's shared memory: the
+    launch of its solve is refused, and the call says so.  (The matrix is zero, so
+    that its factorization ends at the first pivot.)  The handle stays usable."""
+    h = B.BorderedCR()
+    h.allocate(1, 2, 12600, 12600, 0, 0)
+    x = np.zeros(h.ncols())
+    with pytest.raises(B.BCRError, match="launch"):
+        h.factorize_solve(1, x, x.size)
+    s = synth.collocation(5, 4, 0, 0, 2, 2, seed=1)
+    rhs = synth.rhs(s, 1, seed=3)
+    o = po.Oracle(s, "LU", "LU")
+    assert o.factorize(), o.last_error()
+    h.load_system(s)
+    x = rhs.copy()
+    assert h.factorize_solve(1, x.reshape(-1), x.shape[1]), h.last_error()
+    # cond(A) = 19 (dense SVD)
+    assert fwd_err(x[0, :s.ncols], o.solve(rhs)[0, :s.ncols]) < 1e-12
