@@ -4581,25 +4581,18 @@ static int fusable_rhs(const DevState& s, const FactorPlan<T>& p, int nrhs) {
   return 2 * s.d.n + s.d.nx + nrhs <= p.tc_cols ? nrhs : 0;
 }
 
-// One level of k_factor_lu_lub.  Where the level has few pairs, the trailing
-// columns of a pair are split over a cluster of 2, 4 or 8 CTAs (at least 24
-// columns each: every CTA repeats the panel), as long as all clusters are
-// resident at once: 16 pairs of n = 128 in clusters of 8 took two waves, 341 us,
-// and take 212 us in clusters of 4.
-static void launch_lub(const FactorArgs<double>& a, double* slab, size_t slab_elems, const LubPlan& p, long np,
-                       cudaStream_t st) {
-  const long ctas = 148L * (512 / p.threads);
-  const int trail = 2 * a.d.n + a.d.nx;
-  int slices = 1;
-  for (int i = 0; i < 3 && np <= p.clusters[i] && trail >= slices * 2 * 24; ++i) slices *= 2;
+// one level of k_factor_lu_lub (see lub_grid)
+static void launch_lub(const FactorArgs<double>& a, double* slab, size_t slab_elems, int slab_ctas, const LubPlan& p,
+                       long np, cudaStream_t st) {
+  const LubGrid g = lub_grid(p, np, 2 * a.d.n + a.d.nx, slab_ctas);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(slices > 1 ? np * slices : std::min(np, ctas)));
+  cfg.gridDim = dim3(g.ctas);
   cfg.blockDim = dim3((unsigned)p.threads);
   cfg.dynamicSmemBytes = p.smem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)slices;
+  at[0].val.clusterDim.x = (unsigned)g.slices;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
@@ -4676,7 +4669,7 @@ static bool factor_levels(DevState& s, const FactorPlan<T>& p, const WorkSet<T>&
     }
     if (p.umma) p.umma<<<grid_for(np, 1, 148), UM_NT, p.umma_smem, st>>>(a, w.slab, s.slab_elems);
     else if (p.lub.threads) {
-      if constexpr (sizeof(T) == 8) launch_lub(a, w.slab, s.slab_elems, p.lub, np, st);
+      if constexpr (sizeof(T) == 8) launch_lub(a, w.slab, s.slab_elems, s.slab_ctas, p.lub, np, st);
     } else if (p.blk) p.blk<<<grid_for(np, 1, s.slab_ctas), 256, p.blk_smem, st>>>(a, w.slab, s.slab_elems);
     else if (p.cta) p.cta<<<grid_for(np, 1, s.slab_ctas), 256, 0, st>>>(a, w.slab, s.slab_elems);
     else if (p.grp) p.grp<<<grid_for(np, 1, p.grp_ctas), p.grp_threads, p.grp_smem, st>>>(a, nullptr, nullptr);
