@@ -3843,6 +3843,15 @@ __device__ void last_fallback_body(Dims d, LastBufs b, StatusWords* st) {
   last_svd(d, b.A2, b, st);
 }
 
+// 1 / d is a normal number, so that x * (1 / d) stands for the quotient x / d; else
+// (d below 2^-1024, where 1 / d overflows, or at the upper end of the range, where
+// it loses bits) the last block's solves divide, whose longer latency each of the
+// N dependent steps pays
+__device__ __forceinline__ bool reciprocal_is_normal(double rd) {
+  const double a = fabs(rd);
+  return a >= 2.2250738585072014e-308 && a <= 1.7976931348623157e308;
+}
+
 // b <- (L U)^-1 P b with the factors by original row (FACT_LU_ROWS), N <= 512:
 // position r on thread r (the CTA has at least N threads), blocks of 32 columns.
 // Each thread reads its row's 32 elements of a block in one batch, a block ahead
@@ -3900,10 +3909,18 @@ __device__ void last_solve_rows(const double* A, const int* piv, int N, double* 
         if (u == lane) ud = m[u];
       double v = r < N ? b[r] : 0.0;
       const double rdi = r < N ? 1.0 / ud : 0.0;
+      if (__all_sync(FULL, r >= N || reciprocal_is_normal(rdi))) {
 #pragma unroll
-      for (int u = 31; u >= 0; --u) {
-        const double xi = __shfl_sync(FULL, v * rdi, u);
-        v = lane == u ? xi : fma(-m[u], lane < u ? xi : 0.0, v);
+        for (int u = 31; u >= 0; --u) {
+          const double xi = __shfl_sync(FULL, v * rdi, u);
+          v = lane == u ? xi : fma(-m[u], lane < u ? xi : 0.0, v);
+        }
+      } else {
+#pragma unroll
+        for (int u = 31; u >= 0; --u) {
+          const double xi = __shfl_sync(FULL, r < N ? v / ud : 0.0, u);
+          v = lane == u ? xi : fma(-m[u], lane < u ? xi : 0.0, v);
+        }
       }
       if (r < N) b[r] = v;
     }
@@ -3959,7 +3976,9 @@ __device__ void last_solve_body(Dims d, LastBufs lb, const StatusWords* st, T* x
     __syncthreads();
     const int lane = tid & 31, r0 = lane, r1 = lane + 32, ld = N + 1;
     const size_t off = (size_t)d.nblock * n;
-    const T d0 = r0 < N ? T(1) / big[r0 * ld + r0] : T(0), d1 = r1 < N ? T(1) / big[r1 * ld + r1] : T(0);
+    const T d0 = r0 < N ? big[r0 * ld + r0] : T(1), d1 = r1 < N ? big[r1 * ld + r1] : T(1);
+    const T rd0 = T(1) / d0, rd1 = T(1) / d1;
+    const bool plain = __all_sync(0xffffffffu, reciprocal_is_normal(rd0) && reciprocal_is_normal(rd1));
     for (int c = tid >> 5; c < nrhs; c += bs >> 5) {
       T* xc = x + (size_t)c * ldx;
       auto at = [&](int r) -> T& { return r < n ? xc[r] : xc[off + (r - n)]; };
@@ -3971,7 +3990,8 @@ __device__ void last_solve_body(Dims d, LastBufs lb, const StatusWords* st, T* x
         if (r1 > i && r1 < N) x1 = fma(-big[i * ld + r1], bi, x1);
       }
       for (int i = N - 1; i >= 0; --i) {
-        const T xi = __shfl_sync(0xffffffffu, i < 32 ? x0 * d0 : x1 * d1, i & 31);
+        const T y = i < 32 ? x0 : x1;
+        const T xi = __shfl_sync(0xffffffffu, plain ? y * (i < 32 ? rd0 : rd1) : y / (i < 32 ? d0 : d1), i & 31);
         x0 = r0 == i ? xi : r0 < i ? fma(-big[i * ld + r0], xi, x0) : x0;
         x1 = r1 == i ? xi : r1 < i ? fma(-big[i * ld + r1], xi, x1) : x1;
       }

@@ -63,3 +63,44 @@ def test_a_launch_that_does_not_fit_is_an_error():
     assert h.factorize_solve(1, x.reshape(-1), x.shape[1]), h.last_error()
     # cond(A) = 19 (dense SVD)
     assert fwd_err(x[0, :s.ncols], o.solve(rhs)[0, :s.ncols]) < 1e-12
+
+
+@pytest.mark.parametrize("n", [2, 8, 16, 32, 33, 128])
+@pytest.mark.parametrize("nrhs", [1, 3])
+@pytest.mark.parametrize("batch", [False, True])
+def test_last_pivot_below_the_normal_numbers(n, nrhs, batch):
+    """A single block, so that the last block is the matrix, of order 4 to 256, whose
+    last pivot is 2^-1026: its reciprocal overflows, the quotients do not.  The
+    last row has no other element and its unknown is a small integer, so that its
+    right-hand side and the quotient are exact."""
+    if batch and (n > 32 or n == 2 or nrhs > 1):
+        pytest.skip("batches take one right-hand side and their own block orders")
+    N, tiny = 2 * n, np.ldexp(1.0, -1026)
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((N, N)) * 0.1 + 4.0 * np.eye(N)
+    A[-1] = 0.0
+    A[-1, -1] = tiny
+    s = synth.collocation(1, n)
+    s.D[0], s.E[0] = A[:n, :n].T, A[:n, n:].T
+    s.H[:] = A[n:].T
+    want = rng.standard_normal((nrhs, N))
+    want[:, -1] = rng.integers(1, 8, nrhs)
+    x = want @ A.T
+    x[:, -1] = want[:, -1] * tiny
+    assert (x[:, -1] / tiny == want[:, -1]).all()
+    h = B.BorderedCR()
+    h.load_system(s)
+    h.select("LU")
+    h.select_last("LU")
+    if batch:
+        bt = B.Batch([h])
+        bt.prepare()
+        assert bt.factorize(), bt.last_error()
+        xs = [x[0].copy()]
+        assert bt.solve(xs), bt.last_error()
+        x = np.array(xs)
+    else:
+        assert h.factorize(), h.last_error()
+        assert h.solve_n(nrhs, x.reshape(-1), x.shape[1]), h.last_error()
+    assert (x[:, -1] == want[:, -1]).all()
+    assert np.abs(x - want).max() < 1e-12 * np.abs(want).max()
