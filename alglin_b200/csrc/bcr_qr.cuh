@@ -29,6 +29,21 @@ struct QrShape {
 __device__ __forceinline__ double qr_sqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float qr_sqrt(float x) { return sqrtf(x); }
 
+// Exponents of the columns.  The products x_r a_r are of the elements as they are,
+// without the reflector's scale, so a column whose largest element is not within
+// 2^+-MOST is divided by a power of two first (exactly; QR commutes with it, and
+// the column's results are multiplied again): the products of two columns then
+// stay in the range, wherever in it the columns lie.
+__device__ __forceinline__ unsigned qr_key(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned qr_key(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+template <typename T>
+struct QrRange {
+  static constexpr bool F64 = sizeof(T) == 8;
+  static constexpr int MANT = F64 ? 20 : 23, BIAS = F64 ? 1023 : 127, MOST = F64 ? 250 : 30, CLAMP = F64 ? 1000 : 120;
+};
+__device__ __forceinline__ void qr_pow2(int e, double& p) { p = __hiloint2double((1023 + e) << 20, 0); }
+__device__ __forceinline__ void qr_pow2(int e, float& p) { p = __int_as_float((127 + e) << 23); }
+
 template <typename T, bool PIVOT>
 __device__ __forceinline__ void qr_pair(const FactorArgs<T>& a, int j, T* Vs, int lane) {
   using Q = QrShape<T>;
@@ -83,6 +98,25 @@ __device__ __forceinline__ void qr_pair(const FactorArgs<T>& a, int j, T* Vs, in
 #pragma unroll
     for (int r = 0; r < RW; ++r) v[r] = live && r < n2 ? S[r * 33 + lane] : T(0);
     __syncwarp();
+    T un = T(1);  // this lane's column was divided by un
+    {
+      using Rg = QrRange<T>;
+      unsigned key = 0u;
+#pragma unroll
+      for (int r = 0; r < RW; ++r) key = max(key, qr_key(v[r]));
+      const int ex = (int)(key >> Rg::MANT) - Rg::BIAS;
+      const bool out = key != 0u && ex <= Rg::BIAS && (ex > Rg::MOST || ex < -Rg::MOST);
+      if (__any_sync(FULL, out)) {
+        const int e = out ? min(max(ex, -Rg::CLAMP), Rg::CLAMP) : 0;
+        T sc;
+        qr_pow2(e, un);
+        qr_pow2(-e, sc);
+#pragma unroll
+        for (int r = 0; r < RW; ++r) v[r] *= sc;
+#pragma unroll
+        for (int r = 0; r < NRM; ++r) cb[r] *= sc;
+      }
+    }
 #pragma unroll 1
     for (int i = 0; i < n; ++i) {
       T* x = Vs + i * RW;
@@ -97,7 +131,7 @@ __device__ __forceinline__ void qr_pair(const FactorArgs<T>& a, int j, T* Vs, in
             q1 = v[r + 1] * v[r + 1] + q1;
           }
           const bool cand = panel && cpos >= i;
-          T best = cand ? q0 + q1 : T(-1);
+          T best = cand ? (q0 + q1) * un * un : T(-1);
           if (!(best == best)) best = T(-0.5);  // NaN loses against every number
           int at = cand ? cpos : 64;
           warp_argmax(best, at);
@@ -150,7 +184,7 @@ __device__ __forceinline__ void qr_pair(const FactorArgs<T>& a, int j, T* Vs, in
 #pragma unroll
           for (int r = 0; r < NRM; ++r) sc[2 + r] = l[r];
         }
-        S[i * 33 + lane] = r0;  // row i of R and of the trailing columns
+        S[i * 33 + lane] = r0 * un;  // row i of R and of the trailing columns
         // apply and move one row up; finished panel columns are not used again
         v[0] = fma(-ws, x[1], v[1]);
 #pragma unroll
@@ -175,7 +209,7 @@ __device__ __forceinline__ void qr_pair(const FactorArgs<T>& a, int j, T* Vs, in
         const T r0 = v[0] - w;
 #pragma unroll
         for (int r = 0; r < NRM; ++r) cb[r] = fma(-sc[2 + r], r0, cb[r]);
-        S[i * 33 + lane] = r0;
+        S[i * 33 + lane] = r0 * un;
         v[0] = fma(-ws, x[1], v[1]);
 #pragma unroll
         for (int r = 2; r < RW; r += 2) {
@@ -193,7 +227,7 @@ __device__ __forceinline__ void qr_pair(const FactorArgs<T>& a, int j, T* Vs, in
     // the reduced rows below the rows of R
 #pragma unroll
     for (int r = 0; r < 16; ++r)
-      if (r < n) S[(n + r) * 33 + lane] = v[r];
+      if (r < n) S[(n + r) * 33 + lane] = v[r] * un;
     if (c0 == 0) {
       if (panel) cmap[cpos] = (unsigned char)lane;
     }
@@ -245,11 +279,11 @@ __device__ __forceinline__ void qr_pair(const FactorArgs<T>& a, int j, T* Vs, in
         if (r < nr) {
           if (c < n2) {
             const size_t o = (size_t)jp * nrn + (size_t)(c - n) * nr + r;
-            a.C[o] = src(a.C0, a.C, o) + cb[r];
+            a.C[o] = src(a.C0, a.C, o) + cb[r] * un;
           } else if (c < 3 * n) {
-            a.Rbuf[(size_t)j * nrn + (size_t)(c - n2) * nr + r] = cb[r];
+            a.Rbuf[(size_t)j * nrn + (size_t)(c - n2) * nr + r] = cb[r] * un;
           } else {
-            a.Fbuf[(size_t)j * nrnx + (size_t)(c - 3 * n) * nr + r] = (double)cb[r];
+            a.Fbuf[(size_t)j * nrnx + (size_t)(c - 3 * n) * nr + r] = (double)(cb[r] * un);
           }
         }
     }
