@@ -4471,6 +4471,22 @@ static bool tc_pair_selected(const DevState& s) {
          (!s.mixed && (s.pair_kernel == PAIR_TREE || s.pair_kernel == PAIR_TC_GATHER));
 }
 
+// The register QR kernel against the shared-memory one on a level of np pairs.  Its
+// cost is a whole warp's registers per step, in two passes where the work matrix
+// has more than 32 columns; the other's shrinks with the order and with every
+// column beyond a multiple of 32 eliminated.  Few pairs (up to two per scheduler):
+// the chain of a lone pair decides, 0.80 to 1.02 of the other's time from order 7
+// on in one pass, 0.81 to 0.98 at 12 and 13 and 0.79 to 0.90 at 10 and 11 in two
+// passes (1.00 to 1.10 there below 36 columns; 1.01 to 1.15 at 7 to 9).  Many
+// pairs: the work does, 0.70 to 1.05 from order 12 and 39 columns on, and 1.05 to
+// 2.1 below, for which that kernel stays.
+static bool qr_warp_faster(const Dims& d, long np) {
+  const int cols = 3 * d.n + d.nx;
+  if (d.n >= 12 && cols >= 39) return true;
+  if (np > 148L * 8) return false;
+  return cols <= 32 ? d.n >= 7 : d.n >= 12 || (d.n >= 10 && cols >= 36);
+}
+
 template <typename T>
 static FactorPlan<T> plan_factor(const DevState& s) {
   const Dims d = s.d;
@@ -4558,8 +4574,9 @@ static FactorPlan<T> plan_factor(const DevState& s) {
     else if (n <= 8) p.rows = k_factor_lu_rows<T, 8, 4, 4>;
     else if (n <= 16) p.rows = k_factor_lu_rows<T, 16, 4, 4>;
   }
-  // QR panels in registers; a forced family keeps the shared-memory kernels
-  if (s.sel != SEL_LU && n <= 16 && d.nr <= 8 && n + d.nx <= 32 && s.pair_kernel == PAIR_AUTO) {
+  // QR panels in registers where some level gains (see qr_warp_faster); a forced
+  // family keeps the shared-memory kernels
+  if (s.sel != SEL_LU && n <= 16 && d.nr <= 8 && n + d.nx <= 32 && s.pair_kernel == PAIR_AUTO && qr_warp_faster(d, 1)) {
     p.qr = s.sel == SEL_QR ? k_factor_qr_warp<T, false> : k_factor_qr_warp<T, true>;
     smem_limit_once(p.qr, QrShape<T>::BYTES * 4);
   }
@@ -4695,7 +4712,7 @@ static bool factor_levels(DevState& s, const FactorPlan<T>& p, const WorkSet<T>&
     else if (p.grp) p.grp<<<grid_for(np, 1, p.grp_ctas), p.grp_threads, p.grp_smem, st>>>(a, nullptr, nullptr);
     else if (p.tc) p.tc<<<grid_for(np, 4, 148 * 16), 128, p.tc_smem, st>>>(a, nullptr, nullptr);
     else if (p.rows) p.rows<<<grid_for(np, 4, 148 * 16), 128, 0, st>>>(a, nullptr, nullptr);
-    else if (p.qr) p.qr<<<grid_for(np, 4, 148 * 16), 128, QrShape<T>::BYTES * 4, st>>>(a, nullptr, nullptr);
+    else if (p.qr && qr_warp_faster(d, np)) p.qr<<<grid_for(np, 4, 148 * 16), 128, QrShape<T>::BYTES * 4, st>>>(a, nullptr, nullptr);
     else p.smem_k<<<grid_for(np, p.wpb, 148 * 16), p.wpb * 32, p.smem, st>>>(a, nullptr, nullptr);
     check_launch("k_factor_level");
     if (nrn) {

@@ -12,11 +12,13 @@
 // The registers rotate by one row per step, so that one rolled loop covers all
 // steps (row i of R leaves through shared memory; after n steps the registers
 // hold the reduced rows).  Columns beyond the first pass's (the panel and x_jp,
-// or all of them when they fit in a warp) replay the reflectors.
+// or all of them when they fit in a warp) replay the reflectors in a second pass.
 // Bound by the FP64 pipe and the posting's latency; the shared-memory kernel this
 // replaces walked the whole work matrix there, one lane per column with every
 // element loaded and stored at each step: a lone pair at n = 16 took 62 us and
-// takes 30, level 1 of 20,011 blocks 444 and 229 us.
+// takes 30, level 1 of 20,011 blocks 444 and 229 us (the scales of the columns took
+// 2% of that back).  For which orders and levels it is the faster one:
+// qr_warp_faster.
 #pragma once
 
 template <typename T>
@@ -62,8 +64,8 @@ __device__ __forceinline__ void qr_pair(const FactorArgs<T>& a, int j, T* Vs, in
   const bool rok = hr < n;
   int info = 0, cpos = lane;
   auto src = [&](const double* orig, const T* work, size_t i) -> T { return ldsrc(first, orig, work, i); };
-  for (int c0 = 0; c0 < NC; c0 += W0) {
-    const int nc = min(W0, NC - c0);  // columns of this pass
+  for (int c0 = 0; c0 < NC; c0 += c0 == 0 ? W0 : 32) {
+    const int nc = c0 == 0 ? W0 : NC - c0;  // columns of this pass (n + nx <= 32 in the second)
     __syncwarp();
     // stage the pass's columns (half a warp per column, every load in flight
     // before the first store), then one column per lane
