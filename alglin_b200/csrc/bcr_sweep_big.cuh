@@ -56,23 +56,40 @@ __device__ __forceinline__ void fwd_scatter(const SweepArgs<T>& a, int j, int jp
   }
 }
 
-// XB_j = sgn * C_j v (v[c][RW], first n entries), one border row per warp
+// XB_j = sgn * C_j v (v[c][RW], first n entries), one border row per warp; four in
+// the CTAs of two warps, where one after the other cost a solve of 60 blocks of
+// n = 17 with 12 border rows 6 us of 100
 template <int RW, int NT, typename T>
 __device__ __forceinline__ void fwd_border(const SweepArgs<T>& a, int j, int col0, int nc, const double (*v)[RW],
                                            double sgn) {
+  constexpr int U = RW / 64, W = NT / 32, G = W == 2 ? 4 : 1;
   const int n = a.d.n, nr = a.d.nr, lane = threadIdx.x & 31;
   const T* Cj = a.C + (size_t)j * nr * n;
-  for (int r = threadIdx.x >> 5; r < nr; r += NT / 32) {
-    T cv[4];
+  for (int r0 = threadIdx.x >> 5; r0 < nr; r0 += G * W) {
+    T cv[G][U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) cv[u] = ld_batch(lane + 32 * u < n, Cj + (size_t)(lane + 32 * u) * nr + r);
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = lane + 32 * u, r = r0 + g * W;
+        cv[g][u] = ld_batch(i < n && r < nr, Cj + (size_t)i * nr + r);
+      }
     for (int c = 0; c < nc; ++c) {
-      double s = 0.0;
+      double s[G];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (lane + 32 * u < n) s = fma(double(cv[u]), v[c][lane + 32 * u], s);
-      s = warp_sum(s);
-      if (lane == 0) a.XB[(size_t)j * nr * a.nrhs + (size_t)(col0 + c) * nr + r] = sgn * s;
+      for (int g = 0; g < G; ++g) {
+        s[g] = 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (lane + 32 * u < n) s[g] = fma(double(cv[g][u]), v[c][lane + 32 * u], s[g]);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int g = 0; g < G; ++g) s[g] += shfl_xor(s[g], o);
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        if (lane == 0 && r0 + g * W < nr) a.XB[(size_t)j * nr * a.nrhs + (size_t)(col0 + c) * nr + r0 + g * W] = sgn * s[g];
     }
   }
 }
