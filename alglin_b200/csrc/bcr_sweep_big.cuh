@@ -275,8 +275,21 @@ __global__ void __launch_bounds__(RB * (RB / 32), RB == 32 ? 16 : RB == 64 ? 4 :
 #pragma unroll
         for (int u = 0; u < 4; ++u)
           if (h + NH * u < nx) s = fma(double(bv[u]), xb[h + NH * u], s);
-        for (int e = h + NH * 4; e < nx; e += NH)
-          if (i < n) s = fma(double(Bj[(size_t)e * n + i]), xb[e], s);
+        if constexpr (NH == 1) {
+          // more than four border columns on one warp: eight loads in flight (one
+          // after the other, 60 blocks of n = 17 with 14 of them took 86 us, now 79)
+          for (int e0 = 4; e0 < nx; e0 += 8) {
+            T bm[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) bm[u] = ld_batch(i < n && e0 + u < nx, Bj + (size_t)(e0 + u) * n + i);
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              if (e0 + u < nx) s = fma(double(bm[u]), xb[e0 + u], s);
+          }
+        } else {
+          for (int e = h + NH * 4; e < nx; e += NH)
+            if (i < n) s = fma(double(Bj[(size_t)e * n + i]), xb[e], s);
+        }
         part[c][tid] = s;
       }
       load(Tj, n2, i);  // U, on and right of the diagonal
