@@ -70,11 +70,6 @@ __device__ __forceinline__ T ldsrc_c(bool first, const double* orig, const T* wo
   if constexpr (COH) return first ? T(__ldcg(orig + i)) : __ldcg(work + i);
   else return ldsrc(first, orig, work, i);
 }
-template <bool COH, typename T>
-__device__ __forceinline__ T ldro(const T* p) {
-  if constexpr (COH) return __ldcg(p);
-  else return __ldg(p);
-}
 
 // Element of a batch of loads, 0 where p is false.  volatile keeps the loads of
 // an unrolled batch together: scheduled by the compiler, each one waits for the
@@ -1335,18 +1330,6 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // FP64 tensor cores (DMMA 8x8x4) for double, as a 3xTF32 split on the tensor
 // cores for float at n = 32, on the FP32 pipe for float at n = 16.
 // ---------------------------------------------------------------------------
-// total order of pivot candidates: (hi, lo) of |a|, NaN below every number,
-// finished rows below everything
-__device__ __forceinline__ void pivot_key(double av, bool done, unsigned& hi, unsigned& lo) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(av);
-  hi = done ? 0u : (av != av ? 1u : (unsigned)(b >> 32) + 1u);
-  lo = (done || av != av) ? 0u : (unsigned)b;
-}
-__device__ __forceinline__ void pivot_key(float av, bool done, unsigned& hi, unsigned& lo) {
-  hi = done ? 0u : (av != av ? 1u : (unsigned)__float_as_uint(av) + 1u);
-  lo = 0u;
-}
-
 template <typename T, int N>
 struct GrpShape {
   static constexpr int TPP = 2 * N;        // panel threads, one per panel row
@@ -3436,11 +3419,6 @@ __global__ void __launch_bounds__(256, 2) k_backward_rows32(SweepArgs<TF> a0, co
   });
 }
 
-// ---------------------------------------------------------------------------
-// sweeps for large blocks (n > 32, n <= 128): one CTA per pair, the 2n
-// values of the pair in shared memory, the triangular solves blocked by 32
-// rows (one warp solves a diagonal block with shuffles, the CTA applies it to
-// the rows that follow)
 #include "bcr_sweep_big.cuh"
 
 // ---------------------------------------------------------------------------
@@ -3622,8 +3600,9 @@ __device__ void last_svd(Dims d, const double* A, LastBufs b, StatusWords* st) {
 // solvers: LU (getrf), LUPQ (complete pivoting), QR (geqrf), QRP (geqp3: the
 // column of largest remaining 2-norm first), and the SVD family
 // Last blocks of order <= LAST_SMALL (configs with n <= 16 and small borders):
-// the LU runs out of shared memory (the general loop below works in global
-// memory, a round trip per column) and the LU solves run on one warp with the
+// the LU of a batch's systems runs out of shared memory (the general loop below
+// works in global memory, a round trip per column; single systems take
+// k_last_lu_blocked), and the solves give every right-hand side a warp, its
 // values in registers.  Same pivot rule (largest |a|, first row on ties, NaN
 // never chosen), same operation order.
 constexpr int LAST_SMALL = 64;
@@ -5325,9 +5304,7 @@ __device__ bool queue_next(const BatchQueue& qu, const BatchCta* items, const Fa
   return true;
 }
 
-// CTA-wide: count the item's pairs; the CTA completing the (system, level)
-// applies the level's C_jpp updates and publishes the level
-// the C_jpp updates of every pair of (system, level): C_jpp += Rbuf[j], four
+// The C_jpp updates of every pair of (system, level): C_jpp += Rbuf[j], four
 // elements per thread and round with their loads in flight together
 template <typename T>
 __device__ void level_fixup(const FactorArgs<T>& a, const BatchCta& c, int tid, int nthr) {

@@ -25,7 +25,7 @@
 // because the results overwrite the sources.
 //
 // What bounds it (n = 128, nr = nx = 16, cycles of a pair on one SM): the pivot
-// steps, 179,000 (about 1,000 each, dependent integer and reduction latencies),
+// steps, 179,000 (1,400 each, dependent integer and reduction latencies),
 // and the products, 325,000 (8.6 M fused multiply-adds: 148,000 at the FP64
 // rate; the fragment and accumulator traffic takes the L1 pipe nearly as long).
 // 1,024 blocks of n = 128: the factorization's levels 8.8 -> 4.1 ms; a lone pair
@@ -325,7 +325,7 @@ struct LubCols {
 // Columns [cb, cb + 16) of the group, row tiles [t0, t1) of 16 (the first
 // depth / 16 are the block's pivots).  byrow: destinations by original row.
 template <int NT, int NB>
-__device__ __forceinline__ void lub_item(const LubShared<NT>& sh, const double* Pb, int ld, int w, const LubCols& G,
+__device__ __forceinline__ void lub_item(const LubShared<NT>& sh, const double* Pb, int ld, const LubCols& G,
                                          int cb, int t0, int t1, bool u_byrow, bool c_byrow) {
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   constexpr int PT = NB / 2;  // pivot tiles
@@ -424,7 +424,7 @@ __device__ __forceinline__ void lub_item(const LubShared<NT>& sh, const double* 
 // Item `it` of the strips of 16 columns of ng groups, each split in `parts` row
 // ranges; group(i) gives the columns of group i, make(i) its description.
 template <int NB, int NT, typename Cols, typename Make>
-__device__ __forceinline__ void lub_update(const LubShared<NT>& sh, const double* Pb, int ld, int w, int ng,
+__device__ __forceinline__ void lub_update(const LubShared<NT>& sh, const double* Pb, int ld, int ng,
                                            bool whole, bool u_byrow, bool c_byrow, Cols cols, Make make) {
   const int warp = threadIdx.x >> 5, nw = NT / 32;
   int ns = 0;
@@ -447,7 +447,7 @@ __device__ __forceinline__ void lub_update(const LubShared<NT>& sh, const double
       ++i;
     }
     const int t0 = it / ns * tp, t1 = t0 + tp < tiles ? t0 + tp : tiles;
-    if (t0 < t1) lub_item<NT, NB>(sh, Pb, ld, w, make(i), 16 * s, t0, t1, u_byrow, c_byrow);
+    if (t0 < t1) lub_item<NT, NB>(sh, Pb, ld, make(i), 16 * s, t0, t1, u_byrow, c_byrow);
   }
 }
 
@@ -633,7 +633,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_factor_lu_lub(FactorArgs<doubl
         }
         return G;
       };
-      lub_update<NB>(sh, Pb, ld, w, 4, false, false, !last, cols, make);
+      lub_update<NB>(sh, Pb, ld, 4, false, false, !last, cols, make);
       __syncthreads();
       if (!last) {
         lub_shrink(sh, DEPTH);
@@ -704,7 +704,7 @@ __device__ int lub_square(LubShared<NT>& sh, double* smem, double* W, int N, int
     __syncthreads();
     lub_operator(sh, Pb, ld, nl, w, DEPTH);
     __syncthreads();
-    lub_update<NB>(sh, Pb, ld, w, 1, true, true, true, [&](int) { return N - kb - w; },
+    lub_update<NB>(sh, Pb, ld, 1, true, true, true, [&](int) { return N - kb - w; },
                    [&](int) {
                      double* c = W + (size_t)(kb + w) * N;
                      return LubCols{N - kb - w, c, N, 0, N, c, N, c, N, 0, nullptr, nullptr, 0};

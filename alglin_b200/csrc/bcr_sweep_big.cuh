@@ -160,11 +160,13 @@ __global__ void __launch_bounds__(2 * RW, RW == 64 ? 4 : 256 / RW) k_forward_op(
   }
 }
 
-// Forward sweep with L and M (FP32 factors): a thread per row and run of 32
-// columns.  RW: rows, at least 2n; RW / 64 runs.  The triangles' elements wait in
-// shared memory as doubles, each for the lane that wrote it: 1,024 threads leave
-// 64 registers, and the 31 converted values of the serial part were spilled (a
-// lone pair of n = 128: 22 -> 16 us).
+// Forward sweep with L and M (FP32 factors of the tensor-core kernel; factors of
+// k_factor_level, k_factor_cta and k_factor_lu_blocked in either precision): a
+// thread per row and run of 32 columns.  RW: rows, at least 2n; RW / 64 runs.  The
+// triangles' elements wait in shared memory as doubles, each for the lane that wrote
+// it: 1,024 threads leave 64 registers, and the 31 converted values of the serial
+// part were spilled (a lone pair of n = 128: 22 -> 16 us).  The instances of 1,024
+// threads still spill about 270 bytes, of the 32 elements that wait for their use.
 template <int RW, typename T>
 __global__ void __launch_bounds__(RW * (RW / 64), 1) k_forward_lm(SweepArgs<T> a) {
   constexpr int NT = RW * (RW / 64);
@@ -220,6 +222,7 @@ __global__ void __launch_bounds__(RW * (RW / 64), 1) k_forward_lm(SweepArgs<T> a
 
 // Backward sweep: x_j = U^-1 (y_j - D'_j x_jp - E'_j x_jpp - B'_j xb), a thread
 // per row and run of 32 columns.  RB: rows, at least n; RB / 32 runs.
+// (The instances are held to 128 registers; those in FP64 spill 260 bytes.)
 template <int RB, typename T>
 __global__ void __launch_bounds__(RB * (RB / 32), RB == 32 ? 16 : RB == 64 ? 4 : 1) k_backward_big(SweepArgs<T> a) {
   constexpr int NH = RB / 32, NT = RB * NH;
