@@ -4098,8 +4098,7 @@ __global__ void k_last_factor(Dims d, LastBufs b, int sel_last, StatusWords* st)
 // load_and_factorize_last with LU for larger blocks (cc:1319-1346, getrf): the
 // blocked elimination of the pair kernels on the whole block, FP64 tensor-core
 // products, rows left in place (kind FACT_LU_ROWS, piv[pos] = row)
-template <int NB>
-__global__ void __launch_bounds__(512, 1) k_last_lu_blocked(Dims d, LastBufs b, StatusWords* st, int bw) {
+__global__ void __launch_bounds__(512, 1) k_last_lu_blocked(Dims d, LastBufs b, StatusWords* st) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ LubShared<512> sh;
   const int N = d.Nc, tid = threadIdx.x;
@@ -4107,7 +4106,7 @@ __global__ void __launch_bounds__(512, 1) k_last_lu_blocked(Dims d, LastBufs b, 
     if (tid == 0) report(st, DEV_BAD_SHAPE, -1, 0, -1);
     return;
   }
-  const int info = lub_square<NB>(sh, reinterpret_cast<double*>(smem_raw), b.A, N, bw, b.piv);
+  const int info = lub_square(sh, reinterpret_cast<double*>(smem_raw), b.A, N, b.piv);
   if (info != 0) {
     if (tid == 0) report(st, DEV_LAST_SINGULAR, -1, info, -1);
     return;
@@ -4566,7 +4565,7 @@ static FactorPlan<T> plan_factor(const DevState& s) {
     p.cta = s.sel == SEL_LU ? k_factor_cta<T, SEL_LU>
           : s.sel == SEL_QR ? k_factor_cta<T, SEL_QR> : k_factor_cta<T, SEL_QRP>;
     if constexpr (sizeof(T) == 8) {
-      p.lub = s.sel == SEL_LU ? lub_plan(2 * n + d.nr, n, false) : LubPlan{};
+      p.lub = s.sel == SEL_LU ? lub_plan(2 * n + d.nr, n) : LubPlan{};
       if (p.lub.threads) {
         smem_limit_once(lub_kernel(p.lub), p.lub.smem);
         lub_clusters(p.lub);
@@ -4717,11 +4716,10 @@ static void factor_last(DevState& s, const WorkSet<T>& w, cudaStream_t st, bool 
     cudaMemcpyAsync(s.Al, s.Hl, (size_t)d.Nr * d.Nc * 8, cudaMemcpyDeviceToDevice, st);
   }
   const LastBufs lb = last_bufs(s);
-  const LubPlan lp = lub_plan(d.Nc, d.Nc, true);
-  if (s.sel_last == LAST_LU && d.Nr == d.Nc && lp.threads) {
-    auto* kern = lp.depth == 32 ? k_last_lu_blocked<4> : lp.depth == 48 ? k_last_lu_blocked<6> : k_last_lu_blocked<8>;
-    smem_limit_once(kern, lp.smem);
-    kern<<<1, 512, lp.smem, st>>>(d, lb, s.st, lp.bw);
+  if (s.sel_last == LAST_LU && d.Nr == d.Nc && d.Nc >= 1 && d.Nc <= LUB_ROWS_MAX) {
+    const size_t sm = lub_last_smem(d.Nc);
+    smem_limit_once(k_last_lu_blocked, sm);
+    k_last_lu_blocked<<<1, 512, sm, st>>>(d, lb, s.st);
     check_launch("k_last_lu_blocked");
   } else {
     k_last_factor<double><<<1, 512, 0, st>>>(d, lb, s.sel_last, s.st);

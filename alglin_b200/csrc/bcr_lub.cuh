@@ -30,6 +30,9 @@
 // rate; the fragment and accumulator traffic takes the L1 pipe nearly as long).
 // 1,024 blocks of n = 128: the factorization's levels 8.8 -> 4.1 ms; a lone pair
 // 670 -> 193 us with its columns over 8 CTAs.
+//
+// The last block (lub_square) takes the same panels 16 columns at a time, with L and
+// a substitution in place of the operator: its L is less well conditioned.
 #pragma once
 
 #include "bcr_lub_plan.cuh"
@@ -83,8 +86,11 @@ __device__ __forceinline__ void sts_candidate(bool p, unsigned hdr, unsigned hi,
 // getrf pivot rule among the rows below ncand and leaves, by row, U on and right
 // of a pivot row's diagonal and the operator G left of it (rows that did not
 // become pivots: G).  Fills list and nrest, updates pos.  kb: columns factored
-// before.  Lout (may be null): L as it is formed, column stride ldl, by row.
-// Sets info (first zero pivot + 1).
+// before.  Sets info (first zero pivot + 1).
+//
+// SQ (the last block, w <= 16): the columns come from W and go back there by
+// original row, L\U; Pb keeps -L (the rows left, and the pivot rows left of their
+// diagonal) in place of the operator.
 //
 // Sub-blocks of 16 columns, a row of them per thread in registers.  As in the
 // warp-per-pair kernel the register of an eliminated column takes the operator
@@ -98,9 +104,9 @@ __device__ __forceinline__ void sts_candidate(bool p, unsigned hdr, unsigned hi,
 // warp and once over the warps' candidates, with one barrier between.  The
 // steps are one rolled loop over rotating registers: unrolled, each step's code
 // is fetched for a single use.
-template <int NT>
+template <int NT, bool SQ = false>
 __device__ void lub_panel(LubShared<NT>& sh, double* Pb, int ld, double* Xb, double* Ub, int nl, int kb, int w,
-                          int ncand, int depth, double* Lout = nullptr, int ldl = 0) {
+                          int ncand, int depth, double* Wc = nullptr, int ldw = 0) {
   constexpr unsigned FULL = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nwa = (nl + 31) / 32;  // warps with rows
@@ -128,7 +134,8 @@ __device__ void lub_panel(LubShared<NT>& sh, double* Pb, int ld, double* Xb, dou
       for (int attempt = 0;; ++attempt) {
         bool bad = false;
 #pragma unroll
-        for (int c = 0; c < SB; ++c) v[c] = Pb[(size_t)min(c0 + c, w - 1) * ld + tid];
+        for (int c = 0; c < SB; ++c)
+          v[c] = SQ ? ldg_if(act, Wc + (size_t)min(c, w - 1) * ldw + row) : Pb[(size_t)min(c0 + c, w - 1) * ld + tid];
 #pragma unroll 1
       for (int i = 0; i < steps; ++i) {
         // v[0] is column i; a step moves every column one register down and the
@@ -170,7 +177,7 @@ __device__ void lub_panel(LubShared<NT>& sh, double* Pb, int ld, double* Xb, dou
           sh.list[c0 + i] = tid | (row << 10);
         }
         const double l = used ? 0.0 : v0 * u[0];
-        if (Lout && act && !used) Lout[(size_t)(c0 + i) * ldl + row] = l;
+        if (SQ && act && !used) Pb[(size_t)i * ld + tid] = -l;
 #pragma unroll
         for (int c = 1; c < SB; ++c) v[c - 1] = fma(-l, u[c], v[c]);
         v[SB - 1] = used ? v0 : -l;
@@ -192,12 +199,16 @@ __device__ void lub_panel(LubShared<NT>& sh, double* Pb, int ld, double* Xb, dou
       if (act) {
 #pragma unroll
         for (int c = 0; c < SB; ++c) {
+          if constexpr (SQ) {
+            if (c < w) Wc[(size_t)c * ldw + row] = c >= own ? v[c] : -Pb[(size_t)c * ld + tid];
+            continue;
+          }
           if (!before && c0 + c < w) Pb[(size_t)(c0 + c) * ld + tid] = v[c];
           Xb[(size_t)c * ld + tid] = !before && c < own && c0 + c < w ? v[c] : 0.0;
         }
       }
     }
-    if (w <= SB) break;
+    if (SQ || w <= SB) break;
     __syncthreads();
     // the sub-block's pivot rows in the block's other columns, as they are now
     for (int e = tid; e < w * SB; e += NT) {
@@ -306,7 +317,7 @@ __device__ void lub_shrink(LubShared<NT>& sh, int depth) {
 // A group of columns with one source and one set of destinations (all pointers
 // to the group's first column):
 //   src: current values by original row, rows [lo, hi) (zero elsewhere);
-//   du:  the block's U rows, by order (or by row: in place);
+//   du:  the block's U rows, by order;
 //   dc:  the other rows, by order among them (or by row: in place);
 //   db:  the last rows (border), by number; db = dbs + value when dbs is given.
 struct LubCols {
@@ -323,10 +334,10 @@ struct LubCols {
 };
 
 // Columns [cb, cb + 16) of the group, row tiles [t0, t1) of 16 (the first
-// depth / 16 are the block's pivots).  byrow: destinations by original row.
+// depth / 16 are the block's pivots).  c_byrow: the other rows by original row.
 template <int NT, int NB>
 __device__ __forceinline__ void lub_item(const LubShared<NT>& sh, const double* Pb, int ld, const LubCols& G,
-                                         int cb, int t0, int t1, bool u_byrow, bool c_byrow) {
+                                         int cb, int t0, int t1, bool c_byrow) {
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   constexpr int PT = NB / 2;  // pivot tiles
   const int nrest = sh.nrest;
@@ -386,7 +397,7 @@ __device__ __forceinline__ void lub_item(const LubShared<NT>& sh, const double* 
       double add = 0.0;
       const double* as = nullptr;
       if (t < PT) {
-        dst = G.du + (u_byrow ? r : i);
+        dst = G.du + i;
         st = G.us;
       } else {
         const int e = i - 8 * NB, b = e - (nrest - G.nb);
@@ -425,20 +436,17 @@ __device__ __forceinline__ void lub_item(const LubShared<NT>& sh, const double* 
 // ranges; group(i) gives the columns of group i, make(i) its description.
 template <int NB, int NT, typename Cols, typename Make>
 __device__ __forceinline__ void lub_update(const LubShared<NT>& sh, const double* Pb, int ld, int ng,
-                                           bool whole, bool u_byrow, bool c_byrow, Cols cols, Make make) {
+                                           bool c_byrow, Cols cols, Make make) {
   const int warp = threadIdx.x >> 5, nw = NT / 32;
   int ns = 0;
   for (int i = 0; i < ng; ++i) ns += (cols(i) + 15) / 16;
   if (ns == 0) return;
   const int tiles = NB / 2 + (sh.nrest + 15) / 16;
-  // rows split where the strips leave warps idle (in place only whole strips:
-  // the U rows replace pivot rows that the other parts still read)
+  // rows split where the strips leave warps idle
   int parts = 1;
-  if (!whole) {
-    const int rounds = (ns + nw - 1) / nw;  // of whole strips
-    for (int p = 2; p <= 4; ++p)
-      if ((ns * p + nw - 1) / nw * (tiles / p + 3) < rounds * (tiles + 3) * 9 / 10 && p <= tiles) parts = p;
-  }
+  const int rounds = (ns + nw - 1) / nw;  // of whole strips
+  for (int p = 2; p <= 4; ++p)
+    if ((ns * p + nw - 1) / nw * (tiles / p + 3) < rounds * (tiles + 3) * 9 / 10 && p <= tiles) parts = p;
   const int tp = (tiles + parts - 1) / parts;
   for (int it = warp; it < ns * parts; it += nw) {
     int s = it % ns, i = 0;
@@ -447,7 +455,7 @@ __device__ __forceinline__ void lub_update(const LubShared<NT>& sh, const double
       ++i;
     }
     const int t0 = it / ns * tp, t1 = t0 + tp < tiles ? t0 + tp : tiles;
-    if (t0 < t1) lub_item<NT, NB>(sh, Pb, ld, make(i), 16 * s, t0, t1, u_byrow, c_byrow);
+    if (t0 < t1) lub_item<NT, NB>(sh, Pb, ld, make(i), 16 * s, t0, t1, c_byrow);
   }
 }
 
@@ -633,7 +641,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_factor_lu_lub(FactorArgs<doubl
         }
         return G;
       };
-      lub_update<NB>(sh, Pb, ld, 4, false, false, !last, cols, make);
+      lub_update<NB>(sh, Pb, ld, 4, !last, cols, make);
       __syncthreads();
       if (!last) {
         lub_shrink(sh, DEPTH);
@@ -675,42 +683,109 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_factor_lu_lub(FactorArgs<doubl
   }
 }
 
-// Blocked LU of the N x N matrix W in place (rows not moved): L\U by original
-// row, piv[position] = row.  Returns the LAPACK info.
-template <int NB, int NT>
-__device__ int lub_square(LubShared<NT>& sh, double* smem, double* W, int N, int bw, int* piv) {
-  constexpr int DEPTH = 8 * NB;
-  const int tid = threadIdx.x, lane = tid & 31, ld = lub_ld(N);
-  double* Pb = smem;
-  double* Xb = Pb + (size_t)DEPTH * ld;
-  double* Ub = Xb + (size_t)LUB_SB * ld;
+// Columns right of a block of 16 of the last block, a strip of 16 columns per warp,
+// in place: the pivot rows' part by substitution with L11 (a quad holds a column's
+// 16 rows; -L in Pb), then row -= L21 times it, the products summed from zero: they
+// round at the element's size once per block and not once per product.  With L11^-1
+// in place of the substitution, and summed onto the element, the solution's error
+// was 1.4 times as large for blocks of 64 columns at order 288 (1.2 times for 16).
+// Order 288: 360 us then, 340 now (it was 679 with the kernel before those).
+template <int NT>
+__device__ void lub_square_update(const LubShared<NT>& sh, const double* Pb, int ld, double* C, int N, int cols) {
+  constexpr int W = 16;
+  constexpr unsigned FULL = 0xffffffffu;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int tiles = (sh.nrest + 15) / 16;
+  const double* Lr[W / 4];
+  int pr[W / 4];
+#pragma unroll
+  for (int ks = 0; ks < W / 4; ++ks) {
+    const int e = sh.list[4 * ks + q];
+    Lr[ks] = Pb + (e & 1023);
+    pr[ks] = e >> 10;
+  }
+  for (int cb = 16 * warp; cb < cols; cb += 16 * (NT / 32)) {
+    double bf[W / 4][2];
+#pragma unroll
+    for (int ks = 0; ks < W / 4; ++ks)
+#pragma unroll
+      for (int v = 0; v < 2; ++v) bf[ks][v] = ldg_if(cb + 8 * v + g < cols, C + (size_t)(cb + 8 * v + g) * N + pr[ks]);
+#pragma unroll
+    for (int i = 0; i < W - 1; ++i) {
+      const double u0 = __shfl_sync(FULL, bf[i / 4][0], (lane & ~3) | (i & 3));
+      const double u1 = __shfl_sync(FULL, bf[i / 4][1], (lane & ~3) | (i & 3));
+#pragma unroll
+      for (int ks = i / 4; ks < W / 4; ++ks)
+        if (4 * ks + q > i) {
+          const double l = Lr[ks][(size_t)i * ld];
+          bf[ks][0] = fma(l, u0, bf[ks][0]);
+          bf[ks][1] = fma(l, u1, bf[ks][1]);
+        }
+    }
+#pragma unroll
+    for (int ks = 0; ks < W / 4; ++ks)
+#pragma unroll
+      for (int v = 0; v < 2; ++v)
+        if (cb + 8 * v + g < cols) C[(size_t)(cb + 8 * v + g) * N + pr[ks]] = bf[ks][v];
+    for (int t = 0; t < tiles; ++t) {
+      int ent[2];
+      double cur[2][2][2], acc[2][2][2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int e = t * 16 + u * 8 + g;
+        ent[u] = e < sh.nrest ? sh.list[W + e] : -1;
+#pragma unroll
+        for (int v = 0; v < 2; ++v)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int c = cb + 8 * v + 2 * q + h;
+            cur[u][v][h] = ldg_if(ent[u] >= 0 && c < cols, C + (size_t)c * N + (ent[u] >> 10));
+            acc[u][v][h] = 0.0;
+          }
+      }
+      const double* a0 = Pb + (size_t)q * ld + (ent[0] < 0 ? 0 : ent[0] & 1023);
+      const double* a1 = Pb + (size_t)q * ld + (ent[1] < 0 ? 0 : ent[1] & 1023);
+#pragma unroll
+      for (int ks = 0; ks < W / 4; ++ks) {
+        const double f0 = a0[(size_t)(4 * ks) * ld], f1 = a1[(size_t)(4 * ks) * ld];
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          dmma_8x8x4(acc[0][v][0], acc[0][v][1], f0, bf[ks][v]);
+          dmma_8x8x4(acc[1][v][0], acc[1][v][1], f1, bf[ks][v]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int v = 0; v < 2; ++v)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int c = cb + 8 * v + 2 * q + h;
+            if (ent[u] >= 0 && c < cols) C[(size_t)c * N + (ent[u] >> 10)] = cur[u][v][h] + acc[u][v][h];
+          }
+    }
+  }
+}
+
+// Blocked LU of the N x N matrix W in place (rows not moved), blocks of 16 columns:
+// L\U by original row, piv[position] = row.  Returns the LAPACK info.
+template <int NT>
+__device__ int lub_square(LubShared<NT>& sh, double* Pb, double* W, int N, int* piv) {
+  constexpr int BW = LUB_LAST_W;
+  const int tid = threadIdx.x, ld = lub_ld(N);
   for (int r = tid; r < N; r += NT) sh.row[r] = sh.pos[r] = r;
   if (tid == 0) sh.info = 0;
   __syncthreads();
   int nl = N;
-  for (int kb = 0; kb < N; kb += bw) {
-    const int w = N - kb < bw ? N - kb : bw;
-    lub_stage(sh, Pb, ld, W, N, nl, kb, w);
-    __syncthreads();
-    lub_panel(sh, Pb, ld, Xb, Ub, nl, kb, w, N, DEPTH, W + (size_t)kb * N, N);
+  for (int kb = 0; kb < N; kb += BW) {
+    const int w = N - kb < BW ? N - kb : BW;
+    lub_panel<NT, true>(sh, Pb, ld, nullptr, nullptr, nl, kb, w, N, BW, W + (size_t)kb * N, N);
     __syncthreads();
     if (sh.info != 0) break;
     for (int i = tid; i < w; i += NT) piv[kb + i] = sh.list[i] >> 10;
-    for (int c = tid >> 5; c < w; c += NT / 32)  // U (L went out as it was formed)
-      for (int i = lane; i <= c; i += 32) {
-        const int en = sh.list[i];
-        W[(size_t)(kb + c) * N + (en >> 10)] = Pb[(size_t)c * ld + (en & 1023)];
-      }
+    if (kb + w < N) lub_square_update(sh, Pb, ld, W + (size_t)(kb + w) * N, N, N - kb - w);  // w == BW
     __syncthreads();
-    lub_operator(sh, Pb, ld, nl, w, DEPTH);
-    __syncthreads();
-    lub_update<NB>(sh, Pb, ld, 1, true, true, true, [&](int) { return N - kb - w; },
-                   [&](int) {
-                     double* c = W + (size_t)(kb + w) * N;
-                     return LubCols{N - kb - w, c, N, 0, N, c, N, c, N, 0, nullptr, nullptr, 0};
-                   });
-    __syncthreads();
-    lub_shrink(sh, DEPTH);
+    lub_shrink(sh, BW);
     nl -= w;
     __syncthreads();
   }

@@ -6,12 +6,15 @@ constexpr int LUB_W = 64;          // panel columns per block (32 where 64 do no
 constexpr int LUB_ROWS_MAX = 512;  // one row per thread
 constexpr int LUB_SLICES_MAX = 8;  // CTAs of a cluster (the portable limit)
 constexpr int LUB_SB = 16;         // columns of a sub-block (registers of a row)
+constexpr int LUB_LAST_W = LUB_SB; // columns per block of the last block: one sub-block
 constexpr int LUB_UB = LUB_SB + 2; // stride of a column of the sub-block's pivot rows
 
 // column stride of the panel block: 10 mod 16 words of 8 bytes, so that the
 // column pairs of an accumulator tile (stride 2 ld) fall into different banks
 // and the columns of an A fragment (stride ld) nearly so
 __host__ __device__ inline int lub_ld(int rows) { return ((rows + 15) / 16) * 16 + 10; }
+// the last block's panel of 16 columns
+__host__ __device__ inline size_t lub_last_smem(int rows) { return (size_t)LUB_LAST_W * lub_ld(rows) * sizeof(double); }
 // the panel block, the sub-block's operator rows and pivot rows
 __host__ __device__ inline size_t lub_smem(int rows, int depth) {
   return ((size_t)(depth + LUB_SB) * lub_ld(rows) + (size_t)depth * LUB_UB) * sizeof(double);
@@ -28,7 +31,7 @@ struct LubPlan {
   size_t smem = 0;
   int clusters[3] = {0, 0, 0};  // clusters of 2, 4 and 8 CTAs resident at once
 };
-inline LubPlan lub_plan(int rows, int npiv, bool alone) {
+inline LubPlan lub_plan(int rows, int npiv) {
   LubPlan p;
   if (rows > LUB_ROWS_MAX || npiv < 1) return p;
   for (int most : {LUB_W, 32}) {
@@ -36,7 +39,7 @@ inline LubPlan lub_plan(int rows, int npiv, bool alone) {
     const int bw = ((npiv + blocks - 1) / blocks + 7) / 8 * 8;
     const int depth = bw <= 32 ? 32 : bw <= 48 ? 48 : 64;
     const size_t sm = lub_smem(rows, depth);
-    if (!alone && rows <= 256 && sm <= 106 * 1024) return {256, bw, depth, sm};
+    if (rows <= 256 && sm <= 106 * 1024) return {256, bw, depth, sm};
     if (sm <= 210 * 1024) return {512, bw, depth, sm};
   }
   return p;

@@ -17,7 +17,7 @@ int main() {
   for (int n = 1; n <= 128; ++n)
     for (int nr = 0; 2 * n + nr <= LUB_ROWS_MAX + 1; ++nr) {
       const int rows = 2 * n + nr;
-      LubPlan p = lub_plan(rows, n, false);
+      LubPlan p = lub_plan(rows, n);
       bool ok = (p.threads != 0) == (rows <= LUB_ROWS_MAX);
       if (p.threads) {
         ok &= rows <= p.threads && (p.threads == 256 || p.threads == 512);
