@@ -1570,8 +1570,9 @@ struct bcr_batch_s {
     return solve_mixed(fixed, true);
   }
   int read_status() {
-    cudaError_t e = cudaMemcpyAsync(h_st.data(), d_st, h_st.size() * sizeof(bcr::StatusWords),
-                                    cudaMemcpyDeviceToHost, stream);
+    cudaError_t e = bcr::launch_error();
+    if (e != cudaSuccess) return cuda_fail(e, "batch launch");
+    e = cudaMemcpyAsync(h_st.data(), d_st, h_st.size() * sizeof(bcr::StatusWords), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return cuda_fail(e, "batch status");
     for (size_t i = 0; i < h_st.size(); ++i)
