@@ -55,7 +55,7 @@ METRIC = "BABD factor+solve unknowns/s at rel. residual ≤1e-12: mixed vs plain
 # DRAM bytes per block moved by the factorization kernels of this workload,
 # from one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum) of the
 # same workload at nblock=40000 (the traffic grows with the blocks)
-FACT_DRAM_BYTES_PER_BLOCK = 21542
+FACT_DRAM_BYTES_PER_BLOCK = 21069
 CFG = dict(nblock=100000, n=16, qr=2, qx=2, nr=4, nx=4)
 
 
@@ -385,7 +385,7 @@ def run_ours(args):
                          "frac": achieved / peak, "peak_kind": peak_kind,
                          "traffic": FACT_DRAM_BYTES_PER_BLOCK * CFG["nblock"],
                          "traffic_source": "ncu dram__bytes_read+write of one factorization of this "
-                                           "workload at nblock=40000, 21,542 B per block, scaled to "
+                                           "workload at nblock=40000, 21,069 B per block, scaled to "
                                            "100000 blocks (profiles/dram_factor_solve_n16_nblock40000.md)",
                          "algorithmic_bytes": fact_b},
             "e2e": {"value": whole_job_value(world, s.ncols, e2e_t), "unit": "unknowns/s",
